@@ -45,11 +45,6 @@ namespace {
 
 constexpr int kVersion = 1;
 
-struct Timer {
-    cudaEvent_t e[11] = {};
-    bool valid = false;
-};
-
 /* What a captured step graph depends on besides device memory contents. */
 struct GraphKey {
     float dt, dt_ratio, gx, gy;
@@ -121,6 +116,7 @@ struct World {
     bool joint_filter_pending = false;  /* contacts of newly joined bodies to flag for filtering */
     int joint_cap = 0;                  /* joints the device arrays hold */
     bool record_events = false, record_pairs = false;
+    bool events_left = false;  /* the device's event list may hold events of a step before this one */
     bool new_contacts = false;
     float inv_dt0 = 0.0f;
     std::string err;
@@ -161,7 +157,6 @@ struct World {
     bool auto_grow = false;           /* b2g_set_auto_grow: contact / pair capacity grows on overflow */
     int capacity_grows = 0;
     int user_contact_cap = 0, user_pair_cap = 0;
-    Timer timer;
     b2g_profile profile{};
     int last_colours = 0;
     /* CUDA graphs of the steady-state step, one per contact-buffer parity */
@@ -1156,6 +1151,22 @@ int check_status(World* w) {
     return status_error(w, status);
 }
 
+/* When the phases of the last step ended, in ms from its start (the world's stream has drained; zeros
+ * before the first step). A phase the step did not have ends with the one before it. */
+int phase_times(World* w, double* t) {
+    for (int i = 0; i < PH_COUNT; ++i) t[i] = 0.0;
+    if (w->steps == 0) return B2G_OK;
+    unsigned long long at[PH_COUNT];
+    CUDA_OK(w, cudaMemcpy(at, w->d.stamps, sizeof(at), cudaMemcpyDeviceToHost));
+    const int order[PH_COUNT] = {PH_START, PH_INITIAL, PH_COLLIDE, PH_ISLANDS, PH_COLOURING, PH_SOLVER, PH_SORT, PH_HIERARCHY,
+                                 PH_TREE, PH_MERGE, PH_END};
+    for (int i = 1; i < PH_COUNT; ++i) {
+        at[order[i]] = std::max(at[order[i]], at[order[i - 1]]);
+        t[order[i]] = 1e-6 * (double)(at[order[i]] - at[PH_START]);
+    }
+    return B2G_OK;
+}
+
 /* the error for a device status word read after the stream drained (0: none); clears it */
 int status_error(World* w, int status) {
     if (status == 0) return B2G_OK;
@@ -1326,67 +1337,56 @@ int hook_new_pairs(World* w) {
 /* The launch sequence of one step on the world's stream (captured into a graph or run directly).
  * Under capture the profile events become external event-record nodes, so the host can still
  * time the graph's phases with cudaEventElapsedTime. */
-void issue_step(World* w, const StepParams& sp, float dt, bool capturing = false) {
+void issue_step(World* w, const StepParams& sp, float dt) {
     cudaStream_t s = w->stream;
-    Timer& t = w->timer;
-    auto mark = [&](cudaEvent_t e) {
-        if (capturing) cudaEventRecordWithFlags(e, s, cudaEventRecordExternal);
-        else cudaEventRecord(e, s);
-    };
     /* host callbacks (never under capture): the first failure is kept and the rest of the step skipped */
     auto hook = [&](int rc) {
         if (rc != B2G_OK && w->hook_rc == B2G_OK) w->hook_rc = rc;
     };
-    auto pair_hook = [&](int k) {
-        if (k == 2 && w->filter_fn && w->hook_rc == B2G_OK) hook(hook_new_pairs(w));
+    auto pair_hook = [&]() {
+        if (w->filter_fn && w->hook_rc == B2G_OK) hook(hook_new_pairs(w));
     };
-    cudaMemsetAsync(w->d.cnt + CNT_EVENTS, 0, sizeof(int), s);
-    mark(t.e[0]);
-    if (w->new_contacts) {
-        launch_broadphase(w->d, sp, s, w->num_sms, pair_hook);
+    if (w->record_events) cudaMemsetAsync(w->d.cnt + CNT_EVENTS, 0, sizeof(int), s);
+    const bool initial = w->new_contacts;
+    if (initial) {
+        launch_broadphase(w->d, sp, s, w->num_sms, PH_START, pair_hook);
         swap_contacts(w);
         w->new_contacts = false;
     }
-    mark(t.e[1]);
     HostContacts before;
     if ((w->filter_fn || w->pre_solve_fn) && w->hook_rc == B2G_OK) hook(hook_before_collide(w, before));
-    launch_collide(w->d, sp, s, w->allow_sleep || w->asleep_seen, w->num_sms);
+    launch_collide(w->d, sp, s, w->allow_sleep || w->asleep_seen, w->num_sms, !initial);
     if (w->pre_solve_fn && w->hook_rc == B2G_OK) hook(hook_pre_solve(w, before));
-    mark(t.e[2]);
     if (dt > 0.0f) {
-        launch_islands_and_constraints(w->d, sp, s);
-        mark(t.e[6]);
         const bool taping = w->tape && w->tape->recording;
-        launch_colouring(w->d, s, w->num_sms, w->part_solve);
-        if (taping) launch_tape_record(w->d, w->tape->d, sp, s, w->num_sms);
-        mark(t.e[3]);
-        launch_solver(w->d, sp, s, w->num_sms, w->part_solve);
-        if (taping) launch_tape_post(w->d, w->tape->d, sp, s, w->num_sms);
-        mark(t.e[4]);
-        launch_broadphase(w->d, sp, s, w->num_sms, [&](int k) {
-            mark(t.e[k == 0 ? 9 : k == 1 ? 10 : 7]);
-            pair_hook(k);
-        });
+        if (cluster_world(w->d)) {
+            launch_front(w->d, sp, s, w->part_solve, taping ? FRONT_ISLANDS | FRONT_COLOUR : FRONT_ALL);
+            if (taping) {
+                launch_tape_record(w->d, w->tape->d, sp, s, w->num_sms);
+                launch_front(w->d, sp, s, w->part_solve, FRONT_SOLVE);
+                launch_tape_post(w->d, w->tape->d, sp, s, w->num_sms);
+            }
+        } else {
+            launch_islands_and_constraints(w->d, sp, s);
+            launch_colouring(w->d, s, w->num_sms, w->part_solve);
+            if (taping) launch_tape_record(w->d, w->tape->d, sp, s, w->num_sms);
+            launch_solver(w->d, sp, s, w->num_sms, w->part_solve);
+            if (taping) launch_tape_post(w->d, w->tape->d, sp, s, w->num_sms);
+        }
+        /* a host contact filter is asked about the new pairs between the traversal and the merge */
+        if (cluster_world(w->d) && !w->filter_fn) launch_back(w->d, sp, s);
+        else launch_broadphase(w->d, sp, s, w->num_sms, PH_SOLVER, pair_hook);
         swap_contacts(w);
-        mark(t.e[8]);
         /* B2world::solve_toi (private/dynamics/b2_world.rs:946-950); the pass moves hierarchy leaves
          * in place without the four-way records, so the next broadphase pass rebuilds */
         if (w->continuous) {
             launch_continuous(w->d, sp, s, w->num_sms);
             cudaMemsetAsync(w->d.cnt + CNT_BP_FORCE, 1, sizeof(int), s);
         }
-        mark(t.e[5]);
         w->inv_dt0 = sp.inv_dt;
     } else {
-        mark(t.e[6]);
-        mark(t.e[3]);
-        mark(t.e[4]);
-        mark(t.e[9]);
-        mark(t.e[10]);
-        mark(t.e[7]);
+        launch_phase_stamp(w->d, PH_COLLIDE, s);
         if (w->auto_clear) launch_clear_forces(w->d, s);
-        mark(t.e[8]);
-        mark(t.e[5]);
     }
 }
 
@@ -1429,7 +1429,7 @@ int recover_overflow(World* w, const StepParams& sp) {
         int rc = grow_capacities(w, cc, pc);
         if (rc != B2G_OK) return rc;
         launch_touch_all_proxies(w->d, w->stream);
-        launch_broadphase(w->d, sp, w->stream, w->num_sms, nullptr, BP_REPEAT);
+        launch_broadphase(w->d, sp, w->stream, w->num_sms, PH_SOLVER, nullptr, BP_REPEAT);
         swap_contacts(w);
         CUDA_OK(w, cudaGetLastError());
     }
@@ -1456,15 +1456,13 @@ int step(World* w, float dt, int vi, int pi) {
     }
     StepParams sp = make_params(w, dt, vi, pi);
     cudaStream_t s = w->stream;
-    Timer& t = w->timer;
-    if (!t.valid) {
-        for (auto& e : t.e) cudaEventCreate(&e);
-        t.valid = true;
-    }
+    /* the list of begin and end events starts empty: a step that records clears it itself */
+    if (w->events_left && !w->record_events) CUDA_OK(w, cudaMemsetAsync(w->d.cnt + CNT_EVENTS, 0, sizeof(int), s));
+    w->events_left = w->record_events;
     const bool grow = w->auto_grow && !(w->tape && w->tape->recording) && !w->filter_fn;
     if (grow && w->new_contacts) {
         /* the initial pass of new fixtures on its own, checked before the step collides its contacts */
-        launch_broadphase(w->d, sp, s, w->num_sms);
+        launch_broadphase(w->d, sp, s, w->num_sms, PH_START);
         swap_contacts(w);
         w->new_contacts = false;
         rc = recover_overflow(w, sp);
@@ -1503,7 +1501,7 @@ int step(World* w, float dt, int vi, int pi) {
             cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
             if (e == cudaSuccess) {
                 const unsigned long long before = g_kernel_launches;
-                issue_step(w, sp, dt, true);
+                issue_step(w, sp, dt);
                 g.kernels = g_kernel_launches - before;  /* counted per replay instead */
                 g_kernel_launches = before;
                 e = cudaStreamEndCapture(s, &graph);
@@ -1678,6 +1676,14 @@ int b2g_world_create(const b2g_world_def* def, void** out) {
         delete w;
         return B2G_ERR_UNSUPPORTED;
     }
+    /* the phase stamps are not part of a saved state: an allocation of their own */
+    if (cudaMalloc((void**)&w->d.stamps, PH_COUNT * sizeof(unsigned long long)) != cudaSuccess ||
+        cudaMemsetAsync(w->d.stamps, 0, PH_COUNT * sizeof(unsigned long long), w->stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaStreamDestroy(w->stream);
+        delete w;
+        return B2G_ERR_OUT_OF_MEMORY;
+    }
     *out = w;
     return B2G_OK;
 }
@@ -1698,8 +1704,7 @@ int b2g_world_destroy(void* p) {
     tape_free(w);
     if (w->d_states) cudaFree(w->d_states);
     free_all(w);
-    if (w->timer.valid)
-        for (auto& e : w->timer.e) cudaEventDestroy(e);
+    cudaFree(w->d.stamps);
     cudaStreamDestroy(w->stream);
     delete w;
     return B2G_OK;
@@ -2569,27 +2574,18 @@ int b2g_get_profile(void* p, b2g_profile* out) {
     int rc = check_status(w);
     if (rc != B2G_OK) return rc;
     memset(out, 0, sizeof(*out));
-    if (!w->timer.valid || w->steps == 0) return B2G_OK;
-    float ms[6] = {0};
-    for (int i = 1; i < 6; ++i) {
-        if (cudaEventElapsedTime(&ms[i], w->timer.e[0], w->timer.e[i]) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(w, B2G_ERR_CUDA, "profile events could not be timed");
-        }
-    }
-    float toi = 0.0f;
-    if (cudaEventElapsedTime(&toi, w->timer.e[0], w->timer.e[8]) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(w, B2G_ERR_CUDA, "profile events could not be timed");
-    }
-    out->collide = ms[2] - ms[1];
-    out->solve_init = ms[3] - ms[2];
-    out->solve_velocity = ms[4] - ms[3];  /* the persistent solver kernel: velocity and position iterations */
+    double t[PH_COUNT];
+    rc = phase_times(w, t);
+    if (rc != B2G_OK) return rc;
+    out->collide = (float)(t[PH_COLLIDE] - t[PH_INITIAL]);
+    out->solve_init = (float)(t[PH_COLOURING] - t[PH_COLLIDE]);
+    /* the persistent solver kernel: velocity and position iterations */
+    out->solve_velocity = (float)(t[PH_SOLVER] - t[PH_COLOURING]);
     out->solve_position = 0.0f;
-    out->broadphase = (toi - ms[4]) + ms[1];
-    out->solve = toi - ms[2];
-    out->solve_toi = ms[5] - toi;
-    out->step = ms[5];
+    out->broadphase = (float)((t[PH_MERGE] - t[PH_SOLVER]) + t[PH_INITIAL]);
+    out->solve = (float)(t[PH_MERGE] - t[PH_COLLIDE]);
+    out->solve_toi = (float)(t[PH_END] - t[PH_MERGE]);
+    out->step = (float)t[PH_END];
     return B2G_OK;
 }
 
@@ -2599,28 +2595,14 @@ int b2g_get_phase_times(void* p, float* out, int32_t n) {
     int rc = check_status(w);
     if (rc != B2G_OK) return rc;
     for (int i = 0; i < std::min(n, 10); ++i) out[i] = 0.0f;
-    if (!w->timer.valid || w->steps == 0) return B2G_OK;
-    if (n >= 10) {
-        /* the tree pass in three: keys + sort, hierarchy, traversal (events 4, 9, 10, 7) */
-        const int sub[4] = {4, 9, 10, 7};
-        for (int i = 0; i < 3; ++i) {
-            if (cudaEventElapsedTime(&out[7 + i], w->timer.e[sub[i]], w->timer.e[sub[i + 1]]) != cudaSuccess) {
-                cudaGetLastError();
-                return fail(w, B2G_ERR_CUDA, "profile events could not be timed");
-            }
-        }
-    }
-    /* event order within a step: 0 start, 1 after the initial broadphase, 2 after collide,
-     * 6 after islands, 3 after colouring, 4 after the solver, 7 after the tree pass, 5 end */
-    const int order[8] = {0, 1, 2, 6, 3, 4, 7, 5};
-    float t[8] = {0};
-    for (int i = 1; i < 8; ++i) {
-        if (cudaEventElapsedTime(&t[i], w->timer.e[order[0]], w->timer.e[order[i]]) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(w, B2G_ERR_CUDA, "profile events could not be timed");
-        }
-    }
-    for (int i = 0; i < 7; ++i) out[i] = t[i + 1] - t[i];
+    double t[PH_COUNT];
+    rc = phase_times(w, t);
+    if (rc != B2G_OK) return rc;
+    /* the tree pass in three: keys + sort, hierarchy, traversal */
+    const int tree[4] = {PH_SOLVER, PH_SORT, PH_HIERARCHY, PH_TREE};
+    for (int i = 0; n >= 10 && i < 3; ++i) out[7 + i] = (float)(t[tree[i + 1]] - t[tree[i]]);
+    const int order[8] = {PH_START, PH_INITIAL, PH_COLLIDE, PH_ISLANDS, PH_COLOURING, PH_SOLVER, PH_TREE, PH_END};
+    for (int i = 0; i < 7; ++i) out[i] = (float)(t[order[i + 1]] - t[order[i]]);
     return B2G_OK;
 }
 
@@ -2907,6 +2889,7 @@ int b2g_state_load(void* p, const void* in, uint64_t bytes) {
     w->proxies_created = h.proxies_created;
     w->gravity = h.gravity;
     w->device_authoritative = true;
+    w->events_left = true;  /* the saved event list */
     rc = load_host_state(w, src, end);
     if (rc != B2G_OK) return rc;
     /* the barrier and hierarchy settings are the world's, not the saved state's */
@@ -3474,9 +3457,10 @@ int timed_steps(World* w, float dt, int vi, int pi, int steps, double* ms) {
         if (rc != B2G_OK) return rc;
         rc = check_status(w);
         if (rc != B2G_OK) return rc;
-        float t = 0.0f;
-        CUDA_OK(w, cudaEventElapsedTime(&t, w->timer.e[0], w->timer.e[5]));
-        *ms += t;
+        double t[PH_COUNT];
+        rc = phase_times(w, t);
+        if (rc != B2G_OK) return rc;
+        *ms += t[PH_END];
     }
     return B2G_OK;
 }

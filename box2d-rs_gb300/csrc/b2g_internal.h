@@ -345,7 +345,25 @@ struct DevWorld {
     uint32_t* sort_hist;
     int sort_hist_cap;
     int* cnt;
+    unsigned long long* stamps;  /* PH_COUNT: when the last step's phases ended (globaltimer, ns) */
 };
+
+/* The phases of a step whose ends are stamped, for the profile calls: a phase's end is written by one
+ * thread of the kernel that follows it (a time stamp costs one store; event records between the
+ * kernels of the step's graph would be a graph node each and keep a kernel from being scheduled while
+ * the one before it drains). A phase a step does not have keeps an older stamp; readers take the later
+ * of a stamp and the one before it in the order of the phases. */
+enum {
+    PH_START = 0, PH_INITIAL = 1, PH_COLLIDE = 2, PH_COLOURING = 3, PH_SOLVER = 4, PH_END = 5, PH_ISLANDS = 6,
+    PH_TREE = 7, PH_MERGE = 8, PH_SORT = 9, PH_HIERARCHY = 10, PH_COUNT = 11
+};
+__device__ __forceinline__ void phase_stamp(const DevWorld& w, int phase) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        unsigned long long t;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        w.stamps[phase] = t;
+    }
+}
 
 /* After a grid-barrier wait ran out, the step's buffers may be half-written: every later kernel of
  * the world returns at once (it reads no index another kernel computed) until the host reads and
@@ -384,10 +402,31 @@ inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+/* The same with the whole grid as one thread-block cluster (grid_barrier is then the cluster's barrier) */
+template <typename... KArgs, typename... Args>
+inline int launch_cluster(void (*kernel)(KArgs...), int blocks, int threads, size_t smem, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = blocks;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 /* kernel-file launchers */
 /* may_sleep: some body may be asleep (sleeping allowed, or a body made asleep): contacts then see
  * the bodies woken by contacts before them in the table's key order, as in the reference's list */
-void launch_collide(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool may_sleep, int num_sms);
+/* starts_step: no pass of this step ran before it */
+void launch_collide(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool may_sleep, int num_sms,
+                    bool starts_step);
 void launch_shape_rows(const DevWorld& w, int n_fixtures, cudaStream_t s);
 /* contact edits of destroy / refilter calls between steps (k_edit_contacts in k_collide.cu): fix_mark
  * per fixture, bit 0 destroyed (its contacts are destroyed), bit 1 refiltered (its contacts are flagged
@@ -400,6 +439,19 @@ void launch_touch_all_proxies(const DevWorld& w, cudaStream_t s);
 /* flags the contacts of bodies a joint keeps apart (after joints were created) */
 void launch_flag_joint_contacts(const DevWorld& w, cudaStream_t s, int num_sms);
 void launch_islands_and_constraints(const DevWorld& w, const StepParams& sp, cudaStream_t s);
+/* Worlds of up to kClusterMaxProxies proxies (and twice as many bodies) run the whole of islands,
+ * colouring and solver (`passes`: FRONT_* bits) as one kernel on one thread-block cluster, and the whole
+ * broadphase and contact merge as another (launch_back): cluster_world says whether a world does, given
+ * the device's largest cluster. */
+enum { FRONT_ISLANDS = 1, FRONT_COLOUR = 2, FRONT_SOLVE = 4, FRONT_ALL = 7 };
+constexpr int kClusterMaxBlocks = 16;
+constexpr int kClusterMaxProxies = kClusterMaxBlocks * 256;
+bool cluster_world(const DevWorld& w);
+int cluster_size(const DevWorld& w);
+int launch_front(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool parts, int passes);
+int launch_back(const DevWorld& w, const StepParams& sp, cudaStream_t s);
+/* a stamp on its own (a step that ends with a phase no kernel follows) */
+void launch_phase_stamp(const DevWorld& w, int phase, cudaStream_t s);
 /* parts: allow the part-local solve (used where the world's size suits it) */
 void launch_colouring(const DevWorld& w, cudaStream_t s, int num_sms, bool parts);
 int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms, bool parts);
@@ -410,14 +462,13 @@ void launch_time_of_impact(const ShapeRec* sa, const float4* swa, const ShapeRec
 int launch_continuous(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms);
 /* whether the part-local solve applies to this world (parts allowed and the world's size suits it) */
 bool use_parts(const DevWorld& w, int num_sms, bool allowed);
-/* mark (optional) is called with 0 after the keys and their sort, 1 after the hierarchy (build,
- * refit, four-way records, contact rows), 2 after the traversal (before the contact merge), so the
- * caller can record profiling events there */
+/* after_traversal (optional) is called after the traversal, before the contact merge. ends: the phase
+ * (PH_*) that ends where the pass starts */
 /* mode: BP_AUTO (the pass decides whether to rebuild the hierarchy), BP_REBUILD, or BP_REPEAT (the
  * same pass again, after a capacity overflow: the previous decision holds) */
 enum { BP_AUTO = 0, BP_REBUILD = 1, BP_REPEAT = 2 };
-void launch_broadphase(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms,
-                       const std::function<void(int)>& mark = nullptr, int mode = BP_AUTO);
+void launch_broadphase(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms, int ends,
+                       const std::function<void()>& after_traversal = nullptr, int mode = BP_AUTO);
 void launch_set_transform(const DevWorld& w, int body, float px, float py, float angle, cudaStream_t s);
 void launch_clear_forces(const DevWorld& w, cudaStream_t s);
 void launch_collide_pairs(const ShapeRec* a, const float4* xa, const ShapeRec* b, const float4* xb, const int* kind,

@@ -36,6 +36,7 @@
 #include <climits>
 
 #include "b2g_contact.cuh"
+#include "b2g_sort.cuh"
 
 namespace b2g {
 
@@ -67,9 +68,7 @@ __device__ __forceinline__ uint32_t spread16(uint32_t x) {
  * CNT_BP_MAX_AGE passes old (b2g_set_hierarchy_max_age). The decision depends only on the world's own
  * state, so a world and its checkpointed copy decide alike. A repeated pass (the same pass run again
  * after its capacities grew) keeps the decision. */
-__global__ void k_bp_decide(DevWorld w, int mode) {
-    pdl_entry();
-    B2G_RETURN_IF_ABORTED(w);
+__device__ __forceinline__ void bp_decide(const DevWorld& w, int mode) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     int* c = w.cnt;
     const int n = w.n_fixtures;
@@ -99,14 +98,17 @@ __global__ void k_bp_decide(DevWorld w, int mode) {
     c[CNT_BP_LAST_MOVED] = moved;
     c[CNT_BP_MOVED] = 0;
 }
+__global__ void k_bp_decide(DevWorld w, int mode, int ends) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    phase_stamp(w, ends);
+    bp_decide(w, mode);
+}
 
 __device__ __forceinline__ bool bp_rebuilding(const DevWorld& w) { return w.cnt[CNT_BP_REBUILD] != 0; }
 
 
-__global__ void k_bp_bounds(DevWorld w) {
-    pdl_entry();
-    B2G_RETURN_IF_ABORTED(w);
-    if (!bp_rebuilding(w)) return;
+__device__ __forceinline__ void bp_bounds(const DevWorld& w) {
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < w.n_bodies; b += gridDim.x * blockDim.x)
         w.b_rank[b] = INT_MAX;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * w.num_worlds; i += gridDim.x * blockDim.x) {
@@ -159,11 +161,14 @@ __global__ void k_bp_bounds(DevWorld w) {
         atomicMax(&w.cnt[CNT_BOUNDS + 3], mxy);
     }
 }
-
-__global__ void k_bp_keys(DevWorld w) {
+__global__ void k_bp_bounds(DevWorld w) {
     pdl_entry();
     B2G_RETURN_IF_ABORTED(w);
     if (!bp_rebuilding(w)) return;
+    bp_bounds(w);
+}
+
+__device__ __forceinline__ void bp_keys(const DevWorld& w) {
     float lx = 0.0f, ly = 0.0f, sx = 0.0f, sy = 0.0f;
     if (w.cnt[CNT_BOUNDS + 0] != INT_MAX) {
         lx = ord2f(w.cnt[CNT_BOUNDS + 0]);
@@ -193,6 +198,12 @@ __global__ void k_bp_keys(DevWorld w) {
         w.bp_val[f] = (uint32_t)f;
     }
 }
+__global__ void k_bp_keys(DevWorld w) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    if (!bp_rebuilding(w)) return;
+    bp_keys(w);
+}
 
 __device__ __forceinline__ int delta(const unsigned long long* k, int n, int i, int j) {
     if (j < 0 || j >= n) return -1;
@@ -202,10 +213,7 @@ __device__ __forceinline__ int delta(const unsigned long long* k, int n, int i, 
 }
 
 /* Karras, "Maximizing parallelism in the construction of BVHs, octrees, and k-d trees" (HPG 2012) */
-__global__ void k_bp_build(DevWorld w) {
-    pdl_entry();
-    B2G_RETURN_IF_ABORTED(w);
-    if (!bp_rebuilding(w)) return;
+__device__ __forceinline__ void bp_build(const DevWorld& w) {
     const int n = w.n_fixtures;
     const unsigned long long* k = w.bp_key;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n - 1; i += gridDim.x * blockDim.x) {
@@ -253,6 +261,13 @@ __global__ void k_bp_build(DevWorld w) {
         if (first && last) w.bp_world_root[wd] = ~p;  /* a world with a single proxy */
     }
 }
+__global__ void k_bp_build(DevWorld w) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    phase_stamp(w, PH_SORT);
+    if (!bp_rebuilding(w)) return;
+    bp_build(w);
+}
 
 
 __device__ __forceinline__ float4 box_union(float4 a, float4 b) {
@@ -268,10 +283,7 @@ __device__ __forceinline__ unsigned arrive_acq_rel(unsigned* p) {
 
 /* Bottom-up: each leaf's thread stores its box in its parent's record and arrives; the second of
  * the two children to arrive reads its sibling's box (in L2) and carries the union up. */
-__global__ void k_bp_refit(DevWorld w) {
-    pdl_entry();
-    B2G_RETURN_IF_ABORTED(w);
-    if (!bp_rebuilding(w)) return;
+__device__ __forceinline__ void bp_refit(const DevWorld& w) {
     const int n = w.n_fixtures;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         if (n < 2) break;
@@ -291,16 +303,19 @@ __global__ void k_bp_refit(DevWorld w) {
         }
     }
 }
+__global__ void k_bp_refit(DevWorld w) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    if (!bp_rebuilding(w)) return;
+    bp_refit(w);
+}
 
 __device__ __forceinline__ bool box_overlap(float4 a, float4 b) { return overlap4(a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w); }
 
 /* After the refit: each internal node's four-way record, its children's children (a leaf child
  * stands for itself). A traversal then tests four boxes per dependent fetch and descends two
  * levels at a time; the pairs found do not depend on the hierarchy's shape. */
-__global__ void k_bp_quad(DevWorld w) {
-    pdl_entry();
-    B2G_RETURN_IF_ABORTED(w);
-    if (!bp_rebuilding(w)) return;
+__device__ __forceinline__ void bp_quad(const DevWorld& w) {
     const int n = w.n_fixtures;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n - 1; i += gridDim.x * blockDim.x) {
         const int2 ch = w.bp_node_child[i];
@@ -326,6 +341,12 @@ __global__ void k_bp_quad(DevWorld w) {
         w.bp_quad_child[i] = make_int4(ids[0], ids[1], ids[2], ids[3]);
         for (int j = 0; j < 4; ++j) w.bp_quad_box[4 * (size_t)i + j] = qb[j];
     }
+}
+__global__ void k_bp_quad(DevWorld w) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    if (!bp_rebuilding(w)) return;
+    bp_quad(w);
 }
 
 /* componentwise growth of a stored box; returns whether this call changed it */
@@ -374,9 +395,7 @@ __device__ __forceinline__ int quad_place(const DevWorld& w, int node, int id) {
  * parent and the four-way record in its grandparent). A walk stops at the first ancestor whose record already covered the box: whoever grew
  * that record past it carries the growth further up, so when the kernel ends every ancestor covers
  * every leaf below it. */
-__global__ void k_bp_update(DevWorld w) {
-    pdl_entry();
-    B2G_RETURN_IF_ABORTED(w);
+__device__ __forceinline__ void bp_rows(const DevWorld& w) {
     /* every pass: the row index of the key-sorted contact table, c_row[r] = the first contact whose
      * key's high part is proxy id r. Entries of ids with no contact keep stale values; a reader
      * accepts c_row[r] only if that contact's key starts with r, which a stale entry cannot satisfy
@@ -387,7 +406,8 @@ __global__ void k_bp_update(DevWorld w) {
         if (i == 0 || (w.c.key[i - 1] >> w.key_bits) != r) w.c_row[r] = i;
         if (i == nc - 1 || (w.c.key[i + 1] >> w.key_bits) != r) w.c_row_end[r] = i + 1;
     }
-    if (bp_rebuilding(w)) return;
+}
+__device__ __forceinline__ void bp_update_leaves(const DevWorld& w) {
     const int n = w.n_fixtures;
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < n; f += gridDim.x * blockDim.x) {
         if (!w.f_moved[f]) continue;
@@ -420,6 +440,12 @@ __global__ void k_bp_update(DevWorld w) {
             x = px;
         }
     }
+}
+__global__ void k_bp_update(DevWorld w) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    bp_rows(w);
+    if (!bp_rebuilding(w)) bp_update_leaves(w);
 }
 
 __device__ __forceinline__ int lower_bound_u64(const unsigned long long* a, int n, unsigned long long key) {
@@ -559,9 +585,7 @@ __device__ __forceinline__ unsigned check_batch(const DevWorld& w, const StepPar
 constexpr int kLeafQueue = 224;  /* 31 left over + 32 lanes x 4 leaves in one round, or the setup's
                                     2 single-proxy roots per lane */
 
-__global__ void __launch_bounds__(kBlock) k_bp_traverse(DevWorld w, StepParams sp) {
-    pdl_entry();
-    B2G_RETURN_IF_ABORTED(w);
+__device__ __forceinline__ void bp_traverse(const DevWorld& w, const StepParams& sp) {
     __shared__ uint2 s_queue[kBlock / 32][kLeafQueue];
     __shared__ int s_give_node[kBlock / 32][32];
     __shared__ int s_give_f[kBlock / 32][32];
@@ -685,16 +709,26 @@ __global__ void __launch_bounds__(kBlock) k_bp_traverse(DevWorld w, StepParams s
         atomicMax((unsigned*)&w.cnt[CNT_BP_WARP_CHECKS], candidates);
     }
 }
+__global__ void __launch_bounds__(kBlock) k_bp_traverse(DevWorld w, StepParams sp) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    phase_stamp(w, PH_HIERARCHY);
+    bp_traverse(w, sp);
+}
 
 /* the moved flags are consumed; the colouring's rank weights start from zero (they are indexed by
  * Morton rank, of which there are as many as proxies) */
-__global__ void k_bp_clear_moved(DevWorld w) {
-    pdl_entry();
-    B2G_RETURN_IF_ABORTED(w);
+__device__ __forceinline__ void bp_clear_moved(const DevWorld& w) {
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < w.n_fixtures; f += gridDim.x * blockDim.x) {
         w.f_moved[f] = 0;
         w.rank_x[f] = 0ull;
     }
+}
+__global__ void k_bp_clear_moved(DevWorld w) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    phase_stamp(w, PH_TREE);
+    bp_clear_moved(w);
 }
 
 
@@ -753,6 +787,142 @@ __global__ void k_merge_finish(DevWorld w) {
         }
         w.cnt[CNT_CONTACTS] = total;
     }
+    phase_stamp(w, PH_MERGE);
+}
+
+/* ---- the whole pass of a small world on one cluster ---- */
+
+/* Stable sort of n <= kRankMax (key, value) pairs by the whole cluster: a key's place is the number of
+ * keys before it in (key, input place) order, counted by as many threads as there are to spare (a power
+ * of two of a warp's lanes for each key), the others' keys read from shared memory. One count and two
+ * barriers, where the radix sort takes two barriers for each 8 bits. A key has at most 53 bits: its
+ * place rides below it. */
+constexpr int kRankMax = 2048;
+constexpr int kRankTileKeys = 1024;
+static_assert(kRankMax <= 1 << 11, "an input place takes 11 bits");
+
+__device__ __forceinline__ void rank_sort_cluster(const DevWorld& w, unsigned long long* key, uint32_t* val,
+                                                  unsigned long long* key_alt, uint32_t* val_alt, int n) {
+    __shared__ unsigned long long s_key[kRankTileKeys];
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsize = gridDim.x * blockDim.x;
+    int parts = 1;
+    while (parts < 32 && 2 * parts * n <= gsize) parts <<= 1;
+    const int sub = gtid & (parts - 1);
+    for (int j0 = 0; j0 < n; j0 += gsize / parts) {
+        const int j = j0 + gtid / parts;
+        const unsigned long long mine = j < n ? key[j] : 0ull;
+        const unsigned long long at = (mine << 11) | (unsigned)j;
+        int r = 0;
+        for (int t0 = 0; t0 < n; t0 += kRankTileKeys) {
+            const int m = min(kRankTileKeys, n - t0);
+            __syncthreads();
+            for (int i = threadIdx.x; i < m; i += blockDim.x) s_key[i] = (key[t0 + i] << 11) | (unsigned)(t0 + i);
+            __syncthreads();
+            for (int i = sub; i < m; i += parts) r += s_key[i] < at ? 1 : 0;
+        }
+        for (int o = parts >> 1; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        if (sub == 0 && j < n) {
+            key_alt[r] = mine;
+            val_alt[r] = val[j];
+        }
+    }
+    grid_barrier(w);
+    for (int i = gtid; i < n; i += gsize) {
+        key[i] = key_alt[i];
+        val[i] = val_alt[i];
+    }
+}
+
+__device__ __forceinline__ void sort_cluster(const DevWorld& w, unsigned long long* key, uint32_t* val,
+                                             unsigned long long* key_alt, uint32_t* val_alt, int n, int bits) {
+    if (n <= kRankMax && bits <= 53) rank_sort_cluster(w, key, val, key_alt, val_alt, n);
+    else radix_sort_grid(key, val, key_alt, val_alt, n, bits, w.sort_hist, w.cnt);
+}
+
+/* update_pairs, add_pair and the merge of a world of a few thousand proxies as one kernel on one
+ * cluster: the passes of the kernels above, separated by cluster barriers instead of launches. A kept
+ * hierarchy with no new pair takes five barriers; as 20 launches the same pass took 62 us for a 16-body
+ * world, most of it launch and drain times. The merge counts each block's chunk of the table, so that
+ * one more barrier gives every contact its rank. */
+__global__ void __launch_bounds__(kBlock) k_back(const __grid_constant__ DevWorld w, const __grid_constant__ StepParams sp) {
+    pdl_entry();
+    if (cluster_leaves(w)) return;
+    phase_stamp(w, PH_SOLVER);
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsize = gridDim.x * blockDim.x;
+    bp_decide(w, BP_AUTO);
+    bp_rows(w);
+    grid_barrier(w);
+    if (bp_rebuilding(w)) {
+        bp_bounds(w);
+        grid_barrier(w);
+        bp_keys(w);
+        grid_barrier(w);
+        sort_cluster(w, w.bp_key, w.bp_val, w.bp_key_alt, w.bp_val_alt, w.n_fixtures, kMortonBits + w.morton_world_bits);
+        grid_barrier(w);
+        phase_stamp(w, PH_SORT);
+        bp_build(w);
+        grid_barrier(w);
+        bp_refit(w);
+        grid_barrier(w);
+        if (w.n_fixtures > 1) bp_quad(w);
+    } else {
+        phase_stamp(w, PH_SORT);
+        bp_update_leaves(w);
+    }
+    grid_barrier(w);
+    phase_stamp(w, PH_HIERARCHY);
+    bp_traverse(w, sp);
+    grid_barrier(w);
+    phase_stamp(w, PH_TREE);
+    bp_clear_moved(w);
+    /* the merge: every contact's rank among the survivors, from the counts of the blocks' chunks */
+    const int n = w.cnt[CNT_CONTACTS];
+    const int nn = min(w.cnt[CNT_NEW], w.pair_cap);
+    const int chunk = (n + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int c0 = min(n, (int)blockIdx.x * chunk), c1 = min(n, c0 + chunk);
+    uint32_t mine = 0, chunk_alive;
+    for (int i = c0 + threadIdx.x; i < c1; i += blockDim.x) mine += (w.c.flags[i] & CF_DEAD) ? 0u : 1u;
+    block_exclusive_scan(mine, &chunk_alive);
+    if (threadIdx.x == 0) w.blk_tot[blockIdx.x] = chunk_alive;
+    if (nn > 0) sort_cluster(w, w.n_key, w.n_idx, w.n_key_alt, w.n_idx_alt, nn, 2 * w.key_bits);
+    grid_barrier(w);
+    uint32_t before = 0, alive = 0;
+    for (int q = 0; q < (int)gridDim.x; ++q) {
+        const uint32_t t = (uint32_t)w.blk_tot[q];
+        if (q < (int)blockIdx.x) before += t;
+        alive += t;
+    }
+    uint32_t* rank = w.scan_tmp + w.contact_cap;
+    for (int base = c0; base < c1; base += blockDim.x) {
+        const int i = base + threadIdx.x;
+        const bool live = i < c1 && !(w.c.flags[i] & CF_DEAD);
+        uint32_t total;
+        const uint32_t r = before + block_exclusive_scan(live ? 1u : 0u, &total);
+        before += total;
+        if (i < c1 && nn > 0) rank[i] = r;
+        if (live) {
+            const int pos = (int)r + (nn > 0 ? lower_bound_u64(w.n_key, nn, w.c.key[i]) : 0);
+            if (pos < w.contact_cap) copy_contact(w.c, i, w.c_alt, pos);
+            else atomicOr((unsigned*)&w.cnt[CNT_STATUS], ST_CONTACT_OVERFLOW);
+        }
+    }
+    if (nn > 0) {
+        grid_barrier(w);
+        for (int j = gtid; j < nn; j += gsize) {
+            const unsigned long long key = w.n_key[j];
+            const int at = lower_bound_u64(w.c.key, n, key);
+            const int pos = j + (int)(at < n ? rank[at] : alive);
+            if (pos < w.contact_cap) init_contact(w, w.c_alt, pos, key, w.n_fix[w.n_idx[j]]);
+            else atomicOr((unsigned*)&w.cnt[CNT_STATUS], ST_CONTACT_OVERFLOW);
+        }
+    }
+    if (gtid == 0) {
+        w.cnt[CNT_ALIVE] = (int)alive;
+        w.cnt[CNT_MERGE_FROM] = n;
+        if ((int)alive + nn > w.contact_cap) atomicOr((unsigned*)&w.cnt[CNT_STATUS], ST_CONTACT_OVERFLOW);
+        w.cnt[CNT_CONTACTS] = min((int)alive + nn, w.contact_cap);
+    }
+    phase_stamp(w, PH_MERGE);
 }
 
 __global__ void k_touch_all(DevWorld w) {
@@ -767,18 +937,25 @@ void launch_touch_all_proxies(const DevWorld& w, cudaStream_t s) {
     B2G_LAUNCHED(1);
 }
 
+int launch_back(const DevWorld& w, const StepParams& sp, cudaStream_t s) {
+    static const cudaError_t allowed =
+        cudaFuncSetAttribute((const void*)k_back, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    (void)allowed;
+    B2G_LAUNCHED(1);
+    return launch_cluster(k_back, cluster_size(w), kBlock, 0, s, w, sp);
+}
+
 /* Runs update_pairs + add_pair and merges: the caller swaps w.c and w.c_alt afterwards. */
-void launch_broadphase(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms,
-                       const std::function<void(int)>& mark, int mode) {
+void launch_broadphase(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms, int ends,
+                       const std::function<void()>& after_traversal, int mode) {
     const int n = w.n_fixtures;
     const int gf = grid_for(n, kBlock, num_sms * 8);
-    launch_pdl(k_bp_decide, 1, 32, 0, s, w, mode); B2G_LAUNCHED(1);
+    launch_pdl(k_bp_decide, 1, 32, 0, s, w, mode, ends); B2G_LAUNCHED(1);
     if (n > 0) {
         launch_pdl(k_bp_bounds, gf, kBlock, 0, s, w); B2G_LAUNCHED(1);
         launch_pdl(k_bp_keys, gf, kBlock, 0, s, w); B2G_LAUNCHED(1);
         radix_sort_pairs_coop(w.bp_key, w.bp_val, w.bp_key_alt, w.bp_val_alt, &w.cnt[CNT_BP_SORT_N], n,
                               kMortonBits + w.morton_world_bits, w.sort_hist, w.cnt, s, num_sms, true);
-        if (mark) mark(0);
         launch_pdl(k_bp_build, gf, kBlock, 0, s, w); B2G_LAUNCHED(1);
         launch_pdl(k_bp_refit, gf, kBlock, 0, s, w); B2G_LAUNCHED(1);
         if (n > 1) {
@@ -786,12 +963,11 @@ void launch_broadphase(const DevWorld& w, const StepParams& sp, cudaStream_t s, 
         }
         launch_pdl(k_bp_update, grid_for(std::max(n, w.contact_cap), kBlock, num_sms * 8), kBlock, 0, s, w);
         B2G_LAUNCHED(1);
-        if (mark) mark(1);
         const int tb = w.cfg_traverse_block;
         launch_pdl(k_bp_traverse, grid_for(n, tb, num_sms * 2048 / tb), tb, 0, s, w, sp); B2G_LAUNCHED(1);
         launch_pdl(k_bp_clear_moved, gf, kBlock, 0, s, w); B2G_LAUNCHED(1);
     }
-    if (mark) mark(2);
+    if (after_traversal) after_traversal();
     /* sort new keys; payload = emission slot */
     radix_sort_pairs_coop(w.n_key, w.n_idx, w.n_key_alt, w.n_idx_alt, &w.cnt[CNT_NEW], w.pair_cap, 2 * w.key_bits,
                           w.sort_hist, w.cnt, s, num_sms);

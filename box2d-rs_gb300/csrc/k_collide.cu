@@ -166,8 +166,11 @@ __device__ __forceinline__ bool warp_aborted(const DevWorld& w) {
 
 }  // namespace
 
-__global__ void __launch_bounds__(256, 4) k_collide(DevWorld w, StepParams sp, int deferred) {
+__global__ void __launch_bounds__(256, 4) k_collide(DevWorld w, StepParams sp, int deferred, int starts_step) {
+    pdl_entry();
     if (warp_aborted(w)) return;
+    if (starts_step) phase_stamp(w, PH_START);
+    phase_stamp(w, PH_INITIAL);
     const int n = w.cnt[CNT_CONTACTS];
     const int lane = threadIdx.x & 31;
     const int stride = gridDim.x * blockDim.x;
@@ -317,9 +320,11 @@ void launch_shape_rows(const DevWorld& w, int n_fixtures, cudaStream_t s) {
     B2G_LAUNCHED(1);
 }
 
-void launch_collide(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool may_sleep, int num_sms) {
+void launch_collide(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool may_sleep, int num_sms,
+                    bool starts_step) {
     const int block = w.cfg_collide_block;
-    k_collide<<<grid_for(w.contact_cap, block, w.num_sms * 2048 / block), block, 0, s>>>(w, sp, may_sleep ? 1 : 0);
+    launch_pdl(k_collide, grid_for(w.contact_cap, block, w.num_sms * 2048 / block), block, 0, s, w, sp, may_sleep ? 1 : 0,
+               starts_step ? 1 : 0);
     B2G_LAUNCHED(1);
     if (!may_sleep) return;
     DevWorld wc = w;

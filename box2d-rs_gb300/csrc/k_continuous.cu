@@ -876,7 +876,10 @@ __global__ void __launch_bounds__(kTBlock) k_continuous(DevWorld w, StepParams s
         for (int j = gtid; j < nm; j += gstride) w.f_moved[w.t_moved[j]] = 0;
     }
     const int na = appended(w, n_tab);
-    if (na == 0) return;
+    if (na == 0) {
+        phase_stamp(w, PH_END);
+        return;
+    }
     for (int j = gtid; j < na; j += gstride) {
         const unsigned long long key = w.c.key[n_tab + j];
         int rank = 0;
@@ -893,6 +896,7 @@ __global__ void __launch_bounds__(kTBlock) k_continuous(DevWorld w, StepParams s
     if (!grid_barrier(w)) return;
     for (int k = lo + gtid; k < n_tab + na; k += gstride) copy_contact(w.c_alt, k, w.c, k);
     if (gtid == 0) vcnt[CNT_CONTACTS] = n_tab + na;
+    phase_stamp(w, PH_END);
 }
 
 }  // namespace

@@ -28,6 +28,10 @@
  * The host reference solved in the GPU's colour order (the oracle's ordering hook)
  * gives bit-identical bodies, because each operation is the same IEEE f32 operation.
  */
+#include <algorithm>
+#include <mutex>
+#include <vector>
+
 #include "b2g_internal.h"
 #include "b2g_joint.cuh"
 #include "b2g_solver_math.cuh"
@@ -260,9 +264,7 @@ __device__ int colour_tail(const DevWorld& w, int round) {
  * Slots are then ordered part by part, each part by colour, then the boundary colours: solving
  * the parts concurrently is solving them one after the other, as no two parts share a dynamic
  * body, so this slot order is the sequential solve order. */
-__global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
-    B2G_RETURN_IF_ABORTED(w);
-    grid_barrier_start();
+__device__ __forceinline__ bool colour_pass(const DevWorld& w, int nparts) {
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int gsize = gridDim.x * blockDim.x;
     const int n = w.cnt[CNT_CONS];
@@ -300,7 +302,7 @@ __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
             w.part_cend[q] = 0;
             w.part_rbeg[q] = INT_MAX;
         }
-        if (!grid_barrier(w)) return;
+        if (!grid_barrier(w)) return false;
         /* each block scans its chunk of ranks: (weight << 32 | has weight), exclusive */
         const int chunk = (nf + (int)gridDim.x - 1) / (int)gridDim.x;
         const int r0 = min(nf, (int)blockIdx.x * chunk), r1 = min(nf, r0 + chunk);
@@ -315,7 +317,7 @@ __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
             carry += tot;
         }
         if (threadIdx.x == 0) w.blk_tot[blockIdx.x] = carry;
-        if (!grid_barrier(w)) return;
+        if (!grid_barrier(w)) return false;
         unsigned long long before = 0, all = 0;
         {
             unsigned long long mine = 0, every = 0;
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
         const bool aligned = w.num_worlds > 1;
         if (aligned) {
             for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) w.rank_x[r] += before;
-            if (!grid_barrier(w)) return;
+            if (!grid_barrier(w)) return false;
         }
         const unsigned long long base_x = aligned ? 0ull : before;
         for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
             w.b_cidx[b] = c;
             w.cache_body[c] = b;
         }
-        if (!grid_barrier(w)) return;
+        if (!grid_barrier(w)) return false;
         /* each part's range of constraint bodies */
         ncache = min(nf, (int)(uint32_t)all);
         for (int c = gtid; c < ncache; c += gsize) {
@@ -414,7 +416,7 @@ __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
         w.cons_colour[k] = (keep && (kept >> 7) == stamp && ((kept >> 6) & 1u) == cls) ? (int)(kept & 63u) : -1;
     }
     for (int c = gtid; c < (P + 1) * kMaxColours; c += gsize) w.col_hist[c] = 0;
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     /* the kept colours are taken at their bodies */
     for (int k = gtid; k < n; k += gsize) {
         const int c = w.cons_colour[k];
@@ -433,7 +435,7 @@ __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
         w.cnt[CNT_ROUNDS] = 0;
         w.cnt[CNT_TAIL] = 0;
     }
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     int round = 0;
     for (;;) {
         const int remaining = ((volatile int*)w.cnt)[CNT_UNCOLOURED + ((round + 1) & 1)];
@@ -446,9 +448,9 @@ __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
                     const int at = atomicAdd(&w.cnt[CNT_TAIL], 1);
                     if (at < kColourTail) w.col_tail[at] = k;
                 }
-            if (!grid_barrier(w)) return;
+            if (!grid_barrier(w)) return false;
             if (blockIdx.x == 0) round = colour_tail(w, round);
-            if (!grid_barrier(w)) return;
+            if (!grid_barrier(w)) return false;
             break;
         }
         if (round >= kMaxColours - kFirstFitColours) {
@@ -474,7 +476,7 @@ __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
             if (is_dynamic(w.b_flags[bd.y])) atomicMin(&offer[cm + bd.y], key);
         }
         if (gtid == 0) w.cnt[CNT_UNCOLOURED + (round & 1)] = 0;
-        if (!grid_barrier(w)) return;
+        if (!grid_barrier(w)) return false;
         /* B: local minima take the lowest colour free at both bodies */
         for (int k = gtid; k < n; k += gsize) {
             if (w.cons_colour[k] >= 0) continue;
@@ -506,7 +508,7 @@ __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
             }
         }
         ++round;
-        if (!grid_barrier(w)) return;
+        if (!grid_barrier(w)) return false;
     }
     if (gtid == 0 && w.cnt[CNT_TAIL] == 0) w.cnt[CNT_ROUNDS] = round;
     /* histogram rows: part p's interior colours are row p, the boundary colours row P */
@@ -514,13 +516,13 @@ __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
         const int part = w.cons_part[k];
         atomicAdd(&w.col_hist[(part < 0 ? P : part) * kMaxColours + w.cons_colour[k]], 1);
     }
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     for (int r = blockIdx.x; r <= P; r += gridDim.x) {
         int tot;
         block_scan_excl(w.col_hist[r * kMaxColours + threadIdx.x], &tot);
         if (threadIdx.x == 0) w.part_tot[r] = tot;
     }
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     /* dense offsets of each row's non-empty colours; the histogram becomes the slot cursors */
     for (int r = blockIdx.x; r <= P; r += gridDim.x) {
         int part_sum = 0;
@@ -554,7 +556,7 @@ __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
             }
         }
     }
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     const uint32_t next = (stamp + 1u) & kStampMask;
     for (int k = gtid; k < n; k += gsize) {
         const int c = w.cons_colour[k];
@@ -570,6 +572,7 @@ __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
         w.s_cons[slot] = k;
     }
     if (gtid == 0) w.cnt[CNT_COLOURINGS] = (int)next;
+    return true;
 }
 
 /* ---------------- solver (cooperative) ---------------- */
@@ -966,9 +969,7 @@ __device__ __forceinline__ void part_load(const PartCtx& pc, const float4* glob)
  * the solved bodies' flags, then the constraint list in contact order (each block counts its chunk
  * of the table, the chunks' counts give each block its offset, and a block scan places the block's
  * constraints). */
-__global__ void __launch_bounds__(kBlock) k_islands(DevWorld w, int allow_sleep) {
-    B2G_RETURN_IF_ABORTED(w);
-    grid_barrier_start();
+__device__ __forceinline__ bool islands_pass(const DevWorld& w, int allow_sleep) {
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int gsize = gridDim.x * blockDim.x;
     const int nb = w.n_bodies;
@@ -978,7 +979,7 @@ __global__ void __launch_bounds__(kBlock) k_islands(DevWorld w, int allow_sleep)
         w.b_flags[b] &= ~BF_ISLAND;
         if (allow_sleep) w.isl_sleep[b] = kMaxFloat;
     }
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     const int n = w.cnt[CNT_CONTACTS];
     for (int i = gtid; i < n; i += gsize) {
         if (!contact_is_constraint(w.c.flags[i])) continue;
@@ -992,13 +993,13 @@ __global__ void __launch_bounds__(kBlock) k_islands(DevWorld w, int allow_sleep)
         if (is_static(fa) || is_static(fb) || !(fa & BF_ENABLED) || !(fb & BF_ENABLED)) continue;
         uf_union(w.b_island, bd.x, bd.y);
     }
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     for (int b = gtid; b < nb; b += gsize) {
         const int r = uf_find(w.b_island, b);
         const uint32_t f = w.b_flags[b];
         agg_atomic_or(w.isl_minsep + w.body_cap, r, ((f & BF_AWAKE) && (f & BF_ENABLED) && !is_static(f)) ? 1u : 0u);
     }
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     for (int b = gtid; b < nb; b += gsize) {
         int r = w.b_island[b];
         r = w.b_island[r];
@@ -1007,7 +1008,7 @@ __global__ void __launch_bounds__(kBlock) k_islands(DevWorld w, int allow_sleep)
         const uint32_t f = w.b_flags[b];
         if (!is_static(f) && (f & BF_ENABLED) && w.isl_minsep[w.body_cap + r]) w.b_flags[b] = f | BF_AWAKE | BF_ISLAND;
     }
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     /* the constraint list: this block's chunk of the contact table */
     const int chunk = (n + (int)gridDim.x - 1) / (int)gridDim.x;
     const int c0 = min(n, (int)blockIdx.x * chunk), c1 = min(n, c0 + chunk);
@@ -1021,7 +1022,7 @@ __global__ void __launch_bounds__(kBlock) k_islands(DevWorld w, int allow_sleep)
     int block_total;
     block_scan_excl(mine, &block_total);
     if (threadIdx.x == 0) w.blk_tot[blockIdx.x] = (unsigned long long)block_total;
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     int before_part = 0, all_part = 0;
     for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) {
         const int t = (int)w.blk_tot[q];
@@ -1051,14 +1052,13 @@ __global__ void __launch_bounds__(kBlock) k_islands(DevWorld w, int allow_sleep)
         carry += tot;
     }
     if (gtid == 0) w.cnt[CNT_CONS] = min(all, w.cons_cap);
+    return true;
 }
 
 /* k_solve runs 256 or 512 threads per block (cfg_solver_block); nothing in it depends on which */
 constexpr int kSolveMaxBlock = 512;
 
-__global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams sp) {
-    B2G_RETURN_IF_ABORTED(w);
-    grid_barrier_start();
+__device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& sp) {
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int gsize = gridDim.x * blockDim.x;
     const int nb = w.n_bodies;
@@ -1091,16 +1091,16 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
             w.b_vel[b] = v;
         }
     }
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     /* phase 1: constraint initialisation */
     for (int k = gtid; k < ncons; k += gsize) init_slot(w, sp, k);
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     const int interior = w.cnt[CNT_INTERIOR];
     const bool parts = interior > 0;
     const int nparts = w.cnt[CNT_PARTS];
     if (parts && (nparts <= 0 || nparts > (int)gridDim.x)) {  /* the same for every block: all return */
         if (gtid == 0) atomicOr((unsigned*)&w.cnt[CNT_STATUS], ST_PART_MISMATCH);
-        return;
+        return false;
     }
     extern __shared__ float4 s_part[];
     __shared__ int s_off[kMaxColours + 1];
@@ -1176,17 +1176,17 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
                 for (int j = threadIdx.x; j < pc.cap_vel; j += blockDim.x) w.vc_imp[pc.ibeg + j] = vs[j].imp;
             if (ncol > 0 || last) part_store(pc, w.b_vel);
             if (ncol > 0) {
-                if (!grid_barrier(w)) return;
+                if (!grid_barrier(w)) return false;
                 for (int c = 0; c < ncol; ++c) {
                     bnd_vel_sweep(w, pc, c, warm, last);
-                    if (!grid_barrier(w)) return;
+                    if (!grid_barrier(w)) return false;
                 }
                 if (!last) {
                     part_load(pc, w.b_vel);
                     __syncthreads();
                 }
             } else if (last) {
-                if (!grid_barrier(w)) return;
+                if (!grid_barrier(w)) return false;
             }
         }
     } else {
@@ -1195,7 +1195,7 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
             for (int c = 0; c < ncol; ++c) {
                 const int beg = w.col_off[c], end = w.col_off[c + 1];
                 for (int k = beg + gtid; k < end; k += gsize) warm_slot(w, k);
-                if (!grid_barrier(w)) return;
+                if (!grid_barrier(w)) return false;
             }
         }
         /* phase 2b: the joints' init_velocity_constraints (with their warm start) follow the
@@ -1205,7 +1205,7 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
                 const int j = w.j_order[q];
                 if (joint_island(w, j) >= 0) joint_init_velocity(w, sp, j);
             }
-            if (!grid_barrier(w)) return;
+            if (!grid_barrier(w)) return false;
         }
         /* phase 3: velocity iterations, joints before contacts (:205-215) */
         for (int it = 0; it < sp.vi; ++it) {
@@ -1214,12 +1214,12 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
                     const int j = w.j_order[q];
                     if (joint_island(w, j) >= 0) joint_solve_velocity(w, sp, j);
                 }
-                if (!grid_barrier(w)) return;
+                if (!grid_barrier(w)) return false;
             }
             for (int c = 0; c < ncol; ++c) {
                 const int beg = w.col_off[c], end = w.col_off[c + 1];
                 for (int k = beg + gtid; k < end; k += gsize) solve_velocity_slot(w, k);
-                if (!grid_barrier(w)) return;
+                if (!grid_barrier(w)) return false;
             }
         }
     }
@@ -1262,7 +1262,7 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
         w.b_vel[b] = make_float4(vv.x, vv.y, wv, v.w);
         for (int j = 0; j < sp.pi; ++j) w.isl_minsep[(size_t)j * w.body_cap + b] = 0u;
     }
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     /* phase 5: position iterations with the per-island early exit (:257-274).
      * Iteration j accumulates max(-separation) of each island into its own buffer j (all
      * zeroed in phase 4); an island has stopped before iteration `it` if some earlier buffer
@@ -1301,10 +1301,10 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
             part_pos_sweeps(w, pc, it, cur, tol);
             if (ncol > 0) {
                 part_store(pc, w.b_pos);
-                if (!grid_barrier(w)) return;
+                if (!grid_barrier(w)) return false;
                 for (int c = 0; c < ncol; ++c) {
                     bnd_pos_sweep(w, pc, c, it, cur, tol);
-                    if (!grid_barrier(w)) return;
+                    if (!grid_barrier(w)) return false;
                 }
                 if (it < sp.pi - 1) {
                     part_load(pc, w.b_pos);
@@ -1312,7 +1312,7 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
                 }
             } else if (it == sp.pi - 1) {
                 part_store(pc, w.b_pos);
-                if (!grid_barrier(w)) return;
+                if (!grid_barrier(w)) return false;
             }
             continue;
         }
@@ -1327,7 +1327,7 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
                 const float ms = solve_position_slot(w, k);
                 agg_atomic_max(cur, isl, ms < 0.0f ? __float_as_uint(-ms) : 0u);
             }
-            if (!grid_barrier(w)) return;
+            if (!grid_barrier(w)) return false;
         }
         /* the joints after the contacts; a joint out of its slop keeps its island going
          * (contacts_okay && joints_okay, b2_island_private.rs:257-274) */
@@ -1342,7 +1342,7 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
                 if (done) continue;
                 if (!joint_solve_position(w, j)) atomicMax(&cur[isl], __float_as_uint(kMaxFloat));
             }
-            if (!grid_barrier(w)) return;
+            if (!grid_barrier(w)) return false;
         }
     }
     /* phase 6a: copy back (synchronize_transform), sleep bookkeeping, clear forces */
@@ -1373,7 +1373,7 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
         if (sp.auto_clear) w.b_force[b] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     if (sp.allow_sleep) {
-        if (!grid_barrier(w)) return;
+        if (!grid_barrier(w)) return false;
         for (int b = gtid; b < nb; b += gsize) {
             const uint32_t f = w.b_flags[b];
             if (!(f & BF_ISLAND)) continue;
@@ -1388,7 +1388,7 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
             }
         }
     }
-    if (!grid_barrier(w)) return;
+    if (!grid_barrier(w)) return false;
     /* phase 6b: synchronize fixtures (private/dynamics/b2_body.rs:455-475); the proxies moved are
      * counted for the broadphase's rebuild decision */
     unsigned moved = 0;
@@ -1412,7 +1412,57 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
     }
     moved = __reduce_add_sync(0xffffffffu, moved);
     if ((threadIdx.x & 31) == 0 && moved) atomicAdd(&w.cnt[CNT_BP_MOVED], (int)moved);
+    return true;
 }
+
+__global__ void __launch_bounds__(kBlock) k_islands(DevWorld w, int allow_sleep) {
+    B2G_RETURN_IF_ABORTED(w);
+    phase_stamp(w, PH_COLLIDE);
+    grid_barrier_start();
+    islands_pass(w, allow_sleep);
+}
+
+__global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
+    B2G_RETURN_IF_ABORTED(w);
+    phase_stamp(w, PH_ISLANDS);
+    grid_barrier_start();
+    colour_pass(w, nparts);
+}
+
+__global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams sp) {
+    B2G_RETURN_IF_ABORTED(w);
+    phase_stamp(w, PH_COLOURING);
+    grid_barrier_start();
+    solve_pass(w, sp);
+}
+
+/* Islands, colouring and solver of a world of a few thousand bodies as one kernel on one cluster of up
+ * to 16 blocks (passes: FRONT_*; a taped step stops after the colouring to record it). Such a step is
+ * bound by the latency of its barriers and launches, not by work: three cooperative launches of 152
+ * blocks took 20 + 22 + 56 us for a 16-body world (each launch a memset of its counter besides) and
+ * every barrier of their sweeps 1.4 us; here a barrier takes 0.3 us (one block: a __syncthreads) and the
+ * passes follow each other without a launch. */
+__global__ void __launch_bounds__(kBlock) k_front(const __grid_constant__ DevWorld w, const __grid_constant__ StepParams sp,
+                                                  int nparts, int passes) {
+    pdl_entry();
+    if (cluster_leaves(w)) return;
+    if (passes & FRONT_ISLANDS) {
+        phase_stamp(w, PH_COLLIDE);
+        islands_pass(w, sp.allow_sleep);
+    }
+    if (passes & FRONT_COLOUR) {
+        grid_barrier(w);
+        phase_stamp(w, PH_ISLANDS);
+        colour_pass(w, nparts);
+    }
+    if (passes & FRONT_SOLVE) {
+        grid_barrier(w);
+        phase_stamp(w, PH_COLOURING);
+        solve_pass(w, sp);
+    }
+}
+
+__global__ void k_phase_stamp(DevWorld w, int phase) { phase_stamp(w, phase); }
 
 __global__ void k_set_transform(DevWorld w, int body, float px, float py, float angle) {
     /* B2body::set_transform, private/dynamics/b2_body.rs:418-447 */
@@ -1515,6 +1565,16 @@ void launch_colouring(const DevWorld& w, cudaStream_t s, int num_sms, bool parts
 constexpr int kPartSmemOne = 200 * 1024;
 constexpr int kPartSmemTwo = 96 * 1024;
 
+/* the solver's shared memory for the part-local solve, set in the parameters it is launched with */
+size_t part_smem(StepParams& sp, int budget) {
+    /* a part holds at most ceil(n_fixtures / blocks) ranks; bodies take a quarter of the memory */
+    const int nb = (budget / 4 / 20) & ~3;
+    const int body_bytes = (nb + nb / 4) * 16;
+    sp.part_bodies = nb;
+    sp.part_slot_bytes = std::max(0, budget - body_bytes);
+    return (size_t)(budget > 0 ? body_bytes + sp.part_slot_bytes : 0);
+}
+
 int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms, bool parts) {
     static bool attr_set = false;
     if (!attr_set) {
@@ -1527,20 +1587,73 @@ int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int n
     size_t smem = 0;
     spc.part_bodies = 0;
     spc.part_slot_bytes = 0;
-    if (use_parts(w, num_sms, parts)) {
-        const int budget = w.cfg_coop_per_sm == 1 ? kPartSmemOne : (w.cfg_coop_per_sm == 2 ? kPartSmemTwo : 0);
-        /* a part holds at most ceil(n_fixtures / blocks) ranks; bodies take at most half */
-        const int nb = (budget / 4 / 20) & ~3;  /* a quarter of it for bodies */
-        const int body_bytes = (nb + nb / 4) * 16;
-        spc.part_bodies = nb;
-        spc.part_slot_bytes = std::max(0, budget - body_bytes);
-        smem = (size_t)(budget > 0 ? body_bytes + spc.part_slot_bytes : 0);
-    }
+    if (use_parts(w, num_sms, parts))
+        smem = part_smem(spc, w.cfg_coop_per_sm == 1 ? kPartSmemOne : (w.cfg_coop_per_sm == 2 ? kPartSmemTwo : 0));
     void* args[] = {&wc, &spc};
     B2G_LAUNCHED(1);
     cudaMemsetAsync(w.cnt + CNT_BARRIER, 0, sizeof(int), s);
     const int threads = w.cfg_coop_per_sm == 1 && w.cfg_solver_block == kSolveMaxBlock ? kSolveMaxBlock : kBlock;
     return (int)cudaLaunchCooperativeKernel((const void*)k_solve, dim3(blocks), dim3(threads), args, smem, s);
+}
+
+/* The largest cluster k_front and k_back can run as on the current device (0: none), found once per
+ * device: 16 blocks need the non-portable size and as many free SMs in one GPC. */
+static int max_cluster() {
+    static std::mutex m;
+    static std::vector<int> found;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 0;
+    std::lock_guard<std::mutex> lock(m);
+    if ((int)found.size() <= dev) found.resize((size_t)dev + 1, -1);
+    if (found[dev] >= 0) return found[dev];
+    int best = 0;
+    cudaFuncSetAttribute((const void*)k_front, cudaFuncAttributeMaxDynamicSharedMemorySize, kPartSmemOne);
+    cudaFuncSetAttribute((const void*)k_front, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (int c = kClusterMaxBlocks; c >= 1 && best == 0; c >>= 1) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(c);
+        cfg.blockDim = dim3(kBlock);
+        cfg.dynamicSmemBytes = kPartSmemOne;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = c;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, (const void*)k_front, &cfg) == cudaSuccess && n > 0) best = c;
+        else cudaGetLastError();
+    }
+    found[dev] = best;
+    return best;
+}
+
+/* One block of 256 threads for each 128 proxies, a power of two up to 16: at least as many blocks as the
+ * part-local solve has parts (one for each 256 proxies), and enough threads that the passes over a
+ * world's contacts (two to six for each body) take a few rounds. */
+int cluster_size(const DevWorld& w) {
+    int c = 1;
+    while (c < kClusterMaxBlocks && c * 128 < w.n_fixtures) c <<= 1;
+    return c;
+}
+
+bool cluster_world(const DevWorld& w) {
+    return w.n_fixtures > 0 && w.n_fixtures <= kClusterMaxProxies && w.n_bodies <= 2 * kClusterMaxProxies &&
+           cluster_size(w) <= max_cluster();
+}
+
+int launch_front(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool parts, int passes) {
+    StepParams spc = sp;
+    spc.part_bodies = 0;
+    spc.part_slot_bytes = 0;
+    const bool local = use_parts(w, w.num_sms, parts);
+    const size_t smem = local && (passes & FRONT_SOLVE) ? part_smem(spc, kPartSmemOne) : 0;
+    B2G_LAUNCHED(1);
+    return launch_cluster(k_front, cluster_size(w), kBlock, smem, s, w, spc, local ? part_count(w, w.num_sms) : 0, passes);
+}
+
+void launch_phase_stamp(const DevWorld& w, int phase, cudaStream_t s) {
+    k_phase_stamp<<<1, 1, 0, s>>>(w, phase); B2G_LAUNCHED(1);
 }
 
 void launch_set_transform(const DevWorld& w, int body, float px, float py, float angle, cudaStream_t s) {
