@@ -37,6 +37,7 @@
 
 #include "../../include/b2g.h"
 #include "b2g_internal.h"
+#include "b2g_shape.cuh"
 #include "b2g_tape.h"
 
 using namespace b2g;
@@ -305,145 +306,6 @@ int bits_for(uint64_t v) {
     int b = 1;
     while ((1ull << b) <= v) ++b;
     return b;
-}
-
-/* ---- creation-time geometry (host) ---- */
-
-/* B2polygonShape::set_as_box, private/collision/b2_polygon_shape.rs:12-23 */
-void polygon_box(ShapeRec& s, float hx, float hy) {
-    s.v[0] = mk(-hx, -hy);
-    s.v[1] = mk(hx, -hy);
-    s.v[2] = mk(hx, hy);
-    s.v[3] = mk(-hx, hy);
-    s.n[0] = mk(0.0f, -1.0f);
-    s.n[1] = mk(1.0f, 0.0f);
-    s.n[2] = mk(0.0f, 1.0f);
-    s.n[3] = mk(-1.0f, 0.0f);
-    s.centroid = mk(0.0f, 0.0f);
-    s.meta = SHAPE_POLYGON | (4 << 8);
-}
-
-/* polygon centroid, b2_polygon_shape.rs:53-77 */
-V2 polygon_centroid(const V2* vs, int count) {
-    V2 c = mk(0.0f, 0.0f);
-    float area = 0.0f;
-    const V2 s = vs[0];
-    const float inv3 = 1.0f / 3.0f;
-    for (int i = 0; i < count; ++i) {
-        V2 p1 = sub(vs[0], s);
-        V2 p2 = sub(vs[i], s);
-        V2 p3 = (i + 1 < count) ? sub(vs[i + 1], s) : sub(vs[0], s);
-        V2 e1 = sub(p2, p1);
-        V2 e2 = sub(p3, p1);
-        float d = cross(e1, e2);
-        float tri = 0.5f * d;
-        area += tri;
-        c = add(c, scale(tri * inv3, add(add(p1, p2), p3)));
-    }
-    return add(scale(1.0f / area, c), s);
-}
-
-/* B2polygonShape::set (gift wrapping), b2_polygon_shape.rs:96-211; false -> unit box fallback */
-bool polygon_hull(ShapeRec& s, const b2g_vec2* in, int count) {
-    if (count < 3) {
-        polygon_box(s, 1.0f, 1.0f);
-        return false;
-    }
-    int n = count < kMaxPolygonVertices ? count : kMaxPolygonVertices;
-    V2 ps[kMaxPolygonVertices];
-    int temp = 0;
-    for (int i = 0; i < n; ++i) {
-        V2 v = mk(in[i].x, in[i].y);
-        bool unique = true;
-        for (int j = 0; j < temp; ++j) {
-            if (dist_sq(v, ps[j]) < ((0.5f * kLinearSlop) * (0.5f * kLinearSlop))) {
-                unique = false;
-                break;
-            }
-        }
-        if (unique) ps[temp++] = v;
-    }
-    n = temp;
-    if (n < 3) {
-        polygon_box(s, 1.0f, 1.0f);
-        return false;
-    }
-    int i0 = 0;
-    float x0 = ps[0].x;
-    for (int i = 1; i < n; ++i) {
-        float x = ps[i].x;
-        if (x > x0 || (x == x0 && ps[i].y < ps[i0].y)) {
-            i0 = i;
-            x0 = x;
-        }
-    }
-    int hull[kMaxPolygonVertices];
-    int m = 0, ih = i0;
-    for (;;) {
-        if (m >= kMaxPolygonVertices) {
-            polygon_box(s, 1.0f, 1.0f);
-            return false;
-        }
-        hull[m] = ih;
-        int ie = 0;
-        for (int j = 1; j < n; ++j) {
-            if (ie == ih) {
-                ie = j;
-                continue;
-            }
-            V2 r = sub(ps[ie], ps[hull[m]]);
-            V2 v = sub(ps[j], ps[hull[m]]);
-            float c = cross(r, v);
-            if (c < 0.0f) ie = j;
-            if (c == 0.0f && length_sq(v) > length_sq(r)) ie = j;
-        }
-        ++m;
-        ih = ie;
-        if (ie == i0) break;
-    }
-    if (m < 3) {
-        polygon_box(s, 1.0f, 1.0f);
-        return false;
-    }
-    for (int i = 0; i < m; ++i) s.v[i] = ps[hull[i]];
-    for (int i = 0; i < m; ++i) {
-        int i2 = (i + 1 < m) ? i + 1 : 0;
-        s.n[i] = cross_vs(sub(s.v[i2], s.v[i]), 1.0f);
-        normalize(s.n[i]);
-    }
-    s.centroid = polygon_centroid(s.v, m);
-    s.meta = SHAPE_POLYGON | (m << 8);
-    return true;
-}
-
-void build_shape(const b2g_fixture_def& d, ShapeRec& s) {
-    memset(&s, 0, sizeof(s));
-    s.radius = d.radius;
-    if (d.shape_type == B2G_SHAPE_CIRCLE) {
-        s.v[0] = mk(d.vertices[0].x, d.vertices[0].y);
-        s.meta = SHAPE_CIRCLE | (1 << 8);
-    } else if (d.shape_type == B2G_SHAPE_EDGE) {
-        for (int i = 0; i < 4; ++i) s.v[i] = mk(d.vertices[i].x, d.vertices[i].y);
-        s.meta = SHAPE_EDGE | (2 << 8) | ((d.one_sided ? 1 : 0) << 16);
-    } else {
-        if (d.polygon_mode == B2G_POLYGON_BOX) {
-            polygon_box(s, d.box_half_extents.x, d.box_half_extents.y);
-        } else if (d.polygon_mode == B2G_POLYGON_BOX_ORIENTED) {
-            /* set_as_box_angle, b2_polygon_shape.rs:25-50 */
-            polygon_box(s, d.box_half_extents.x, d.box_half_extents.y);
-            Xf xf;
-            xf.p = mk(d.box_center.x, d.box_center.y);
-            xf.q = rot(d.box_angle);
-            s.centroid = xf.p;
-            for (int i = 0; i < 4; ++i) {
-                s.v[i] = mul(xf, s.v[i]);
-                s.n[i] = mul(xf.q, s.n[i]);
-            }
-        } else {
-            polygon_hull(s, d.vertices, d.vertex_count);
-        }
-        s.radius = d.radius;
-    }
 }
 
 /* compute_mass of each shape: b2_polygon_shape.rs:314-390, b2_circle_shape.rs:79-86, b2_edge_shape.rs:126-132 */
@@ -3082,55 +2944,57 @@ int b2g_collide_pairs(const b2g_fixture_def* da, const float* xfa, const b2g_fix
 
 }  // extern "C"
 
+/* The definitions go to the device as they are and the shapes are built there (k_toi.cu). With coherent
+ * access to pageable memory (Grace) the kernels read the caller's arrays in place and write the results
+ * into its array; else they work on device copies. */
 int b2g_time_of_impact(const b2g_fixture_def* da, const b2g_sweep* swa, const b2g_fixture_def* db,
                        const b2g_sweep* swb, const float* t_max, int32_t n, b2g_toi_output* out) {
     if (n < 0 || (n > 0 && (!da || !db || !swa || !swb || !out))) return B2G_ERR_INVALID_ARG;
     if (n == 0) return B2G_OK;
-    std::vector<ShapeRec> sa(n), sb(n);
-    std::vector<float4> wa(2 * (size_t)n), wb(2 * (size_t)n);
-    for (int i = 0; i < n; ++i) {
-        for (const b2g_fixture_def* d : {&da[i], &db[i]})
-            if (d->shape_type != B2G_SHAPE_CIRCLE && d->shape_type != B2G_SHAPE_POLYGON && d->shape_type != B2G_SHAPE_EDGE)
-                return B2G_ERR_INVALID_ARG;
-        build_shape(da[i], sa[i]);
-        build_shape(db[i], sb[i]);
-        const b2g_sweep& a = swa[i];
-        const b2g_sweep& b = swb[i];
-        wa[2 * i] = make_float4(a.local_center.x, a.local_center.y, a.c0.x, a.c0.y);
-        wa[2 * i + 1] = make_float4(a.c.x, a.c.y, a.a0, a.a);
-        wb[2 * i] = make_float4(b.local_center.x, b.local_center.y, b.c0.x, b.c0.y);
-        wb[2 * i + 1] = make_float4(b.c.x, b.c.y, b.a0, b.a);
+    int dev = 0, in_place = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&in_place, cudaDevAttrPageableMemoryAccess, dev) != cudaSuccess)
+        return B2G_ERR_CUDA;
+    const cudaStream_t s = 0;
+    /* (an array off its type's alignment, which the device cannot load from, goes by way of a copy) */
+    const auto aligned = [](const void* a, const void* b, size_t to) { return (((uintptr_t)a | (uintptr_t)b) & (to - 1)) == 0; };
+    if (in_place && aligned(da, db, 8) && aligned(swa, swb, 4) && aligned(t_max, out, 4)) {
+        /* a page that is not mapped yet costs the device a fault: touch the results' pages here */
+        volatile char* page = (volatile char*)out;
+        const size_t bytes = (size_t)n * sizeof(b2g_toi_output);
+        for (size_t at = 0; at < bytes; at += 4096) page[at] = page[at];
+        page[bytes - 1] = page[bytes - 1];
+        int bad = 0;
+        launch_time_of_impact(da, swa, db, swb, t_max, n, out, &bad, s);
+        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) return B2G_ERR_CUDA;
+        return ((volatile int&)bad) ? B2G_ERR_INVALID_ARG : B2G_OK;
     }
-    ShapeRec *d_sa = nullptr, *d_sb = nullptr;
-    float4 *d_wa = nullptr, *d_wb = nullptr;
-    float* d_t = nullptr;
-    int2* d_out = nullptr;
-    int rc = B2G_OK;
-    if (cudaMalloc(&d_sa, n * sizeof(ShapeRec)) != cudaSuccess || cudaMalloc(&d_sb, n * sizeof(ShapeRec)) != cudaSuccess ||
-        cudaMalloc(&d_wa, 2 * n * sizeof(float4)) != cudaSuccess || cudaMalloc(&d_wb, 2 * n * sizeof(float4)) != cudaSuccess ||
-        cudaMalloc(&d_out, n * sizeof(int2)) != cudaSuccess || (t_max && cudaMalloc(&d_t, n * sizeof(float)) != cudaSuccess))
-        rc = B2G_ERR_OUT_OF_MEMORY;
-    if (rc == B2G_OK) {
-        cudaMemcpy(d_sa, sa.data(), n * sizeof(ShapeRec), cudaMemcpyHostToDevice);
-        cudaMemcpy(d_sb, sb.data(), n * sizeof(ShapeRec), cudaMemcpyHostToDevice);
-        cudaMemcpy(d_wa, wa.data(), 2 * n * sizeof(float4), cudaMemcpyHostToDevice);
-        cudaMemcpy(d_wb, wb.data(), 2 * n * sizeof(float4), cudaMemcpyHostToDevice);
-        if (t_max) cudaMemcpy(d_t, t_max, n * sizeof(float), cudaMemcpyHostToDevice);
-        launch_time_of_impact(d_sa, d_wa, d_sb, d_wb, d_t, n, d_out, 0);
-        std::vector<int2> res(n);
-        if (cudaMemcpy(res.data(), d_out, n * sizeof(int2), cudaMemcpyDeviceToHost) != cudaSuccess) rc = B2G_ERR_CUDA;
-        for (int i = 0; rc == B2G_OK && i < n; ++i) {
-            out[i].state = res[i].x;
-            memcpy(&out[i].t, &res[i].y, sizeof(float));
-        }
+    const void* in[5] = {da, swa, db, swb, t_max};
+    const size_t size[7] = {sizeof(b2g_fixture_def), sizeof(b2g_sweep), sizeof(b2g_fixture_def), sizeof(b2g_sweep),
+                            t_max ? sizeof(float) : 0, sizeof(b2g_toi_output), 0};
+    size_t at[7], total = 256;  /* the flag, then the arrays */
+    for (int k = 0; k < 6; ++k) {
+        at[k] = total;
+        total += (size[k] * (size_t)n + 255) & ~(size_t)255;
     }
-    cudaFree(d_sa);
-    cudaFree(d_sb);
-    cudaFree(d_wa);
-    cudaFree(d_wb);
-    cudaFree(d_t);
-    cudaFree(d_out);
-    return rc;
+    unsigned char* d = nullptr;
+    if (cudaMalloc((void**)&d, total) != cudaSuccess) {
+        cudaGetLastError();
+        return B2G_ERR_OUT_OF_MEMORY;
+    }
+    int bad = 0;
+    bool ok = cudaMemsetAsync(d, 0, sizeof(int), s) == cudaSuccess;
+    for (int k = 0; k < 5; ++k)
+        if (size[k]) ok = ok && cudaMemcpyAsync(d + at[k], in[k], size[k] * n, cudaMemcpyHostToDevice, s) == cudaSuccess;
+    if (ok) {
+        launch_time_of_impact((const b2g_fixture_def*)(d + at[0]), (const b2g_sweep*)(d + at[1]),
+                              (const b2g_fixture_def*)(d + at[2]), (const b2g_sweep*)(d + at[3]),
+                              t_max ? (const float*)(d + at[4]) : nullptr, n, (b2g_toi_output*)(d + at[5]), (int*)d, s);
+        ok = cudaMemcpy(&bad, d, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess;
+    }
+    if (ok && !bad) ok = cudaMemcpy(out, d + at[5], size[5] * n, cudaMemcpyDeviceToHost) == cudaSuccess;
+    cudaFree(d);
+    return !ok ? B2G_ERR_CUDA : bad ? B2G_ERR_INVALID_ARG : B2G_OK;
 }
 
 /* ---- allocation-free variant of b2g_collide_pairs ----

@@ -24,6 +24,7 @@
 
 #include <functional>
 
+#include "b2g.h"
 #include "b2g_collide.cuh"
 
 namespace b2g {
@@ -455,9 +456,10 @@ void launch_phase_stamp(const DevWorld& w, int phase, cudaStream_t s);
 /* parts: allow the part-local solve (used where the world's size suits it) */
 void launch_colouring(const DevWorld& w, cudaStream_t s, int num_sms, bool parts);
 int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms, bool parts);
-/* time of impact of n shape pairs (sweeps as 2 float4: (lc, c0), (c, a0, a)); out = (state, t bits) */
-void launch_time_of_impact(const ShapeRec* sa, const float4* swa, const ShapeRec* sb, const float4* swb,
-                           const float* t_max, int n, int2* out, cudaStream_t s);
+/* time of impact of n shape pairs; every pointer is memory the device reaches. A definition that is no
+ * circle, polygon or edge sets *bad, and no result is written then */
+void launch_time_of_impact(const b2g_fixture_def* da, const b2g_sweep* swa, const b2g_fixture_def* db,
+                           const b2g_sweep* swb, const float* t_max, int n, b2g_toi_output* out, int* bad, cudaStream_t s);
 /* continuous physics of a step (B2world::solve_toi) as one cooperative launch; returns a CUDA error */
 int launch_continuous(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms);
 /* whether the part-local solve applies to this world (parts allowed and the world's size suits it) */
