@@ -175,6 +175,8 @@ struct World {
     LaunchCfg cfg;
     bool cfg_set = false;    /* chosen by the user or the autotuner: no bucket lookup */
     bool pageable = false;   /* the device reads/writes pageable host memory coherently */
+    unsigned char* query_mem = nullptr;  /* device buffers of the world queries, kept between calls */
+    size_t query_bytes = 0;
     b2g_body_state* d_states = nullptr;  /* packing buffer for b2g_get_body_states otherwise */
     int d_states_cap = 0;
     /* b2g_get_body_states_async: two device snapshots, copied out on a second stream */
@@ -1566,6 +1568,7 @@ int b2g_world_destroy(void* p) {
     tape_free(w);
     if (w->d_states) cudaFree(w->d_states);
     free_all(w);
+    cudaFree(w->query_mem);
     cudaFree(w->d.stamps);
     cudaStreamDestroy(w->stream);
     delete w;
@@ -2951,14 +2954,14 @@ int b2g_time_of_impact(const b2g_fixture_def* da, const b2g_sweep* swa, const b2
                        const b2g_sweep* swb, const float* t_max, int32_t n, b2g_toi_output* out) {
     if (n < 0 || (n > 0 && (!da || !db || !swa || !swb || !out))) return B2G_ERR_INVALID_ARG;
     if (n == 0) return B2G_OK;
-    int dev = 0, in_place = 0;
+    int dev = 0, reachable = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&in_place, cudaDevAttrPageableMemoryAccess, dev) != cudaSuccess)
+        cudaDeviceGetAttribute(&reachable, cudaDevAttrPageableMemoryAccess, dev) != cudaSuccess)
         return B2G_ERR_CUDA;
     const cudaStream_t s = 0;
     /* (an array off its type's alignment, which the device cannot load from, goes by way of a copy) */
     const auto aligned = [](const void* a, const void* b, size_t to) { return (((uintptr_t)a | (uintptr_t)b) & (to - 1)) == 0; };
-    if (in_place && aligned(da, db, 8) && aligned(swa, swb, 4) && aligned(t_max, out, 4)) {
+    if (reachable && aligned(da, db, 8) && aligned(swa, swb, 4) && aligned(t_max, out, 4)) {
         /* a page that is not mapped yet costs the device a fault: touch the results' pages here */
         volatile char* page = (volatile char*)out;
         const size_t bytes = (size_t)n * sizeof(b2g_toi_output);
@@ -3177,6 +3180,65 @@ int b2g_get_solver_order(void* p, uint32_t* out, int32_t cap, int32_t* n) {
 
 /* ---- world queries ---- */
 
+namespace {
+
+/* Device buffers of one query call, pieces of an allocation the world keeps for the next call (it is freed
+ * with the world; a call that needed more than kQueryKeep bytes leaves none). The arrays themselves only
+ * where the device cannot reach the caller's. */
+struct QueryBuffers {
+    int* result;       /* status, total, the find's counter, the write's flag */
+    int2* lists;
+    uint32_t* found;
+    float* query;
+    uint32_t* world;
+    void* out;
+};
+constexpr size_t kQueryKeep = 64u << 20;
+
+int query_buffers(World* w, QueryBuffers& b, const float* query, const uint32_t* world, int n, int found, size_t out_bytes) {
+    const size_t size[6] = {4 * sizeof(int), found > 0 ? n * sizeof(int2) : 0, (size_t)found * sizeof(uint32_t),
+                            query ? n * 4 * sizeof(float) : 0, world ? n * sizeof(uint32_t) : 0, out_bytes};
+    size_t at[6], total = 0;
+    for (int k = 0; k < 6; ++k) {
+        at[k] = total;
+        total += (size[k] + 255) & ~(size_t)255;
+    }
+    if (w->query_bytes < total || (w->query_bytes > kQueryKeep && total <= kQueryKeep)) {
+        CUDA_OK(w, cudaStreamSynchronize(w->stream));
+        cudaFree(w->query_mem);
+        w->query_mem = nullptr;
+        w->query_bytes = 0;
+        if (cudaMalloc((void**)&w->query_mem, total) != cudaSuccess) {
+            cudaGetLastError();
+            w->query_mem = nullptr;
+            return fail(w, B2G_ERR_OUT_OF_MEMORY, "no memory for a query's buffers");
+        }
+        w->query_bytes = total;
+    }
+    unsigned char* m = w->query_mem;
+    b = {(int*)(m + at[0]), (int2*)(m + at[1]), (uint32_t*)(m + at[2]), (float*)(m + at[3]), world ? (uint32_t*)(m + at[4]) : nullptr,
+         m + at[5]};
+    if (query) CUDA_OK(w, cudaMemcpyAsync(b.query, query, size[3], cudaMemcpyHostToDevice, w->stream));
+    if (world) CUDA_OK(w, cudaMemcpyAsync(b.world, world, size[4], cudaMemcpyHostToDevice, w->stream));
+    return B2G_OK;
+}
+
+/* whether a query's arrays can be used where they are: the device reaches host memory, and all of them
+ * lie on 4-byte boundaries */
+bool in_place(const World* w, const void* a, const void* b, const void* c) {
+    return w->pageable && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 3u) == 0;
+}
+
+/* A page that is not mapped yet costs the device a fault: the host maps a result's pages before the
+ * kernels write them (the bytes keep their values). */
+void touch_pages(void* p, size_t bytes) {
+    volatile char* c = (volatile char*)p;
+    for (size_t at = 0; at < bytes; at += 4096) c[at] = c[at];
+    if (bytes) c[bytes - 1] = c[bytes - 1];
+}
+
+}  // namespace
+
 extern "C" {
 
 int b2g_ray_cast_closest(void* p, const float* rays, const uint32_t* world_index, int32_t n, b2g_ray_hit* out) {
@@ -3184,40 +3246,25 @@ int b2g_ray_cast_closest(void* p, const float* rays, const uint32_t* world_index
     if (!w || n < 0 || (n > 0 && (!rays || !out))) return B2G_ERR_INVALID_ARG;
     if (n == 0) return B2G_OK;
     if (!w->allocated || w->steps == 0) return fail(w, B2G_ERR_INVALID_ARG, "queries use the last step's hierarchy: step once first");
-    int rc = check_status(w);
-    if (rc != B2G_OK) return rc;
-    float4 *d_rays = nullptr, *d_a = nullptr, *d_b = nullptr;
-    uint32_t* d_world = nullptr;
     cudaStream_t s = w->stream;
-    cudaError_t e = cudaMalloc((void**)&d_rays, n * sizeof(float4));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&d_a, n * sizeof(float4));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&d_b, n * sizeof(float4));
-    if (e == cudaSuccess && world_index) e = cudaMalloc((void**)&d_world, n * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_rays, rays, n * sizeof(float4), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess && world_index)
-        e = cudaMemcpyAsync(d_world, world_index, n * sizeof(uint32_t), cudaMemcpyHostToDevice, s);
-    std::vector<float4> a(n), b(n);
-    if (e == cudaSuccess) {
-        launch_ray_cast(w->d, d_rays, d_world, n, d_a, d_b, s);
-        e = cudaGetLastError();
+    int status = 0;
+    if (in_place(w, rays, world_index, out)) {
+        touch_pages(out, (size_t)n * sizeof(b2g_ray_hit));
+        launch_ray_cast(w->d, rays, world_index, n, out, &status, s);
+        CUDA_OK(w, cudaGetLastError());
+        CUDA_OK(w, cudaStreamSynchronize(s));
+        return status_error(w, ((volatile int&)status));
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(a.data(), d_a, n * sizeof(float4), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(b.data(), d_b, n * sizeof(float4), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(d_rays);
-    cudaFree(d_a);
-    cudaFree(d_b);
-    if (d_world) cudaFree(d_world);
-    if (e != cudaSuccess) return fail(w, B2G_ERR_CUDA, cudaGetErrorString(e));
-    for (int i = 0; i < n; ++i) {
-        int f;
-        memcpy(&f, &a[i].x, 4);
-        out[i].fixture = f;
-        out[i].point = b2g_vec2{a[i].y, a[i].z};
-        out[i].normal = b2g_vec2{b[i].x, b[i].y};
-        out[i].fraction = b[i].z;
-    }
-    return check_status(w);
+    QueryBuffers b;
+    int rc = query_buffers(w, b, rays, world_index, n, 0, (size_t)n * sizeof(b2g_ray_hit));
+    if (rc != B2G_OK) return rc;
+    launch_ray_cast(w->d, b.query, b.world, n, (b2g_ray_hit*)b.out, b.result, s);
+    CUDA_OK(w, cudaGetLastError());
+    CUDA_OK(w, cudaMemcpyAsync(&status, b.result, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CUDA_OK(w, cudaStreamSynchronize(s));
+    if (!(status & ~ST_STACK_OVERFLOW))
+        CUDA_OK(w, cudaMemcpy(out, b.out, (size_t)n * sizeof(b2g_ray_hit), cudaMemcpyDeviceToHost));
+    return status_error(w, status);
 }
 
 int b2g_query_aabb(void* p, const float* boxes, const uint32_t* world_index, int32_t n, uint32_t* out_pairs,
@@ -3228,46 +3275,58 @@ int b2g_query_aabb(void* p, const float* boxes, const uint32_t* world_index, int
     *out_count = 0;
     if (n == 0) return B2G_OK;
     if (!w->allocated || w->steps == 0) return fail(w, B2G_ERR_INVALID_ARG, "queries use the last step's hierarchy: step once first");
-    int rc = check_status(w);
-    if (rc != B2G_OK) return rc;
-    const int cap = capacity > 0 ? capacity : 1;
-    float4* d_boxes = nullptr;
-    uint32_t* d_world = nullptr;
-    uint2* d_out = nullptr;
-    int* d_count = nullptr;
     cudaStream_t s = w->stream;
-    cudaError_t e = cudaMalloc((void**)&d_boxes, n * sizeof(float4));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&d_out, (size_t)cap * sizeof(uint2));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&d_count, sizeof(int));
-    if (e == cudaSuccess && world_index) e = cudaMalloc((void**)&d_world, n * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_boxes, boxes, n * sizeof(float4), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess && world_index)
-        e = cudaMemcpyAsync(d_world, world_index, n * sizeof(uint32_t), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_count, 0, sizeof(int), s);
-    if (e == cudaSuccess) {
-        launch_query_aabb(w->d, d_boxes, d_world, n, d_out, cap, d_count, s);
-        e = cudaGetLastError();
+    const bool direct = in_place(w, boxes, world_index, out_pairs);
+    /* the lists find room for 16 fixtures a box, then for what a first pass counted */
+    int room = (int)std::min<long long>(1 << 24, 16LL * n);
+    for (int pass = 0;; ++pass) {
+        QueryBuffers b;
+        int rc = query_buffers(w, b, direct ? nullptr : boxes, direct ? nullptr : world_index, n, room, 0);
+        if (rc != B2G_OK) return rc;
+        int got[2] = {0, 0};  /* status, total */
+        CUDA_OK(w, cudaMemsetAsync(b.result, 0, 4 * sizeof(int), s));
+        launch_query_find(w->d, direct ? boxes : b.query, direct ? world_index : b.world, n, b.found, room, b.lists,
+                          b.result + 2, direct ? got : b.result, s);
+        CUDA_OK(w, cudaGetLastError());
+        if (!direct) CUDA_OK(w, cudaMemcpyAsync(got, b.result, sizeof(got), cudaMemcpyDeviceToHost, s));
+        CUDA_OK(w, cudaStreamSynchronize(s));
+        const int status = ((volatile int*)got)[0], total = ((volatile int*)got)[1];
+        if (status & ~ST_STACK_OVERFLOW) return status_error(w, status);
+        *out_count = total;
+        if (total > capacity) {
+            status_error(w, status);
+            return fail(w, B2G_ERR_CAPACITY, "more overlaps than capacity; *out_count holds the total");
+        }
+        if (total > room) {
+            room = total;
+            continue;
+        }
+        int unsorted = 0;
+        const size_t bytes = 2 * (size_t)total * sizeof(uint32_t);
+        if (direct) {
+            touch_pages(out_pairs, bytes);
+            launch_query_write(w->d, n, b.found, b.lists, out_pairs, &unsorted, s);
+            CUDA_OK(w, cudaGetLastError());
+            CUDA_OK(w, cudaStreamSynchronize(s));
+            unsorted = ((volatile int&)unsorted);
+        } else if (total > 0) {
+            uint32_t* pairs = nullptr;
+            CUDA_OK(w, cudaMalloc((void**)&pairs, bytes));
+            launch_query_write(w->d, n, b.found, b.lists, pairs, b.result + 3, s);
+            cudaError_t e = cudaMemcpyAsync(&unsorted, b.result + 3, sizeof(int), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            if (e == cudaSuccess) e = cudaMemcpy(out_pairs, pairs, bytes, cudaMemcpyDeviceToHost);
+            cudaFree(pairs);
+            CUDA_OK(w, e);
+        }
+        if (unsorted) {
+            std::vector<std::pair<uint32_t, uint32_t>> pairs((size_t)total);
+            memcpy(pairs.data(), out_pairs, bytes);
+            std::sort(pairs.begin(), pairs.end());
+            memcpy(out_pairs, pairs.data(), bytes);
+        }
+        return status_error(w, status);
     }
-    int total = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&total, d_count, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    std::vector<uint2> pairs(std::min(total, cap > 0 ? cap : 0));
-    if (e == cudaSuccess && !pairs.empty())
-        e = cudaMemcpy(pairs.data(), d_out, pairs.size() * sizeof(uint2), cudaMemcpyDeviceToHost);
-    cudaFree(d_boxes);
-    cudaFree(d_out);
-    cudaFree(d_count);
-    if (d_world) cudaFree(d_world);
-    if (e != cudaSuccess) return fail(w, B2G_ERR_CUDA, cudaGetErrorString(e));
-    *out_count = total;
-    if (total > capacity) return fail(w, B2G_ERR_CAPACITY, "more overlaps than capacity; *out_count holds the total");
-    std::sort(pairs.begin(), pairs.end(),
-              [](const uint2& x, const uint2& y) { return x.x != y.x ? x.x < y.x : x.y < y.y; });
-    for (size_t i = 0; i < pairs.size(); ++i) {
-        out_pairs[2 * i] = pairs[i].x;
-        out_pairs[2 * i + 1] = pairs[i].y;
-    }
-    return check_status(w);
 }
 
 }  // extern "C"

@@ -476,11 +476,18 @@ void launch_clear_forces(const DevWorld& w, cudaStream_t s);
 void launch_collide_pairs(const ShapeRec* a, const float4* xa, const ShapeRec* b, const float4* xb, const int* kind,
                           int n, float4* geo, float4* pts, uint4* ids, cudaStream_t s);
 
-/* world queries on the last step's LBVH (k_query.cu) */
-void launch_ray_cast(const DevWorld& w, const float4* rays, const uint32_t* ray_world, int n, float4* out_a,
-                     float4* out_b, cudaStream_t s);
-void launch_query_aabb(const DevWorld& w, const float4* boxes, const uint32_t* box_world, int n, uint2* out, int cap,
-                       int* count, cudaStream_t s);
+/* World queries on the last step's LBVH (k_query.cu). Every pointer is memory the device reaches; the
+ * last kernel of a call writes the world's status word (and the total) to status / status_total. */
+void launch_ray_cast(const DevWorld& w, const float* rays, const uint32_t* ray_world, int n, b2g_ray_hit* out, int* status,
+                     cudaStream_t s);
+/* found: the boxes' fixtures, box by box in no order, lists[i] = (first entry, entries) of box i; written only
+ * while they fit cap. *total (zero before) counts all */
+void launch_query_find(const DevWorld& w, const float* boxes, const uint32_t* box_world, int n, uint32_t* found, int cap,
+                       int2* lists, int* total, int* status_total, cudaStream_t s);
+/* out: (box, fixture) pairs sorted by box then fixture, but for lists of more than 1024 fixtures, which
+ * are left as found (*unsorted is then set) */
+void launch_query_write(const DevWorld& w, int n, const uint32_t* found, const int2* lists, uint32_t* out, int* unsorted,
+                        cudaStream_t s);
 
 /* primitives (k_prims.cu) */
 void scan_exclusive_u32(const uint32_t* in, uint32_t* out, const int* d_n, int max_n, uint32_t* tmp, int* d_total,
@@ -510,6 +517,18 @@ inline int grid_for(int n, int block, int max_blocks) {
     int g = (n + block - 1) / block;
     if (g < 1) g = 1;
     return g < max_blocks ? g : max_blocks;
+}
+
+/* Lanes of a warp that take an item each, in a kernel whose items are long serial chains of unlike length
+ * and branches (a ray's walk, a time of impact): a warp runs all of its lanes' branches one after
+ * another, so while there are fewer items than the GPU has warps for (about 16 an SM) an item does best
+ * nearly alone in its warp. A power of two. With full warps 16k rays took 195 us (134 so, 203 with 4 warps
+ * an SM, 119 with 64), 500 times of impact 139 us (93 so) and 20k of them 223 us (228; 385 with 64 warps). */
+constexpr int kLanesWarps = 16;
+inline int lanes_for(int n, int num_sms) {
+    int per = 1;
+    while (per < 32 && (long long)per * num_sms * kLanesWarps < n) per <<= 1;
+    return per;
 }
 
 }  // namespace b2g

@@ -7,8 +7,11 @@
  * (private/collision/b2_polygon_shape.rs:226-287) and B2edgeShape
  * (private/collision/b2_edge_shape.rs:39-102).
  *
- * One thread per query walks the hierarchy built by the last step's broadphase (fat AABBs as of
- * that step). A ray keeps the reference's clipping: every hit clips the segment to its fraction,
+ * The hierarchy walked is the one of the last step's broadphase (fat AABBs as of that step): a thread
+ * for each ray, a warp for each box. The queries and their results are the caller's arrays where the
+ * device reaches them (Grace's coherent access), so a call is its kernels and a wait: 16k rays and 2k
+ * boxes against 20k bodies take 134 + 50 us, and took 373 + 887 us with an allocation for every array,
+ * host loops over the results and a host sort of the boxes' pairs. A ray keeps the reference's clipping: every hit clips the segment to its fraction,
  * so the result is the closest hit; only the order in which equally distant fixtures are met can
  * differ from the reference's tree (the GPU keeps the first it meets).
  */
@@ -120,13 +123,16 @@ __device__ __forceinline__ Xf body_xf(const DevWorld& w, int b) {
     return xf;
 }
 
-/* one thread per ray: out_a = (fixture as int bits or -1, point x, point y, -),
- * out_b = (normal x, normal y, fraction, -) */
-__global__ void __launch_bounds__(kBlock) k_ray_cast(DevWorld w, const float4* rays, const uint32_t* ray_world, int n,
-                                                     float4* out_a, float4* out_b) {
-    B2G_RETURN_IF_ABORTED(w);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 ray = rays[i];
+/* one thread per ray, `per` rays to a warp (lanes_for). A world whose status holds an error answers
+ * nothing: the caller reports it */
+__global__ void __launch_bounds__(kBlock) k_ray_cast(DevWorld w, const float* rays, const uint32_t* ray_world, int n,
+                                                     int per, b2g_ray_hit* out) {
+    if (((volatile int*)w.cnt)[CNT_STATUS] & ~ST_STACK_OVERFLOW) return;
+    const int lane = threadIdx.x & 31, warps = (int)blockDim.x >> 5;
+    if (lane >= per) return;
+    for (int i = (blockIdx.x * warps + ((int)threadIdx.x >> 5)) * per + lane; i < n; i += gridDim.x * warps * per) {
+        const float4 ray = make_float4(rays[4 * (size_t)i], rays[4 * (size_t)i + 1], rays[4 * (size_t)i + 2],
+                                       rays[4 * (size_t)i + 3]);
         const V2 p1 = mk(ray.x, ray.y), p2 = mk(ray.z, ray.w);
         int hit = -1;
         V2 hit_point = mk(0.0f, 0.0f), hit_normal = mk(0.0f, 0.0f);
@@ -182,60 +188,178 @@ __global__ void __launch_bounds__(kBlock) k_ray_cast(DevWorld w, const float4* r
                 }
             }
         }
-        out_a[i] = make_float4(__int_as_float(hit), hit_point.x, hit_point.y, 0.0f);
-        out_b[i] = make_float4(hit_normal.x, hit_normal.y, hit_fraction, 0.0f);
+        b2g_ray_hit h;
+        h.fixture = hit;
+        h.point = b2g_vec2{hit_point.x, hit_point.y};
+        h.normal = b2g_vec2{hit_normal.x, hit_normal.y};
+        h.fraction = hit_fraction;
+        out[i] = h;
     }
 }
 
-/* one thread per box: every fixture whose fat AABB overlaps it, as (query, fixture) pairs */
-__global__ void __launch_bounds__(kBlock) k_query_aabb(DevWorld w, const float4* boxes, const uint32_t* box_world,
-                                                       int n, uint2* out, int cap, int* count) {
-    B2G_RETURN_IF_ABORTED(w);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 q = boxes[i];
-        const uint32_t wd = box_world ? box_world[i] : 0u;
-        if (wd >= (uint32_t)w.num_worlds) continue;
-        auto emit = [&](int p) {
-            const int slot = atomicAdd(count, 1);
-            if (slot < cap) out[slot] = make_uint2((uint32_t)i, w.bp_val[p]);
-        };
-        for (int h = 0; h < 2; ++h) {
-            const int root = w.bp_world_root[wd + (h ? (uint32_t)w.num_worlds : 0u)];
-            if (root == INT_MIN) continue;
-            if (root < 0) {
-                if (aabb_overlap(w.bp_leaf[~root], q)) emit(~root);
-                continue;
-            }
-            int stack[kStack];
-            int top = 0;
-            stack[top++] = root;
-            while (top > 0) {
-                const int node = stack[--top];
-                const int2 ch = w.bp_node_child[node];
-                const float4 bx[2] = {w.bp_node_b0[node], w.bp_node_b1[node]};
-                const int kids[2] = {ch.x, ch.y};
-                for (int c = 0; c < 2; ++c) {
-                    if (!aabb_overlap(bx[c], q)) continue;
-                    if (kids[c] < 0) emit(~kids[c]);
-                    else if (top < kStack) stack[top++] = kids[c];
-                    else atomicOr((unsigned*)&w.cnt[CNT_STATUS], ST_STACK_OVERFLOW);
-                }
-            }
-        }
+/* The fixtures whose fat AABBs overlap each box, in two kernels. k_query_find: a warp walks the hierarchy
+ * for its box (up to 32 pending nodes a round, from a stack in shared memory) and keeps what it finds in shared
+ * memory; the box's list then goes to a piece of `found` that it reserves with one atomic (a longer list
+ * than fits is written by a second walk). lists[i] = (first entry, entries); *total counts all of them,
+ * written or not. k_query_write: the lists in the order of the boxes, each by fixture. */
+constexpr int kBoxWarps = 4;
+constexpr int kFoundMax = 256;   /* a box's fixtures kept in shared memory */
+constexpr int kPendMax = 512;    /* pending nodes of a walk */
+constexpr int kPendWide = 384;   /* above so many a round pops one node, a depth-first walk that adds at
+                                    most one pending node for each level below it */
+constexpr int kRankMax = 1024;   /* longer lists are left to the host to sort */
+
+/* one walk: found(leaf) for the lanes whose leaf overlaps q (called by the whole warp, ok: this lane has
+ * one) */
+template <typename Found>
+__device__ __forceinline__ void walk_box(const DevWorld& w, float4 q, uint32_t wd, int* pend, Found found) {
+    const int lane = threadIdx.x & 31;
+    const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
+    int top = 0;
+    for (int h = 0; h < 2; ++h) {
+        const int root = w.bp_world_root[wd + (h ? (uint32_t)w.num_worlds : 0u)];
+        if (root == INT_MIN) continue;
+        if (root < 0) found(lane == 0 && aabb_overlap(w.bp_leaf[~root], q), ~root);
+        else if (lane == 0) pend[top] = root;
+        top += root >= 0 ? 1 : 0;
     }
+    __syncwarp();
+    while (top > 0) {
+        const int take = min(top, top <= kPendWide ? 32 : 1);
+        const bool mine = lane < take;
+        const int node = mine ? pend[top - 1 - lane] : 0;
+        top -= take;
+        __syncwarp();
+        int kids[2] = {0, 0};
+        bool hit[2] = {false, false};
+        if (mine) {
+            const int2 ch = w.bp_node_child[node];
+            kids[0] = ch.x;
+            kids[1] = ch.y;
+            hit[0] = aabb_overlap(w.bp_node_b0[node], q);
+            hit[1] = aabb_overlap(w.bp_node_b1[node], q);
+        }
+        for (int c = 0; c < 2; ++c) {
+            const bool leaf = hit[c] && kids[c] < 0, inner = hit[c] && kids[c] >= 0;
+            if (__any_sync(full, leaf)) found(leaf, ~kids[c]);
+            const unsigned in = __ballot_sync(full, inner);
+            const int at = top + __popc(in & below);
+            if (inner && at < kPendMax) pend[at] = kids[c];
+            if (inner && at >= kPendMax) atomicOr((unsigned*)&w.cnt[CNT_STATUS], ST_STACK_OVERFLOW);
+            top = min(top + __popc(in), kPendMax);
+        }
+        __syncwarp();
+    }
+}
+
+__global__ void __launch_bounds__(32 * kBoxWarps) k_query_find(DevWorld w, const float* boxes, const uint32_t* box_world,
+                                                               int n, uint32_t* found, int cap, int2* lists, int* total) {
+    if (((volatile int*)w.cnt)[CNT_STATUS] & ~ST_STACK_OVERFLOW) return;
+    __shared__ int s_pend[kBoxWarps][kPendMax];
+    __shared__ uint32_t s_found[kBoxWarps][kFoundMax];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    for (int i = blockIdx.x * kBoxWarps + wid; i < n; i += gridDim.x * kBoxWarps) {
+        const float v = lane < 4 ? boxes[4 * (size_t)i + lane] : 0.0f;
+        const float4 q = make_float4(__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 1),
+                                     __shfl_sync(0xffffffffu, v, 2), __shfl_sync(0xffffffffu, v, 3));
+        const uint32_t wd = box_world ? box_world[i] : 0u;
+        int count = 0;
+        if (wd < (uint32_t)w.num_worlds)
+            walk_box(w, q, wd, s_pend[wid], [&](bool ok, int p) {
+                const unsigned who = __ballot_sync(0xffffffffu, ok);
+                const int at = count + __popc(who & below);
+                if (ok && at < kFoundMax) s_found[wid][at] = w.bp_val[p];
+                count += __popc(who);
+            });
+        __syncwarp();
+        int first = 0;
+        if (lane == 0) {
+            first = count > 0 ? atomicAdd(total, count) : 0;
+            lists[i] = make_int2(first, count);
+        }
+        first = __shfl_sync(0xffffffffu, first, 0);
+        if (first > cap - count) continue;  /* the caller learns the total and asks again with room for it */
+        if (count <= kFoundMax) {
+            for (int k = lane; k < count; k += 32) found[first + k] = s_found[wid][k];
+        } else {
+            int done = 0;
+            walk_box(w, q, wd, s_pend[wid], [&](bool ok, int p) {
+                const unsigned who = __ballot_sync(0xffffffffu, ok);
+                if (ok) found[first + done + __popc(who & below)] = w.bp_val[p];
+                done += __popc(who);
+            });
+        }
+        __syncwarp();
+    }
+}
+
+/* A block of 8 warps takes 8 boxes at a time; their lists start after all those of the boxes before,
+ * whose entries the block adds up itself. *unsorted: a list longer than kRankMax was written as found */
+__global__ void __launch_bounds__(256) k_query_write(int n, const uint32_t* found, const int2* lists, uint32_t* out,
+                                                     int* unsorted) {
+    __shared__ int s_sum[8];
+    __shared__ int s_count[8];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int before = 0, next = 0;  /* entries of the boxes before `next` */
+    for (int base = blockIdx.x * 8; base < n; base += gridDim.x * 8) {
+        int sum = 0;
+        for (int i = next + threadIdx.x; i < base; i += 256) sum += lists[i].y;
+        next = base;
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        __syncthreads();
+        const int i = base + wid;
+        const int2 list = i < n ? lists[i] : make_int2(0, 0);
+        if (lane == 0) {
+            s_sum[wid] = sum;
+            s_count[wid] = list.y;
+        }
+        __syncthreads();
+        for (int k = 0; k < 8; ++k) before += s_sum[k];
+        int at = before;
+        for (int k = 0; k < wid; ++k) at += s_count[k];
+        const uint32_t* f = found + list.x;
+        for (int k = lane; k < list.y; k += 32) {
+            const uint32_t mine = f[k];
+            int rank = k;
+            if (list.y <= kRankMax) {
+                rank = 0;
+                for (int j = 0; j < list.y; ++j) rank += f[j] < mine ? 1 : 0;
+            }
+            out[2 * (size_t)(at + rank)] = (uint32_t)i;
+            out[2 * (size_t)(at + rank) + 1] = mine;
+        }
+        if (lane == 0 && list.y > kRankMax) *(volatile int*)unsorted = 1;
+    }
+}
+
+/* the status word, and a count if there is one, where the host reads them */
+__global__ void k_query_end(DevWorld w, const int* total, int* out) {
+    out[0] = ((volatile int*)w.cnt)[CNT_STATUS];
+    if (total) out[1] = *total;
 }
 
 }  // namespace
 
-void launch_ray_cast(const DevWorld& w, const float4* rays, const uint32_t* ray_world, int n, float4* out_a,
-                     float4* out_b, cudaStream_t s) {
-    k_ray_cast<<<grid_for(n, kBlock, w.num_sms * 16), kBlock, 0, s>>>(w, rays, ray_world, n, out_a, out_b);
-    B2G_LAUNCHED(1);
+void launch_ray_cast(const DevWorld& w, const float* rays, const uint32_t* ray_world, int n, b2g_ray_hit* out, int* status,
+                     cudaStream_t s) {
+    const int per = lanes_for(n, w.num_sms);
+    k_ray_cast<<<grid_for(n, kBlock / 32 * per, w.num_sms * 16), kBlock, 0, s>>>(w, rays, ray_world, n, per, out);
+    k_query_end<<<1, 1, 0, s>>>(w, nullptr, status);
+    B2G_LAUNCHED(2);
 }
 
-void launch_query_aabb(const DevWorld& w, const float4* boxes, const uint32_t* box_world, int n, uint2* out, int cap,
-                       int* count, cudaStream_t s) {
-    k_query_aabb<<<grid_for(n, kBlock, w.num_sms * 16), kBlock, 0, s>>>(w, boxes, box_world, n, out, cap, count);
+void launch_query_find(const DevWorld& w, const float* boxes, const uint32_t* box_world, int n, uint32_t* found, int cap,
+                       int2* lists, int* total, int* status_total, cudaStream_t s) {
+    k_query_find<<<grid_for(n, kBoxWarps, w.num_sms * 16), 32 * kBoxWarps, 0, s>>>(w, boxes, box_world, n, found, cap,
+                                                                                  lists, total);
+    k_query_end<<<1, 1, 0, s>>>(w, total, status_total);
+    B2G_LAUNCHED(2);
+}
+
+void launch_query_write(const DevWorld& w, int n, const uint32_t* found, const int2* lists, uint32_t* out, int* unsorted,
+                        cudaStream_t s) {
+    k_query_write<<<grid_for(n, 8, w.num_sms * 8), 256, 0, s>>>(n, found, lists, out, unsorted);
     B2G_LAUNCHED(1);
 }
 

@@ -12,7 +12,7 @@
  *
  * The caller's arrays (144-byte definitions, 40-byte sweeps) are read as they are, and the shapes
  * (gift-wrapped hulls among them) are built by the pair's thread: 100k pairs take 0.60 ms with the call's
- * overheads, where a host loop over the shapes, copies and allocations took 10.7 ms. A block reads its 128 definitions in one contiguous piece into shared memory
+ * overheads, where a host loop over the shapes, copies and allocations took 10.7 ms. A block reads its definitions (up to 128) in one contiguous piece into shared memory
  * (8 bytes a thread, coalesced: the array may lie in host memory, across C2C) and every thread takes
  * its own from there, rows an odd number of words apart so that lanes meet different banks.
  */
@@ -75,12 +75,16 @@ __device__ __forceinline__ Sweep sweep_of(const uint32_t* row) {
 
 __global__ void __launch_bounds__(kBlock) k_time_of_impact(const b2g_fixture_def* da, const b2g_sweep* swa,
                                                            const b2g_fixture_def* db, const b2g_sweep* swb,
-                                                           const float* t_max, int n, b2g_toi_output* out, const int* bad) {
+                                                           const float* t_max, int n, int per, b2g_toi_output* out,
+                                                           const int* bad) {
     __shared__ uint32_t s_rows[kBlock * kDefRow];
     static_assert(kDefRow >= 2 * kSweepRow, "two sweeps fit a definition's row");
     if (__syncthreads_or(threadIdx.x == 0 && *(const volatile int*)bad != 0)) return;
-    for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const int m = min((int)blockDim.x, n - base), t = threadIdx.x;
+    /* `per` pairs to a warp (lanes_for); a lane without one only helps to fetch */
+    const int items = kBlock / 32 * per;
+    const int t = (int)(threadIdx.x & 31) < per ? (int)(threadIdx.x >> 5) * per + (int)(threadIdx.x & 31) : kBlock;
+    for (int base = blockIdx.x * items; base < n; base += gridDim.x * items) {
+        const int m = min(items, n - base);
         DistProxy pa, pb;
         Sweep a, b;
         __syncthreads();
@@ -114,7 +118,8 @@ void launch_time_of_impact(const b2g_fixture_def* da, const b2g_sweep* swa, cons
                            const b2g_sweep* swb, const float* t_max, int n, b2g_toi_output* out, int* bad, cudaStream_t s) {
     const int sms = current_sm_count();
     k_toi_check<<<grid_for(n, kBlock, sms * 8), kBlock, 0, s>>>(da, db, n, bad);
-    k_time_of_impact<<<grid_for(n, kBlock, sms * 16), kBlock, 0, s>>>(da, swa, db, swb, t_max, n, out, bad);
+    const int per = lanes_for(n, sms);
+    k_time_of_impact<<<grid_for(n, kBlock / 32 * per, sms * 16), kBlock, 0, s>>>(da, swa, db, swb, t_max, n, per, out, bad);
     B2G_LAUNCHED(2);
 }
 
