@@ -92,6 +92,7 @@ enum {
     CNT_TOUCHING = 11,
     CNT_BOUNDS = 12,      /* 4 ints: ordered-int min.x, min.y, max.x, max.y of proxy centres */
     CNT_BARRIER = 16,     /* grid barrier arrivals of the running cooperative launch (zeroed per launch) */
+    CNT_BARRIER2 = 17,    /* the same for every second one, so that a kernel can zero the next one's word */
     CNT_ISLANDS = 18,
     CNT_COLOURINGS = 19,  /* colourings done so far: the stamp of colours kept in contacts (mids.w) */
     CNT_DYN_EXTENT = 20,  /* largest half-extent of a dynamic body's fat AABB (float bits), this pass */
@@ -497,11 +498,13 @@ void radix_sort_pairs(unsigned long long* key_a, uint32_t* val_a, unsigned long 
                       const int* d_n, int max_n, int bits, uint32_t* hist, cudaStream_t s);
 /* the same sort as one cooperative launch (2 grid barriers per 8-bit pass; inputs of at most
  * 2048 items are sorted by a single block, inputs of at most 8192 by a rank count in three small
- * kernels); uses cnt's barrier words. zero_or_max: the count is known to be 0 or max_n (no
+ * kernels). The caller has zeroed cnt[barrier_word] (the launch's grid barriers) and, unless zero_or_max
+ * and max_n > kSortRankWords, hist[0, kSortRankWords). zero_or_max: the count is known to be 0 or max_n (no
  * rank-count launches when max_n is large). */
+constexpr int kSortRankWords = 8192;
 void radix_sort_pairs_coop(unsigned long long* key_a, uint32_t* val_a, unsigned long long* key_b, uint32_t* val_b,
                            const int* d_n, int max_n, int bits, uint32_t* hist, int* cnt, cudaStream_t s, int num_sms,
-                           bool zero_or_max = false);
+                           int barrier_word, bool zero_or_max = false);
 size_t radix_sort_hist_size(int max_n);
 size_t scan_tmp_size(int max_n);
 

@@ -1,8 +1,9 @@
 /*
  * b2g_sync.cuh — grid-wide barrier for the cooperative (persistent) kernels.
  *
- * Counting barrier over the co-resident blocks of a cooperative launch. The launcher zeroes the
- * counter before every launch (a memset node in the step graph), so the k-th barrier of the
+ * Counting barrier over the co-resident blocks of a cooperative launch. The counter is one of two words
+ * (CNT_BARRIER, CNT_BARRIER2), zero when the kernel starts: zeroed by a kernel that ran before it and after
+ * the word's last user, or by the launcher (a memset), so the k-th barrier of the
  * launch completes when the counter reaches (k + 1) x gridDim.x. Thread 0 of each block keeps k in
  * shared memory, arrives with one fire-and-forget release add and polls the counter with acquire
  * loads; nobody resets anything, so the last block to arrive waits for no extra round trip, and a
@@ -64,12 +65,17 @@ __device__ __forceinline__ void cluster_barrier() {
 static __shared__ unsigned b2g_barrier_epoch;
 static __shared__ long long b2g_barrier_limit;
 static __shared__ unsigned b2g_barrier_hold;
+static __shared__ int b2g_barrier_word;
 
-__device__ __forceinline__ void grid_barrier_start() {
-    if (threadIdx.x == 0) b2g_barrier_epoch = 0u;  /* ordered by the barrier's first __syncthreads */
+/* word: the launch's counter, CNT_BARRIER or CNT_BARRIER2 */
+__device__ __forceinline__ void grid_barrier_start(int word = CNT_BARRIER) {
+    if (threadIdx.x == 0) {  /* ordered by the barrier's first __syncthreads */
+        b2g_barrier_epoch = 0u;
+        b2g_barrier_word = word;
+    }
 }
 
-/* cnt: the counter block (uses CNT_BARRIER, zeroed by the launcher, and CNT_STATUS) */
+/* cnt: the counter block (uses the launch's counter and CNT_STATUS) */
 __device__ __forceinline__ bool grid_barrier(int* cnt) {
     __shared__ int s_ok;
     if (cluster_blocks() == gridDim.x) {
@@ -86,7 +92,7 @@ __device__ __forceinline__ bool grid_barrier(int* cnt) {
             b2g_barrier_limit = lim_hold.x > 0 ? (long long)lim_hold.x << 10 : 2000000000LL;
             b2g_barrier_hold = (unsigned)max(lim_hold.y, 0);
         }
-        unsigned* count = (unsigned*)&cnt[CNT_BARRIER];
+        unsigned* count = (unsigned*)&cnt[b2g_barrier_word];
         const unsigned target = (b2g_barrier_epoch + 1u) * gridDim.x + b2g_barrier_hold;
         ++b2g_barrier_epoch;
         red_release_add_gpu(count, 1u);

@@ -102,6 +102,7 @@ __global__ void k_bp_decide(DevWorld w, int mode, int ends) {
     pdl_entry();
     B2G_RETURN_IF_ABORTED(w);
     phase_stamp(w, ends);
+    if (blockIdx.x == 0 && threadIdx.x == 0) w.cnt[CNT_BARRIER] = w.cnt[CNT_BARRIER2] = 0;  /* the two sorts' */
     bp_decide(w, mode);
 }
 
@@ -716,13 +717,14 @@ __global__ void __launch_bounds__(kBlock) k_bp_traverse(DevWorld w, StepParams s
     bp_traverse(w, sp);
 }
 
-/* the moved flags are consumed; the colouring's rank weights start from zero (they are indexed by
+/* the moved flags are consumed; the new keys' sort counts from zero; the colouring's rank weights start from zero (they are indexed by
  * Morton rank, of which there are as many as proxies) */
 __device__ __forceinline__ void bp_clear_moved(const DevWorld& w) {
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < w.n_fixtures; f += gridDim.x * blockDim.x) {
         w.f_moved[f] = 0;
         w.rank_x[f] = 0ull;
     }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kSortRankWords; i += gridDim.x * blockDim.x) w.sort_hist[i] = 0u;
 }
 __global__ void k_bp_clear_moved(DevWorld w) {
     pdl_entry();
@@ -952,10 +954,11 @@ void launch_broadphase(const DevWorld& w, const StepParams& sp, cudaStream_t s, 
     const int gf = grid_for(n, kBlock, num_sms * 8);
     launch_pdl(k_bp_decide, 1, 32, 0, s, w, mode, ends); B2G_LAUNCHED(1);
     if (n > 0) {
+        if (n <= kSortRankWords) cudaMemsetAsync(w.sort_hist, 0, kSortRankWords * sizeof(uint32_t), s);
         launch_pdl(k_bp_bounds, gf, kBlock, 0, s, w); B2G_LAUNCHED(1);
         launch_pdl(k_bp_keys, gf, kBlock, 0, s, w); B2G_LAUNCHED(1);
         radix_sort_pairs_coop(w.bp_key, w.bp_val, w.bp_key_alt, w.bp_val_alt, &w.cnt[CNT_BP_SORT_N], n,
-                              kMortonBits + w.morton_world_bits, w.sort_hist, w.cnt, s, num_sms, true);
+                              kMortonBits + w.morton_world_bits, w.sort_hist, w.cnt, s, num_sms, CNT_BARRIER, true);
         launch_pdl(k_bp_build, gf, kBlock, 0, s, w); B2G_LAUNCHED(1);
         launch_pdl(k_bp_refit, gf, kBlock, 0, s, w); B2G_LAUNCHED(1);
         if (n > 1) {
@@ -967,10 +970,11 @@ void launch_broadphase(const DevWorld& w, const StepParams& sp, cudaStream_t s, 
         launch_pdl(k_bp_traverse, grid_for(n, tb, num_sms * 2048 / tb), tb, 0, s, w, sp); B2G_LAUNCHED(1);
         launch_pdl(k_bp_clear_moved, gf, kBlock, 0, s, w); B2G_LAUNCHED(1);
     }
+    if (n == 0) cudaMemsetAsync(w.sort_hist, 0, kSortRankWords * sizeof(uint32_t), s);
     if (after_traversal) after_traversal();
     /* sort new keys; payload = emission slot */
     radix_sort_pairs_coop(w.n_key, w.n_idx, w.n_key_alt, w.n_idx_alt, &w.cnt[CNT_NEW], w.pair_cap, 2 * w.key_bits,
-                          w.sort_hist, w.cnt, s, num_sms);
+                          w.sort_hist, w.cnt, s, num_sms, CNT_BARRIER2);
     uint32_t* flag = w.scan_tmp;
     uint32_t* rank = w.scan_tmp + w.contact_cap;
     uint32_t* tmp = w.scan_tmp + 2 * (size_t)w.contact_cap;

@@ -171,6 +171,8 @@ __global__ void __launch_bounds__(256, 4) k_collide(DevWorld w, StepParams sp, i
     if (warp_aborted(w)) return;
     if (starts_step) phase_stamp(w, PH_START);
     phase_stamp(w, PH_INITIAL);
+    if (blockIdx.x == 0 && threadIdx.x < 3) w.cnt[CNT_CASCADE + threadIdx.x] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) w.cnt[CNT_BARRIER] = w.cnt[CNT_BARRIER2] = 0;
     const int n = w.cnt[CNT_CONTACTS];
     const int lane = threadIdx.x & 31;
     const int stride = gridDim.x * blockDim.x;
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(256, 4) k_collide(DevWorld w, StepParams sp, i
  * rounds until a round finds none (a chain of wakes along the table's order). */
 __global__ void __launch_bounds__(256) k_collide_cascade(DevWorld w, StepParams sp) {
     if (warp_aborted(w)) return;
-    grid_barrier_start();
+    grid_barrier_start(CNT_BARRIER2);
     const int n = w.cnt[CNT_CONTACTS];
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
@@ -330,8 +332,6 @@ void launch_collide(const DevWorld& w, const StepParams& sp, cudaStream_t s, boo
     DevWorld wc = w;
     StepParams p = sp;
     void* args[] = {&wc, &p};
-    cudaMemsetAsync(w.cnt + CNT_BARRIER, 0, sizeof(int), s);
-    cudaMemsetAsync(w.cnt + CNT_CASCADE, 0, 3 * sizeof(int), s);
     cudaLaunchCooperativeKernel((const void*)k_collide_cascade, dim3(num_sms), dim3(256), args, 0, s);
     k_collide_wake<<<grid_for(w.n_bodies, 256, num_sms * 8), 256, 0, s>>>(w);
     B2G_LAUNCHED(2);

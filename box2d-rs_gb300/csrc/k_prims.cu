@@ -251,9 +251,9 @@ __global__ void k_rank_copy(const unsigned long long* __restrict__ kin, const ui
 
 __global__ void __launch_bounds__(kSortBlock) k_radix_coop(unsigned long long* ka, uint32_t* va, unsigned long long* kb,
                                                            uint32_t* vb, const int* d_n, int max_n, int bits,
-                                                           uint32_t* hist, int* cnt) {
+                                                           uint32_t* hist, int* cnt, int barrier_word) {
     if (world_aborted(cnt)) return;
-    grid_barrier_start();
+    grid_barrier_start(barrier_word);
     const int n = load_n(d_n, max_n);
     if (n > kSortTile && n <= kRankSort && max_n > kSortTile) return;  /* the rank count sorted it */
     radix_sort_grid(ka, va, kb, vb, n, bits, hist, cnt);
@@ -282,7 +282,7 @@ void scan_exclusive_u32(const uint32_t* in, uint32_t* out, const int* d_n, int m
 
 void radix_sort_pairs_coop(unsigned long long* key_a, uint32_t* val_a, unsigned long long* key_b, uint32_t* val_b,
                            const int* d_n, int max_n, int bits, uint32_t* hist, int* cnt, cudaStream_t s, int num_sms,
-                           bool zero_or_max) {
+                           int barrier_word, bool zero_or_max) {
     static int per_sm = 0;
     if (!per_sm) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_radix_coop, kSortBlock, 0);
@@ -295,7 +295,6 @@ void radix_sort_pairs_coop(unsigned long long* key_a, uint32_t* val_a, unsigned 
         /* the rank count for inputs between one tile and kRankSort keys (each kernel checks n) */
         const int m = std::min(max_n, kRankSort);
         const int tiles = (m + kRankTile - 1) / kRankTile;
-        cudaMemsetAsync(hist, 0, (size_t)m * sizeof(uint32_t), s);
         launch_pdl(k_rank_count, kRankBlocks, kRankTile, 0, s, (const unsigned long long*)key_a, d_n, max_n, hist, cnt);
         launch_pdl(k_rank_scatter, tiles, kRankTile, 0, s, (const unsigned long long*)key_a, (const uint32_t*)val_a,
                    key_b, val_b, d_n, max_n, (const uint32_t*)hist, cnt);
@@ -303,8 +302,7 @@ void radix_sort_pairs_coop(unsigned long long* key_a, uint32_t* val_a, unsigned 
                    val_a, d_n, max_n, cnt);
         B2G_LAUNCHED(3);
     }
-    void* args[] = {&key_a, &val_a, &key_b, &val_b, (void*)&d_n, &max_n, &bits, &hist, &cnt};
-    cudaMemsetAsync(cnt + CNT_BARRIER, 0, sizeof(int), s);
+    void* args[] = {&key_a, &val_a, &key_b, &val_b, (void*)&d_n, &max_n, &bits, &hist, &cnt, &barrier_word};
     cudaLaunchCooperativeKernel((const void*)k_radix_coop, dim3(blocks), dim3(kSortBlock), args, 0, s);
     B2G_LAUNCHED(1);
 }
@@ -312,6 +310,7 @@ void radix_sort_pairs_coop(unsigned long long* key_a, uint32_t* val_a, unsigned 
 size_t radix_sort_hist_size(int max_n) {
     const int tiles = (max_n + kSortTile - 1) / kSortTile;
     /* the rank count uses the first kRankSort entries */
+    static_assert(kRankSort == kSortRankWords, "the callers zero that many");
     return std::max((size_t)tiles * 256 * 2 + scan_tmp_size(tiles * 256) + 16, (size_t)kRankSort);
 }
 

@@ -1058,14 +1058,12 @@ __device__ __forceinline__ bool islands_pass(const DevWorld& w, int allow_sleep)
 /* k_solve runs 256 or 512 threads per block (cfg_solver_block); nothing in it depends on which */
 constexpr int kSolveMaxBlock = 512;
 
-__device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& sp) {
+/* phase 0: integrate velocities (b2_island_private.rs:136-170) */
+__device__ __forceinline__ void integrate_velocities(const DevWorld& w, const StepParams& sp) {
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int gsize = gridDim.x * blockDim.x;
     const int nb = w.n_bodies;
-    const int ncons = w.cnt[CNT_CONS];
-    const int ncol = w.cnt[CNT_COLOURS];
     const float h = sp.dt;
-    /* phase 0: integrate velocities (b2_island_private.rs:136-170) */
     for (int b = gtid; b < nb; b += gsize) {
         const uint32_t f = w.b_flags[b];
         if (!(f & BF_ISLAND)) continue;
@@ -1091,10 +1089,107 @@ __device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& 
             w.b_vel[b] = v;
         }
     }
-    if (!grid_barrier(w)) return false;
-    /* phase 1: constraint initialisation */
-    for (int k = gtid; k < ncons; k += gsize) init_slot(w, sp, k);
-    if (!grid_barrier(w)) return false;
+}
+
+/* phase 6a: copy back (synchronize_transform), sleep bookkeeping, clear forces */
+__device__ __forceinline__ void finish_bodies(const DevWorld& w, const StepParams& sp) {
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int gsize = gridDim.x * blockDim.x;
+    const int nb = w.n_bodies;
+    const float h = sp.dt;
+    const float linTolSqr = kLinearSleepTolerance * kLinearSleepTolerance;
+    const float angTolSqr = kAngularSleepTolerance * kAngularSleepTolerance;
+    for (int b = gtid; b < nb; b += gsize) {
+        const uint32_t f = w.b_flags[b];
+        if (f & BF_ISLAND) {
+            const float4 p = w.b_pos[b];
+            const float2 lc = w.b_lc[b];
+            Rot q = rot(p.z);
+            V2 xp = sub(mk(p.x, p.y), mul(q, mk(lc.x, lc.y)));
+            w.b_xf[b] = make_float4(xp.x, xp.y, q.s, q.c);
+            if (sp.allow_sleep) {
+                float4 v = w.b_vel[b];
+                float st;
+                if (!(f & BF_AUTO_SLEEP) || v.z * v.z > angTolSqr || v.x * v.x + v.y * v.y > linTolSqr) {
+                    st = 0.0f;
+                    v.w = 0.0f;
+                } else {
+                    v.w += h;
+                    st = v.w;
+                }
+                w.b_vel[b] = v;
+                agg_atomic_min((unsigned*)w.isl_sleep, w.b_island[b], __float_as_uint(st));
+            }
+        }
+        if (sp.auto_clear) w.b_force[b] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+}
+
+/* phase 6a, after every body: islands at rest long enough fall asleep */
+__device__ __forceinline__ void finish_sleep(const DevWorld& w, const StepParams& sp) {
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int gsize = gridDim.x * blockDim.x;
+    const int nb = w.n_bodies;
+    const float tol = 3.0f * kLinearSlop;
+    for (int b = gtid; b < nb; b += gsize) {
+        const uint32_t f = w.b_flags[b];
+        if (!(f & BF_ISLAND)) continue;
+        const int r = w.b_island[b];
+        bool solved = false;  /* position_solved: some iteration ended with min separation >= -3 slop */
+        for (int j = 0; j < sp.pi && !solved; ++j)
+            solved = __uint_as_float(w.isl_minsep[(size_t)j * w.body_cap + r]) <= tol;
+        if (solved && w.isl_sleep[r] >= kTimeToSleep) {
+            w.b_flags[b] = f & ~BF_AWAKE;
+            w.b_vel[b] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            w.b_force[b] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    }
+}
+
+/* phase 6b: synchronize fixtures (private/dynamics/b2_body.rs:455-475); the proxies moved are counted for
+ * the broadphase's rebuild decision */
+__device__ __forceinline__ void finish_fixtures(const DevWorld& w) {
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int gsize = gridDim.x * blockDim.x;
+    unsigned moved = 0;
+    for (int f = gtid; f < w.n_fixtures; f += gsize) {
+        const int b = w.f_body[f];
+        const uint32_t bf = w.b_flags[b];
+        if (!(bf & BF_ISLAND) || is_static(bf)) continue;
+        const float4 x = w.b_xf[b];
+        Xf xf2;
+        xf2.p = mk(x.x, x.y);
+        xf2.q.s = x.z;
+        xf2.q.c = x.w;
+        Xf xf1 = xf2;
+        if (bf & BF_AWAKE) {
+            const float4 p0 = w.b_pos0[b];
+            const float2 lc = w.b_lc[b];
+            xf1.q = rot(p0.z);
+            xf1.p = sub(mk(p0.x, p0.y), mul(xf1.q, mk(lc.x, lc.y)));
+        }
+        if (sync_fixture(w, f, xf1, xf2)) ++moved;
+    }
+    moved = __reduce_add_sync(0xffffffffu, moved);
+    if ((threadIdx.x & 31) == 0 && moved) atomicAdd(&w.cnt[CNT_BP_MOVED], (int)moved);
+}
+
+/* WHOLE: the solver from the velocities' integration to the fixtures' synchronisation (one cluster); else
+ * the sweeps between them, whose kernels before and after it spread over more threads */
+template <bool WHOLE>
+__device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& sp) {
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int gsize = gridDim.x * blockDim.x;
+    const int nb = w.n_bodies;
+    const int ncons = w.cnt[CNT_CONS];
+    const int ncol = w.cnt[CNT_COLOURS];
+    const float h = sp.dt;
+    if (WHOLE) {
+        integrate_velocities(w, sp);
+        if (!grid_barrier(w)) return false;
+        for (int k = gtid; k < ncons; k += gsize) init_slot(w, sp, k);
+        if (!grid_barrier(w)) return false;
+    }
     const int interior = w.cnt[CNT_INTERIOR];
     const bool parts = interior > 0;
     const int nparts = w.cnt[CNT_PARTS];
@@ -1345,79 +1440,22 @@ __device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& 
             if (!grid_barrier(w)) return false;
         }
     }
-    /* phase 6a: copy back (synchronize_transform), sleep bookkeeping, clear forces */
-    const float linTolSqr = kLinearSleepTolerance * kLinearSleepTolerance;
-    const float angTolSqr = kAngularSleepTolerance * kAngularSleepTolerance;
-    for (int b = gtid; b < nb; b += gsize) {
-        const uint32_t f = w.b_flags[b];
-        if (f & BF_ISLAND) {
-            const float4 p = w.b_pos[b];
-            const float2 lc = w.b_lc[b];
-            Rot q = rot(p.z);
-            V2 xp = sub(mk(p.x, p.y), mul(q, mk(lc.x, lc.y)));
-            w.b_xf[b] = make_float4(xp.x, xp.y, q.s, q.c);
-            if (sp.allow_sleep) {
-                float4 v = w.b_vel[b];
-                float st;
-                if (!(f & BF_AUTO_SLEEP) || v.z * v.z > angTolSqr || v.x * v.x + v.y * v.y > linTolSqr) {
-                    st = 0.0f;
-                    v.w = 0.0f;
-                } else {
-                    v.w += h;
-                    st = v.w;
-                }
-                w.b_vel[b] = v;
-                agg_atomic_min((unsigned*)w.isl_sleep, w.b_island[b], __float_as_uint(st));
-            }
+    if (WHOLE) {
+        finish_bodies(w, sp);
+        if (sp.allow_sleep) {
+            if (!grid_barrier(w)) return false;
+            finish_sleep(w, sp);
         }
-        if (sp.auto_clear) w.b_force[b] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-    if (sp.allow_sleep) {
         if (!grid_barrier(w)) return false;
-        for (int b = gtid; b < nb; b += gsize) {
-            const uint32_t f = w.b_flags[b];
-            if (!(f & BF_ISLAND)) continue;
-            const int r = w.b_island[b];
-            bool solved = false;  /* position_solved: some iteration ended with min separation >= -3 slop */
-            for (int j = 0; j < sp.pi && !solved; ++j)
-                solved = __uint_as_float(w.isl_minsep[(size_t)j * w.body_cap + r]) <= tol;
-            if (solved && w.isl_sleep[r] >= kTimeToSleep) {
-                w.b_flags[b] = f & ~BF_AWAKE;
-                w.b_vel[b] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                w.b_force[b] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
-        }
+        finish_fixtures(w);
     }
-    if (!grid_barrier(w)) return false;
-    /* phase 6b: synchronize fixtures (private/dynamics/b2_body.rs:455-475); the proxies moved are
-     * counted for the broadphase's rebuild decision */
-    unsigned moved = 0;
-    for (int f = gtid; f < w.n_fixtures; f += gsize) {
-        const int b = w.f_body[f];
-        const uint32_t bf = w.b_flags[b];
-        if (!(bf & BF_ISLAND) || is_static(bf)) continue;
-        const float4 x = w.b_xf[b];
-        Xf xf2;
-        xf2.p = mk(x.x, x.y);
-        xf2.q.s = x.z;
-        xf2.q.c = x.w;
-        Xf xf1 = xf2;
-        if (bf & BF_AWAKE) {
-            const float4 p0 = w.b_pos0[b];
-            const float2 lc = w.b_lc[b];
-            xf1.q = rot(p0.z);
-            xf1.p = sub(mk(p0.x, p0.y), mul(xf1.q, mk(lc.x, lc.y)));
-        }
-        if (sync_fixture(w, f, xf1, xf2)) ++moved;
-    }
-    moved = __reduce_add_sync(0xffffffffu, moved);
-    if ((threadIdx.x & 31) == 0 && moved) atomicAdd(&w.cnt[CNT_BP_MOVED], (int)moved);
     return true;
 }
 
 __global__ void __launch_bounds__(kBlock) k_islands(DevWorld w, int allow_sleep) {
     B2G_RETURN_IF_ABORTED(w);
     phase_stamp(w, PH_COLLIDE);
+    if (blockIdx.x == 0 && threadIdx.x == 0) w.cnt[CNT_BARRIER2] = 0;  /* k_colour's */
     grid_barrier_start();
     islands_pass(w, allow_sleep);
 }
@@ -1425,15 +1463,51 @@ __global__ void __launch_bounds__(kBlock) k_islands(DevWorld w, int allow_sleep)
 __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
     B2G_RETURN_IF_ABORTED(w);
     phase_stamp(w, PH_ISLANDS);
-    grid_barrier_start();
+    grid_barrier_start(CNT_BARRIER2);
     colour_pass(w, nparts);
 }
 
 __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams sp) {
     B2G_RETURN_IF_ABORTED(w);
-    phase_stamp(w, PH_COLOURING);
     grid_barrier_start();
-    solve_pass(w, sp);
+    solve_pass<false>(w, sp);
+}
+
+/* The passes before and after the sweeps, each a thread for every body, slot or fixture: long chains of
+ * gathers, which the persistent kernel's 8 warps an SM left waiting for memory (of the 250k-box pile's solve
+ * 1306 us: initialisation 270, bodies and fixtures 60; the solve takes 1020 us with these kernels, that of
+ * 4096 worlds 4.24 ms instead of 5.3). */
+__global__ void __launch_bounds__(kBlock) k_solve_velocities(const __grid_constant__ DevWorld w,
+                                                             const __grid_constant__ StepParams sp) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    phase_stamp(w, PH_COLOURING);
+    if (blockIdx.x == 0 && threadIdx.x == 0) w.cnt[CNT_BARRIER] = 0;  /* k_solve's */
+    integrate_velocities(w, sp);
+}
+__global__ void __launch_bounds__(kBlock) k_solve_init(const __grid_constant__ DevWorld w,
+                                                       const __grid_constant__ StepParams sp) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    const int ncons = w.cnt[CNT_CONS];
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < ncons; k += gridDim.x * blockDim.x) init_slot(w, sp, k);
+}
+__global__ void __launch_bounds__(kBlock) k_solve_bodies(const __grid_constant__ DevWorld w,
+                                                         const __grid_constant__ StepParams sp) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    finish_bodies(w, sp);
+}
+__global__ void __launch_bounds__(kBlock) k_solve_sleep(const __grid_constant__ DevWorld w,
+                                                        const __grid_constant__ StepParams sp) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    finish_sleep(w, sp);
+}
+__global__ void __launch_bounds__(kBlock) k_solve_fixtures(const __grid_constant__ DevWorld w) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    finish_fixtures(w);
 }
 
 /* Islands, colouring and solver of a world of a few thousand bodies as one kernel on one cluster of up
@@ -1458,7 +1532,7 @@ __global__ void __launch_bounds__(kBlock) k_front(const __grid_constant__ DevWor
     if (passes & FRONT_SOLVE) {
         grid_barrier(w);
         phase_stamp(w, PH_COLOURING);
-        solve_pass(w, sp);
+        solve_pass<true>(w, sp);
     }
 }
 
@@ -1514,7 +1588,6 @@ void launch_islands_and_constraints(const DevWorld& w, const StepParams& sp, cud
         DevWorld wc = w;
         int allow_sleep = sp.allow_sleep;
         void* args[] = {&wc, &allow_sleep};
-        cudaMemsetAsync(w.cnt + CNT_BARRIER, 0, sizeof(int), s);
         cudaLaunchCooperativeKernel((const void*)k_islands, dim3(w.num_sms * per_sm), dim3(kBlock), args, 0, s);
         B2G_LAUNCHED(1);
     }
@@ -1554,7 +1627,6 @@ void launch_colouring(const DevWorld& w, cudaStream_t s, int num_sms, bool parts
     DevWorld wc = w;
     int nparts = use_parts(w, num_sms, parts) ? part_count(w, num_sms) : 0;
     void* args[] = {&wc, &nparts};
-    cudaMemsetAsync(w.cnt + CNT_BARRIER, 0, sizeof(int), s);
     cudaLaunchCooperativeKernel((const void*)k_colour, dim3(blocks), dim3(kBlock), args, 0, s);
     B2G_LAUNCHED(1);
 }
@@ -1590,10 +1662,16 @@ int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int n
     if (use_parts(w, num_sms, parts))
         smem = part_smem(spc, w.cfg_coop_per_sm == 1 ? kPartSmemOne : (w.cfg_coop_per_sm == 2 ? kPartSmemTwo : 0));
     void* args[] = {&wc, &spc};
-    B2G_LAUNCHED(1);
-    cudaMemsetAsync(w.cnt + CNT_BARRIER, 0, sizeof(int), s);
+    const int gb = grid_for(w.n_bodies, kBlock, num_sms * 8), gc = grid_for(w.cons_cap, kBlock, num_sms * 8);
+    launch_pdl(k_solve_velocities, gb, kBlock, 0, s, w, spc);
+    launch_pdl(k_solve_init, gc, kBlock, 0, s, w, spc);
     const int threads = w.cfg_coop_per_sm == 1 && w.cfg_solver_block == kSolveMaxBlock ? kSolveMaxBlock : kBlock;
-    return (int)cudaLaunchCooperativeKernel((const void*)k_solve, dim3(blocks), dim3(threads), args, smem, s);
+    const int rc = (int)cudaLaunchCooperativeKernel((const void*)k_solve, dim3(blocks), dim3(threads), args, smem, s);
+    launch_pdl(k_solve_bodies, gb, kBlock, 0, s, w, spc);
+    if (sp.allow_sleep) launch_pdl(k_solve_sleep, gb, kBlock, 0, s, w, spc);
+    launch_pdl(k_solve_fixtures, grid_for(w.n_fixtures, kBlock, num_sms * 8), kBlock, 0, s, w);
+    B2G_LAUNCHED(sp.allow_sleep ? 6 : 5);
+    return rc;
 }
 
 /* The largest cluster k_front and k_back can run as on the current device (0: none), found once per
