@@ -75,44 +75,85 @@ __device__ __forceinline__ void grid_barrier_start(int word = CNT_BARRIER) {
     }
 }
 
-/* cnt: the counter block (uses the launch's counter and CNT_STATUS) */
+/* Thread 0's wait until the launch's counter (in the block cnt, which also holds CNT_STATUS) has reached
+ * `target` arrivals; false when it ran out or another block's did. */
+__device__ __forceinline__ bool grid_wait(int* cnt, unsigned target) {
+    const unsigned* count = (const unsigned*)&cnt[b2g_barrier_word];
+    target += b2g_barrier_hold;
+    const long long t0 = clock64();
+    unsigned polls = 0;
+    while ((int)(ld_acquire_gpu(count) - target) < 0) {
+        if ((++polls & 255u) == 0u) {
+            if (((volatile int*)cnt)[CNT_STATUS] & ST_BARRIER_TIMEOUT) return false;
+            if (clock64() - t0 > b2g_barrier_limit) {
+                atomicOr((unsigned*)&cnt[CNT_STATUS], ST_BARRIER_TIMEOUT);
+                return false;
+            }
+        }
+    }
+    return true;
+}
+/* thread 0's arrival at the next barrier of the launch, for `blocks` blocks; returns the barrier's number */
+__device__ __forceinline__ unsigned grid_arrive(int* cnt, unsigned blocks) {
+    if (b2g_barrier_epoch == 0u) {
+        int2 lim_hold;
+        asm volatile("ld.volatile.global.v2.s32 {%0, %1}, [%2];"
+                     : "=r"(lim_hold.x), "=r"(lim_hold.y) : "l"(&cnt[CNT_BARRIER_LIMIT]) : "memory");
+        b2g_barrier_limit = lim_hold.x > 0 ? (long long)lim_hold.x << 10 : 2000000000LL;
+        b2g_barrier_hold = (unsigned)max(lim_hold.y, 0);
+    }
+    ++b2g_barrier_epoch;
+    if (blocks) red_release_add_gpu((unsigned*)&cnt[b2g_barrier_word], blocks);
+    return b2g_barrier_epoch;
+}
+/* the grid is one cluster: its barrier */
+__device__ __forceinline__ bool grid_is_cluster() { return cluster_blocks() == gridDim.x; }
+__device__ __forceinline__ void cluster_grid_barrier() {
+    if (gridDim.x == 1) __syncthreads();
+    else cluster_barrier();
+}
+
+/* cnt: the counter block */
 __device__ __forceinline__ bool grid_barrier(int* cnt) {
     __shared__ int s_ok;
-    if (cluster_blocks() == gridDim.x) {
-        if (gridDim.x == 1) __syncthreads();
-        else cluster_barrier();
+    if (grid_is_cluster()) {
+        cluster_grid_barrier();
+        return true;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_ok = grid_wait(cnt, grid_arrive(cnt, 1u) * gridDim.x) ? 1 : 0;
+    __syncthreads();
+    return s_ok != 0;
+}
+
+/* A barrier in two halves around work of one block, `one`: grid_gather returns to that block when every
+ * block has arrived (to the others at once), grid_release to the others when that block has come to it.
+ * Work that would take several grid barriers when it is spread over the blocks takes __syncthreads there. */
+__device__ __forceinline__ bool grid_gather(int* cnt, int one) {
+    __shared__ int s_ok;
+    if (grid_is_cluster()) {
+        cluster_grid_barrier();
         return true;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (b2g_barrier_epoch == 0u) {
-            int2 lim_hold;
-            asm volatile("ld.volatile.global.v2.s32 {%0, %1}, [%2];"
-                         : "=r"(lim_hold.x), "=r"(lim_hold.y) : "l"(&cnt[CNT_BARRIER_LIMIT]) : "memory");
-            b2g_barrier_limit = lim_hold.x > 0 ? (long long)lim_hold.x << 10 : 2000000000LL;
-            b2g_barrier_hold = (unsigned)max(lim_hold.y, 0);
-        }
-        unsigned* count = (unsigned*)&cnt[b2g_barrier_word];
-        const unsigned target = (b2g_barrier_epoch + 1u) * gridDim.x + b2g_barrier_hold;
-        ++b2g_barrier_epoch;
-        red_release_add_gpu(count, 1u);
-        const long long t0 = clock64();
-        unsigned polls = 0;
-        int ok = 1;
-        while ((int)(ld_acquire_gpu(count) - target) < 0) {
-            if ((++polls & 255u) == 0u) {
-                if (((volatile int*)cnt)[CNT_STATUS] & ST_BARRIER_TIMEOUT) {
-                    ok = 0;
-                    break;
-                }
-                if (clock64() - t0 > b2g_barrier_limit) {
-                    atomicOr((unsigned*)&cnt[CNT_STATUS], ST_BARRIER_TIMEOUT);
-                    ok = 0;
-                    break;
-                }
-            }
-        }
-        s_ok = ok;
+        const unsigned k = grid_arrive(cnt, 1u);
+        s_ok = (int)blockIdx.x != one || grid_wait(cnt, k * gridDim.x) ? 1 : 0;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+__device__ __forceinline__ bool grid_release(int* cnt, int one) {
+    __shared__ int s_ok;
+    if (grid_is_cluster()) {
+        cluster_grid_barrier();
+        return true;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const bool mine = (int)blockIdx.x == one;
+        const unsigned k = grid_arrive(cnt, mine ? gridDim.x : 0u);
+        s_ok = mine || grid_wait(cnt, k * gridDim.x) ? 1 : 0;
     }
     __syncthreads();
     return s_ok != 0;

@@ -734,7 +734,9 @@ struct PartCtx {
     float4* state;     /* shared: cached velocities or positions */
     int* body;         /* shared: the cached bodies */
     void* slots;       /* shared: VelSlot[cap_vel] or PosSlot[cap_pos] */
-    void* bslots;      /* shared: this block's boundary slots, VelSlot or PosSlot[kBndSlots] */
+    void* bslots;      /* shared: this block's boundary slots, VelSlot or PosSlot[bcap] */
+    int bcap;          /* boundary slots cached */
+    int one;           /* the block that sweeps the boundary colours, -1: spread over all */
     const int* bco;    /* shared: boundary colour offsets */
     const int* boff;   /* shared: per boundary colour, this block's first entry of bslots */
 };
@@ -744,8 +746,21 @@ struct PartCtx {
 constexpr int kBndSlots = 128;
 constexpr int kBndBytes = kBndSlots * (int)sizeof(VelSlot);
 
+/* A world with few boundary constraints has one block sweep all of their colours, a __syncthreads after
+ * each, between the halves of one grid barrier, instead of a grid barrier after each colour's share of
+ * every block. Solver, us, spread and in one block: 37 boundary slots of 31 parts 146 and 130, 170 of 117
+ * parts 174 and 165, 390 of 152 parts 213 and 214, 2400 of 39 parts 366 and 503; on a cluster, whose blocks
+ * load the slots' bodies from L2 again after each barrier, 50 slots of 5 parts 237 and 208, 290 of 11 parts
+ * 290 and 262. */
+constexpr int kOneBlockSlots = 256, kOneBlockSlotsCluster = 1024;
+
 __device__ __forceinline__ void bnd_range(const PartCtx& pc, int c, int* lo, int* hi) {
     const int len = pc.bco[c + 1] - pc.bco[c];
+    if (pc.one >= 0) {
+        *lo = 0;
+        *hi = (int)blockIdx.x == pc.one ? len : 0;
+        return;
+    }
     *lo = (int)((long long)len * blockIdx.x / gridDim.x);
     *hi = (int)((long long)len * (blockIdx.x + 1) / gridDim.x);
 }
@@ -766,7 +781,7 @@ __device__ void bnd_vel_sweep(const DevWorld& w, const PartCtx& pc, int c, bool 
     VelSlot* bs = (VelSlot*)pc.bslots;
     for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
         const int k = pc.bco[c] + i, j = pc.boff[c] + i - lo;
-        const bool cached = j < kBndSlots;
+        const bool cached = j < pc.bcap;
         const VelSlot sl = cached ? bs[j] : vel_slot(w, k);
         float4 va = w.b_vel[sl.idx.x], vb = w.b_vel[sl.idx.y];
         if (warm) {
@@ -790,7 +805,7 @@ __device__ void bnd_pos_sweep(const DevWorld& w, const PartCtx& pc, int c, int i
     const PosSlot* bs = (const PosSlot*)pc.bslots;
     for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
         const int k = pc.bco[c] + i, j = pc.boff[c] + i - lo;
-        const bool cached = j < kBndSlots;
+        const bool cached = j < pc.bcap;
         const PosSlot sl = cached ? bs[j] : pos_slot(w, k);
         if (cached ? sl.pad[0] != 0 : island_done(w, sl.island, it, tol)) continue;
         float4 pa = w.b_pos[sl.idx.x], pb = w.b_pos[sl.idx.y];
@@ -1216,7 +1231,11 @@ __device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& 
         pc.state = s_part;
         pc.body = (int*)(s_part + sp.part_bodies);
         pc.bslots = (void*)(s_part + sp.part_bodies + (sp.part_bodies + 3) / 4);
-        pc.slots = (void*)((char*)pc.bslots + kBndBytes);
+        /* spread, the boundary slots' caches come first; in one block after its interior slots (a block
+         * without a part where there is one) */
+        const int few = grid_is_cluster() ? kOneBlockSlotsCluster : kOneBlockSlots;
+        pc.one = ncol > 0 && ncons - interior <= few ? (nparts < (int)gridDim.x ? nparts : 0) : -1;
+        pc.slots = pc.one < 0 ? (void*)((char*)pc.bslots + kBndBytes) : pc.bslots;
         pc.bco = s_bco;
         pc.boff = s_boff;
         for (int i = threadIdx.x; i <= ncol; i += blockDim.x) s_bco[i] = w.col_off[i];
@@ -1233,9 +1252,14 @@ __device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& 
         }
         pc.ibeg = pc.ncol > 0 ? s_off[0] : 0;
         const int nint = pc.ncol > 0 ? s_off[pc.ncol] - pc.ibeg : 0;
-        const int islot_bytes = max(0, sp.part_slot_bytes - kBndBytes);
+        const int islot_bytes = max(0, sp.part_slot_bytes - (pc.one < 0 ? kBndBytes : 0));
         pc.cap_vel = min(nint, islot_bytes / (int)sizeof(VelSlot));
         pc.cap_pos = min(nint, islot_bytes / (int)sizeof(PosSlot));
+        pc.bcap = kBndSlots;
+        if (pc.one >= 0) {
+            pc.bslots = (void*)((VelSlot*)pc.slots + pc.cap_vel);
+            pc.bcap = islot_bytes / (int)sizeof(VelSlot) - pc.cap_vel;
+        }
         for (int l = threadIdx.x; l < pc.nloc; l += blockDim.x) {
             const int b = w.cache_body[pc.cbeg + l];
             pc.body[l] = b;
@@ -1256,7 +1280,7 @@ __device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& 
             bnd_range(pc, c, &lo, &hi);
             for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
                 const int j = s_boff[c] + i - lo;
-                if (j < kBndSlots) ((VelSlot*)pc.bslots)[j] = vel_slot(w, s_bco[c] + i);
+                if (j < pc.bcap) ((VelSlot*)pc.bslots)[j] = vel_slot(w, s_bco[c] + i);
             }
         }
         __syncthreads();
@@ -1271,10 +1295,20 @@ __device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& 
                 for (int j = threadIdx.x; j < pc.cap_vel; j += blockDim.x) w.vc_imp[pc.ibeg + j] = vs[j].imp;
             if (ncol > 0 || last) part_store(pc, w.b_vel);
             if (ncol > 0) {
-                if (!grid_barrier(w)) return false;
-                for (int c = 0; c < ncol; ++c) {
-                    bnd_vel_sweep(w, pc, c, warm, last);
+                if (pc.one >= 0) {
+                    if (!grid_gather(w.cnt, pc.one)) return false;
+                    if ((int)blockIdx.x == pc.one)
+                        for (int c = 0; c < ncol; ++c) {
+                            bnd_vel_sweep(w, pc, c, warm, last);
+                            __syncthreads();
+                        }
+                    if (!grid_release(w.cnt, pc.one)) return false;
+                } else {
                     if (!grid_barrier(w)) return false;
+                    for (int c = 0; c < ncol; ++c) {
+                        bnd_vel_sweep(w, pc, c, warm, last);
+                        if (!grid_barrier(w)) return false;
+                    }
                 }
                 if (!last) {
                     part_load(pc, w.b_vel);
@@ -1370,18 +1404,22 @@ __device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& 
             if (b >= 0) pc.state[l] = w.b_pos[b];
         }
         PosSlot* ps = (PosSlot*)pc.slots;
+        if (pc.one >= 0) {
+            pc.bslots = (void*)(ps + pc.cap_pos);
+            pc.bcap = max(0, sp.part_slot_bytes) / (int)sizeof(PosSlot) - pc.cap_pos;
+        }
         for (int j = threadIdx.x; j < pc.cap_pos; j += blockDim.x) ps[j] = part_pos_slot(w, pc, pc.ibeg + j);
         for (int c = 0; c < ncol; ++c) {
             int lo, hi;
             bnd_range(pc, c, &lo, &hi);
             for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
                 const int j = s_boff[c] + i - lo;
-                if (j < kBndSlots) ((PosSlot*)pc.bslots)[j] = pos_slot(w, s_bco[c] + i);
+                if (j < pc.bcap) ((PosSlot*)pc.bslots)[j] = pos_slot(w, s_bco[c] + i);
             }
         }
         __syncthreads();
     }
-    const int nbnd = parts ? min(s_boff[ncol], kBndSlots) : 0;
+    const int nbnd = parts ? min(s_boff[ncol], pc.bcap) : 0;
     for (int it = 0; it < sp.pi; ++it) {
         uint32_t* cur = w.isl_minsep + (size_t)it * w.body_cap;
         if (parts) {
@@ -1396,10 +1434,20 @@ __device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& 
             part_pos_sweeps(w, pc, it, cur, tol);
             if (ncol > 0) {
                 part_store(pc, w.b_pos);
-                if (!grid_barrier(w)) return false;
-                for (int c = 0; c < ncol; ++c) {
-                    bnd_pos_sweep(w, pc, c, it, cur, tol);
+                if (pc.one >= 0) {
+                    if (!grid_gather(w.cnt, pc.one)) return false;
+                    if ((int)blockIdx.x == pc.one)
+                        for (int c = 0; c < ncol; ++c) {
+                            bnd_pos_sweep(w, pc, c, it, cur, tol);
+                            __syncthreads();
+                        }
+                    if (!grid_release(w.cnt, pc.one)) return false;
+                } else {
                     if (!grid_barrier(w)) return false;
+                    for (int c = 0; c < ncol; ++c) {
+                        bnd_pos_sweep(w, pc, c, it, cur, tol);
+                        if (!grid_barrier(w)) return false;
+                    }
                 }
                 if (it < sp.pi - 1) {
                     part_load(pc, w.b_pos);
