@@ -92,6 +92,8 @@ B2G_HD Rot rot(float angle) {
     b2g_sincosf(angle, &q.s, &q.c);
     return q;
 }
+/* the rotations of a pair of bodies, computed side by side */
+B2G_HD void rot2(float a, float b, Rot& qa, Rot& qb) { b2g_sincosf2(a, b, &qa.s, &qa.c, &qb.s, &qb.c); }
 B2G_HD V2 mul(Rot q, V2 v) { return mk(q.c * v.x - q.s * v.y, q.s * v.x + q.c * v.y); }
 B2G_HD V2 mul_t(Rot q, V2 v) { return mk(q.c * v.x + q.s * v.y, -q.s * v.x + q.c * v.y); }
 B2G_HD Rot mul_t(Rot q, Rot r) { Rot o; o.s = q.c * r.s - q.s * r.c; o.c = q.c * r.c + q.s * r.s; return o; }

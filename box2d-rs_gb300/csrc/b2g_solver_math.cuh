@@ -82,7 +82,9 @@ __device__ __forceinline__ void make_constraint(const ConstraintIn& in, VelSlot&
     } else if (mtype == MANIFOLD_FACE_A) {
         normal = mul(xfA.q, ln);
         V2 plane = mul(xfA, lpt);
-        for (int j = 0; j < count; ++j) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            if (j >= count) break;
             V2 clip = mul(xfB, lp[j]);
             V2 ca = add(clip, scale(rA - dot(sub(clip, plane), normal), normal));
             V2 cb = sub(clip, scale(rB, normal));
@@ -91,7 +93,9 @@ __device__ __forceinline__ void make_constraint(const ConstraintIn& in, VelSlot&
     } else {
         normal = mul(xfB.q, ln);
         V2 plane = mul(xfB, lpt);
-        for (int j = 0; j < count; ++j) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            if (j >= count) break;
             V2 clip = mul(xfA, lp[j]);
             V2 cb = add(clip, scale(rB - dot(sub(clip, plane), normal), normal));
             V2 ca = sub(clip, scale(rA, normal));
@@ -106,7 +110,9 @@ __device__ __forceinline__ void make_constraint(const ConstraintIn& in, VelSlot&
         ra[j] = mk(0.0f, 0.0f);
         rb[j] = mk(0.0f, 0.0f);
     }
-    for (int j = 0; j < count; ++j) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        if (j >= count) break;
         ra[j] = sub(wp[j], cA);
         rb[j] = sub(wp[j], cB);
         float rnA = cross(ra[j], normal);
@@ -175,11 +181,13 @@ __device__ __forceinline__ void warm_math(const VelSlot& sl, float4& va, float4&
     float wA = va.z, wB = vb.z;
     const V2 normal = mk(nf.x, nf.y);
     const V2 tangent = cross_vs(normal, 1.0f);
-    const float4 r[2] = {sl.r0, sl.r1};
-    const float ni[2] = {imp.x, imp.z}, ti[2] = {imp.y, imp.w};
-    for (int j = 0; j < idx.z; ++j) {
-        const V2 rA = mk(r[j].x, r[j].y), rB = mk(r[j].z, r[j].w);
-        const V2 P = add(scale(ni[j], normal), scale(ti[j], tangent));
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        if (j >= idx.z) break;
+        const float4 r = j == 0 ? sl.r0 : sl.r1;
+        const float ni = j == 0 ? imp.x : imp.z, ti = j == 0 ? imp.y : imp.w;
+        const V2 rA = mk(r.x, r.y), rB = mk(r.z, r.w);
+        const V2 P = add(scale(ni, normal), scale(ti, tangent));
         wA -= inv.z * cross(rA, P);
         vA = sub(vA, scale(inv.x, P));
         wB += inv.w * cross(rB, P);
@@ -310,39 +318,30 @@ __device__ __forceinline__ float solve_position_math(const PosSlot& sl, float4& 
     const int count = __float_as_int(meta.w);
     const float rA = meta.x, rB = meta.y;
     const V2 ln = mk(geo.x, geo.y), lpt = mk(geo.z, geo.w);
-    const V2 lps[2] = {mk(lp.x, lp.y), mk(lp.z, lp.w)};
     V2 cA = mk(pa.x, pa.y), cB = mk(pb.x, pb.y);
     float aA = pa.z, aB = pb.z;
     float minSep = 0.0f;
+    /* The three manifold types share one flow: the shape P holds the reference point (A for circles and
+     * face A, B for face B), Q the clip point, so a warp whose lanes differ in type runs it once; and both
+     * points share one loop body, short enough for the instruction cache nearest the scheduler. */
+    const bool circles = mtype == MANIFOLD_CIRCLES, faceB = mtype != MANIFOLD_CIRCLES && mtype != MANIFOLD_FACE_A;
+#pragma unroll 1
     for (int j = 0; j < count; ++j) {
         Xf xfA, xfB;
-        xfA.q = rot(aA);
-        xfB.q = rot(aB);
+        rot2(aA, aB, xfA.q, xfB.q);
         xfA.p = sub(cA, mul(xfA.q, lcA));
         xfB.p = sub(cB, mul(xfB.q, lcB));
-        V2 normal, point;
-        float separation;
-        if (mtype == MANIFOLD_CIRCLES) {
-            V2 pA = mul(xfA, lpt);
-            V2 pB = mul(xfB, lps[0]);
-            normal = sub(pB, pA);
+        const Xf P = faceB ? xfB : xfA, Q = faceB ? xfA : xfB;
+        const V2 plane = mul(P, lpt);
+        const V2 clip = mul(Q, circles || j == 0 ? mk(lp.x, lp.y) : mk(lp.z, lp.w));
+        V2 normal = mul(P.q, ln), point = clip;
+        if (circles) {
+            normal = sub(clip, plane);
             normalize(normal);
-            point = scale(0.5f, add(pA, pB));
-            separation = dot(sub(pB, pA), normal) - rA - rB;
-        } else if (mtype == MANIFOLD_FACE_A) {
-            normal = mul(xfA.q, ln);
-            V2 plane = mul(xfA, lpt);
-            V2 clip = mul(xfB, lps[j]);
-            separation = dot(sub(clip, plane), normal) - rA - rB;
-            point = clip;
-        } else {
-            normal = mul(xfB.q, ln);
-            V2 plane = mul(xfB, lpt);
-            V2 clip = mul(xfA, lps[j]);
-            separation = dot(sub(clip, plane), normal) - rA - rB;
-            point = clip;
-            normal = neg(normal);
+            point = scale(0.5f, add(plane, clip));
         }
+        const float separation = dot(sub(clip, plane), normal) - rA - rB;
+        if (faceB) normal = neg(normal);
         V2 ra = sub(point, cA);
         V2 rb = sub(point, cB);
         minSep = fminr(minSep, separation);
@@ -351,11 +350,11 @@ __device__ __forceinline__ float solve_position_math(const PosSlot& sl, float4& 
         float rnB = cross(rb, normal);
         float K = mA + mB + iA * rnA * rnA + iB * rnB * rnB;
         float impulse = K > 0.0f ? fdiv(-C, K) : 0.0f;
-        V2 P = scale(impulse, normal);
-        cA = sub(cA, scale(mA, P));
-        aA -= iA * cross(ra, P);
-        cB = add(cB, scale(mB, P));
-        aB += iB * cross(rb, P);
+        V2 P1 = scale(impulse, normal);
+        cA = sub(cA, scale(mA, P1));
+        aA -= iA * cross(ra, P1);
+        cB = add(cB, scale(mB, P1));
+        aB += iB * cross(rb, P1);
     }
     pa = make_float4(cA.x, cA.y, aA, pa.w);
     pb = make_float4(cB.x, cB.y, aB, pb.w);

@@ -269,14 +269,13 @@ struct Sweep {
     float a0, a, alpha0;
 };
 
-/* B2Sweep::get_transform, src/b2_math.rs:764-771 */
-__device__ __forceinline__ Xf sweep_xf(const Sweep& s, float beta) {
-    Xf xf;
-    xf.p = add(scale(1.0f - beta, s.c0), scale(beta, s.c));
-    const float angle = (1.0f - beta) * s.a0 + beta * s.a;
-    xf.q = rot(angle);
-    xf.p = sub(xf.p, mul(xf.q, s.lc));
-    return xf;
+/* B2Sweep::get_transform (src/b2_math.rs:764-771) of both sweeps at beta, their rotations side by side */
+__device__ __forceinline__ void sweep_xf2(const Sweep& a, const Sweep& b, float beta, Xf& xa, Xf& xb) {
+    xa.p = add(scale(1.0f - beta, a.c0), scale(beta, a.c));
+    xb.p = add(scale(1.0f - beta, b.c0), scale(beta, b.c));
+    rot2((1.0f - beta) * a.a0 + beta * a.a, (1.0f - beta) * b.a0 + beta * b.a, xa.q, xb.q);
+    xa.p = sub(xa.p, mul(xa.q, a.lc));
+    xb.p = sub(xb.p, mul(xb.q, b.lc));
 }
 
 enum { SEP_POINTS = 0, SEP_FACE_A = 1, SEP_FACE_B = 2 };
@@ -291,7 +290,8 @@ __device__ SepFn sep_init(const SimplexCache& cache, const DistProxy& pa, const 
                           const Sweep& sb, float t1) {
     SepFn f;
     f.local_point = mk(0.0f, 0.0f);
-    const Xf xa = sweep_xf(sa, t1), xb = sweep_xf(sb, t1);
+    Xf xa, xb;
+    sweep_xf2(sa, sb, t1, xa, xb);
     if (cache.count == 1) {
         f.type = SEP_POINTS;
         const V2 point_a = mul(xa, pa.v[cache.ia[0]]);
@@ -326,7 +326,8 @@ __device__ SepFn sep_init(const SimplexCache& cache, const DistProxy& pa, const 
 
 __device__ float sep_find_min(const SepFn& f, const DistProxy& pa, const Sweep& sa, const DistProxy& pb, const Sweep& sb,
                               int& ia, int& ib, float t) {
-    const Xf xa = sweep_xf(sa, t), xb = sweep_xf(sb, t);
+    Xf xa, xb;
+    sweep_xf2(sa, sb, t, xa, xb);
     if (f.type == SEP_POINTS) {
         ia = support(pa, mul_t(xa.q, f.axis));
         ib = support(pb, mul_t(xb.q, neg(f.axis)));
@@ -351,7 +352,8 @@ __device__ float sep_find_min(const SepFn& f, const DistProxy& pa, const Sweep& 
 
 __device__ float sep_evaluate(const SepFn& f, const DistProxy& pa, const Sweep& sa, const DistProxy& pb, const Sweep& sb,
                               int ia, int ib, float t) {
-    const Xf xa = sweep_xf(sa, t), xb = sweep_xf(sb, t);
+    Xf xa, xb;
+    sweep_xf2(sa, sb, t, xa, xb);
     if (f.type == SEP_POINTS) {
         const V2 point_a = mul(xa, pa.v[ia]), point_b = mul(xb, pb.v[ib]);
         return dot(sub(point_b, point_a), f.axis);
@@ -393,7 +395,8 @@ __device__ void time_of_impact(const DistProxy& pa, Sweep sa, const DistProxy& p
     cache.count = 0;
     cache.metric = 0.0f;
     for (int iter = 0;;) {
-        const Xf xa = sweep_xf(sa, t1), xb = sweep_xf(sb, t1);
+        Xf xa, xb;
+        sweep_xf2(sa, sb, t1, xa, xb);
         const float distance = gjk_distance(pa, xa, pb, xb, cache);
         if (distance <= 0.0f) {
             state = B2G_TOI_OVERLAPPED;

@@ -34,13 +34,15 @@
  * The solver's position sweeps are chains of these calls (two bodies, two points), so their length
  * is what counts: about 40 dependent operations here. The earlier form (a 1/32 table, pairs throughout,
  * and the double routine for x = 0, the angle of most static bodies) took 4.0 us per colour of the
- * 210-box pyramid's position sweeps, this one takes 1.8 us. tests/trig_check.cpp compares the two routines on every float in
+ * 210-box pyramid's position sweeps, this one takes 1.3 us (a call 380 -> 220 cycles against this file's
+ * form with branches, integer conversions and a normalised remainder). tests/trig_check.cpp compares the two routines on every float in
  * the fast range.
  */
 #ifndef B2G_TRIG_H
 #define B2G_TRIG_H
 
 #include <math.h>
+#include <string.h>
 
 #if defined(__CUDACC__)
 #define B2G_HD __host__ __device__ __forceinline__
@@ -146,75 +148,111 @@ B2G_HD float b2g_fmaf_(float a, float b, float c) {
 #endif
 }
 
-/* sin(x), cos(x) for f32 x: the same results as b2g_sincosf_ref. */
-B2G_HD void b2g_sincosf(float x, float* out_s, float* out_c)
+/* The double routine as the fast path calls it: on the device a function of its own, so that its 150
+ * instructions are not in the loops that call b2g_sincosf (the kernel of a small world waited more than
+ * half of its cycles an instruction for instruction fetches). */
+#if defined(__CUDACC__)
+static __device__ __noinline__ float2 b2g_sincosf_slow_dev(float x) {
+    float2 r;
+    b2g_sincosf_ref(x, &r.x, &r.y);
+    return r;
+}
+#endif
+B2G_HD void b2g_sincosf_slow_(float x, float* out_s, float* out_c) {
+#if defined(__CUDA_ARCH__)
+    const float2 r = b2g_sincosf_slow_dev(x);
+    *out_s = r.x;
+    *out_c = r.y;
+#else
+    b2g_sincosf_ref(x, out_s, out_c);
+#endif
+}
+
+B2G_HD int b2g_f2i_(float v) {
+#if defined(__CUDA_ARCH__)
+    return __float_as_int(v);
+#else
+    int i;
+    memcpy(&i, &v, 4);
+    return i;
+#endif
+}
+B2G_HD float b2g_flip_(float v, int sign_bit) {  /* v with its sign flipped where sign_bit's bit 31 is set */
+#if defined(__CUDA_ARCH__)
+    return __int_as_float(__float_as_int(v) ^ (sign_bit & (int)0x80000000));
+#else
+    return sign_bit < 0 ? -v : v;
+#endif
+}
+
+/* The fast path for any x: whether its results are certain. Without a branch, so that two calls (a
+ * constraint's two bodies) run side by side; nearest integers by the 1.5 * 2^23 shift, whose bits are the
+ * integer too. */
+B2G_HD bool b2g_sincosf_try_(float x, float* out_s, float* out_c)
 {
-    const float ax = x < 0.0f ? -x : x;
-    if (!(ax <= 8192.0f)) {
-        b2g_sincosf_ref(x, out_s, out_c);
-        return;
-    }
-    /* r = x - k*pi/2 as rh + rl */
-    const float kf = rintf(x * 0x1.45f306p-1f);
+    const float shifter = 0x1.8p23f;
+    /* x - k*pi/2 = t + e */
+    const float km = b2g_fmaf_(x, 0x1.45f306p-1f, shifter);
+    const float kf = km - shifter;
     const float a = b2g_fmaf_(-kf, 0x1.921fb6p+0f, x);
     const float p = kf * -0x1.777a5cp-25f;
     const float pe = b2g_fmaf_(kf, -0x1.777a5cp-25f, -p);
-    const float t = a - p;                       /* t + e = a - p exactly (two-sum) */
+    const float t = a - p;                       /* and the rest exactly (two-sum) */
     const float bb = t - a;
-    float e = (a - (t - bb)) - (p + bb);
-    e = b2g_fmaf_(kf, 0x1.ee59dap-50f, e - pe);
-    const float rh = t + e;
-    const float rl = e - (rh - t);
-    /* r = j/512 + d */
-    const float jf = rintf(rh * 512.0f);
-    const float dh = b2g_fmaf_(jf, -0x1.0p-9f, rh);  /* exact */
-    const int j = (int)jf;
-    const int aj = j < 0 ? -j : j;
-    float sth, stl, cth, ctl;
+    const float e = b2g_fmaf_(kf, 0x1.ee59dap-50f, ((a - (t - bb)) - (p + bb)) - pe);
+    /* t + e = j/512 + (d + e) */
+    const float jm = b2g_fmaf_(t, 512.0f, shifter);
+    const float jf = jm - shifter;
+    const float d = b2g_fmaf_(jf, -0x1.0p-9f, t);  /* exact */
+    const int j = b2g_f2i_(jm) - 0x4b400000;
+    const unsigned aj = (unsigned)(j < 0 ? -j : j);
+    const unsigned at = aj < (unsigned)b2g_sc_rows ? aj : 0u;  /* always so for |x| <= 8192 */
 #if defined(__CUDA_ARCH__)
-    const float4 row = b2g_sc_table_dev[aj];
-    sth = row.x;
-    stl = row.y;
-    cth = row.z;
-    ctl = row.w;
+    const float4 row = b2g_sc_table_dev[at];
+    const float sth = b2g_flip_(row.x, j), stl = b2g_flip_(row.y, j), cth = row.z, ctl = row.w;
 #else
-    sth = b2g_sc_table_host[4 * aj];
-    stl = b2g_sc_table_host[4 * aj + 1];
-    cth = b2g_sc_table_host[4 * aj + 2];
-    ctl = b2g_sc_table_host[4 * aj + 3];
+    const float sth = b2g_flip_(b2g_sc_table_host[4 * at], j), stl = b2g_flip_(b2g_sc_table_host[4 * at + 1], j);
+    const float cth = b2g_sc_table_host[4 * at + 2], ctl = b2g_sc_table_host[4 * at + 3];
 #endif
-    if (j < 0) {
-        sth = -sth;
-        stl = -stl;
-    }
-    const float d2 = dh * dh;
-    /* sin d = dh + sd, cos d - 1 = m */
-    const float sd = b2g_fmaf_(dh * d2, b2g_fmaf_(d2, 0x1.111112p-7f, -0x1.555556p-3f), rl);
-    const float m = b2g_fmaf_(d2 * d2, 0x1.555556p-5f, b2g_fmaf_(-dh, rl, -0.5f * d2));
-    /* sin r = st + ct*sin d + st*m, cos r = ct - st*sin d + ct*m */
-    const float bh = cth * dh, bl = b2g_fmaf_(cth, dh, -bh);
+    const float d2 = d * d;
+    /* sin(d + e) = d + sd, cos(d + e) - 1 = m */
+    const float sd = b2g_fmaf_(d * d2, b2g_fmaf_(d2, 0x1.111112p-7f, -0x1.555556p-3f), e);
+    const float m = b2g_fmaf_(d2 * d2, 0x1.555556p-5f, b2g_fmaf_(-d, e, -0.5f * d2));
+    /* sin r = st + ct*sin(d + e) + st*m, cos r = ct - st*sin(d + e) + ct*m */
+    const float bh = cth * d, bl = b2g_fmaf_(cth, d, -bh);
     const float sh = sth + bh;                   /* |sth| >= |bh|, or sth = 0 */
-    float sl = bh - (sh - sth);
-    sl = sl + (((stl + bl) + b2g_fmaf_(cth, sd, ctl * dh)) + sth * m);
-    const float gh = sth * dh, gl = b2g_fmaf_(sth, dh, -gh);
+    const float sl = (bh - (sh - sth)) + (((stl + bl) + b2g_fmaf_(cth, sd, ctl * d)) + sth * m);
+    const float gh = sth * d, gl = b2g_fmaf_(sth, d, -gh);
     const float ch = cth - gh;
-    float cl = (cth - ch) - gh;
-    cl = cl + (((ctl - gl) - b2g_fmaf_(sth, sd, stl * dh)) + cth * m);
+    const float cl = ((cth - ch) - gh) + (((ctl - gl) - b2g_fmaf_(sth, sd, stl * d)) + cth * m);
     /* the rounding test */
     const float abs_err = kf != 0.0f ? 0x1.0p-60f : 0.0f;
     const float se = b2g_fmaf_(0x1.0p-42f, sh < 0.0f ? -sh : sh, abs_err);
     const float ce = b2g_fmaf_(0x1.0p-42f, ch, abs_err);
     const float s1 = sh + (sl + se), s2 = sh + (sl - se);
     const float c1 = ch + (cl + ce), c2 = ch + (cl - ce);
-    if (!(s1 == s2 && c1 == c2)) {
-        b2g_sincosf_ref(x, out_s, out_c);
-        return;
-    }
     /* quadrant k mod 4 */
-    const int q = (int)kf;
-    const float rs = (q & 1) ? c1 : s1, rc = (q & 1) ? s1 : c1;
-    *out_s = (q & 2) ? -rs : rs;
-    *out_c = ((q + 1) & 2) ? -rc : rc;
+    const int q = b2g_f2i_(km);
+    *out_s = b2g_flip_((q & 1) ? c1 : s1, q << 30);
+    *out_c = b2g_flip_((q & 1) ? s1 : c1, (q + 1) << 30);
+    const float ax = x < 0.0f ? -x : x;
+    return s1 == s2 && c1 == c2 && ax <= 8192.0f;
+}
+
+/* sin(x), cos(x) for f32 x: the same results as b2g_sincosf_ref. */
+B2G_HD void b2g_sincosf(float x, float* out_s, float* out_c)
+{
+    if (!b2g_sincosf_try_(x, out_s, out_c)) b2g_sincosf_slow_(x, out_s, out_c);
+}
+
+/* the same of two angles */
+B2G_HD void b2g_sincosf2(float x, float y, float* xs, float* xc, float* ys, float* yc)
+{
+    const bool okx = b2g_sincosf_try_(x, xs, xc), oky = b2g_sincosf_try_(y, ys, yc);
+    if (!(okx && oky)) {
+        if (!okx) b2g_sincosf_slow_(x, xs, xc);
+        if (!oky) b2g_sincosf_slow_(y, ys, yc);
+    }
 }
 
 #endif /* B2G_TRIG_H */

@@ -1564,7 +1564,7 @@ __global__ void __launch_bounds__(kBlock) k_solve_fixtures(const __grid_constant
  * blocks took 20 + 22 + 56 us for a 16-body world (each launch a memset of its counter besides) and
  * every barrier of their sweeps 1.4 us; here a barrier takes 0.3 us (one block: a __syncthreads) and the
  * passes follow each other without a launch. */
-__global__ void __launch_bounds__(kBlock) k_front(const __grid_constant__ DevWorld w, const __grid_constant__ StepParams sp,
+__global__ void __launch_bounds__(kBlock, 1) k_front(const __grid_constant__ DevWorld w, const __grid_constant__ StepParams sp,
                                                   int nparts, int passes) {
     pdl_entry();
     if (cluster_leaves(w)) return;
