@@ -136,6 +136,7 @@ enum {
     CNT_BP_MAX_AGE = 56,  /* passes a kept hierarchy may reach before a rebuild (0: rebuild every pass) */
     CNT_BP_WARP_VISITS = 57, /* the most node fetches one warp of the last traversal made */
     CNT_BP_WARP_CHECKS = 58, /* the most leaf checks one warp of the last traversal made */
+    CNT_LIST = 59,           /* colouring: constraints that keep no colour of the previous colouring */
     CNT_SIZE = 64
 };
 

@@ -7,8 +7,8 @@
  *
  * GPU formulation
  *   islands     lock-free union-find over touching contacts whose bodies are both
- *               non-static (the reference's DFS does not cross static bodies); the
- *               root is the smallest body index, so labels are deterministic. An
+ *               non-static (the reference's DFS does not cross static bodies); an
+ *               island's label is its smallest body index, so labels are deterministic. An
  *               island is solved if any member is awake; its members are woken.
  *   constraints the touching, enabled, non-sensor contacts of solved islands, compacted
  *               in contact-table order by a scan.
@@ -66,6 +66,15 @@ __device__ __forceinline__ void agg_atomic_min(unsigned* words, int key, unsigne
     const unsigned m = __reduce_min_sync(peers, v);
     if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicMin(&words[key], m);
 }
+/* a place in a list whose length is *counter, for every lane that executes this */
+__device__ __forceinline__ int agg_slot(int* counter) {
+    const unsigned act = __activemask();
+    const int lane = (int)(threadIdx.x & 31), leader = __ffs(act) - 1;
+    int base = 0;
+    if (lane == leader) base = atomicAdd(counter, __popc(act));
+    base = __shfl_sync(act, base, leader);
+    return base + __popc(act & ((1u << lane) - 1u));
+}
 /* a counter incremented by every lane that executes this */
 __device__ __forceinline__ void agg_increment(int* counter) {
     const unsigned act = __activemask();
@@ -73,6 +82,19 @@ __device__ __forceinline__ void agg_increment(int* counter) {
 }
 
 /* ---------------- islands ---------------- */
+/* Which of two roots stays one: the smaller by a hash of its index. Linked by the index itself, the rows
+ * and columns of a pile become chains as long as the pile while thousands of threads link at once, and every
+ * find walks them in L2; linked in hash order the trees stay logarithmic (islands of 3001 bodies 64 -> 35 us,
+ * of the 210-box pyramid 24 -> 18). hash32 is a bijection: no two roots are equal in it. */
+__device__ __forceinline__ uint32_t hash32(uint32_t x) {
+    x ^= x >> 16;
+    x *= 0x7feb352dU;
+    x ^= x >> 15;
+    x *= 0x846ca68bU;
+    x ^= x >> 16;
+    return x;
+}
+
 /* Other SMs relink roots during the union pass, and a link cached in this SM's L1 may still show
  * a root that is no longer one: a find can stop early, at an ancestor. uf_union therefore goes on
  * from the parent a failed link returns (read in L2), so every retry climbs at least one link. */
@@ -87,12 +109,13 @@ __device__ __forceinline__ int uf_find(int* parent, int x) {
     return x;
 }
 
-/* link the larger root under the smaller; a failed link continues from the parent it found */
+/* link the root later in hash order under the other; a failed link continues from the parent it found */
 __device__ __forceinline__ void uf_union(int* parent, int a, int b) {
     a = uf_find(parent, a);
     b = uf_find(parent, b);
     for (int guard = 0; guard < 1 << 20 && a != b; ++guard) {
-        const int hi = a > b ? a : b, lo = a > b ? b : a;
+        const bool a_first = hash32((uint32_t)a) < hash32((uint32_t)b);
+        const int hi = a_first ? b : a, lo = a_first ? a : b;
         const int old = atomicCAS(&parent[hi], hi, lo);
         if (old == hi) return;
         a = uf_find(parent, old);
@@ -105,15 +128,6 @@ __device__ __forceinline__ bool contact_is_constraint(uint32_t cf) {
 }
 
 /* ---------------- colouring (cooperative) ---------------- */
-__device__ __forceinline__ uint32_t hash32(uint32_t x) {
-    x ^= x >> 16;
-    x *= 0x7feb352dU;
-    x ^= x >> 15;
-    x *= 0x846ca68bU;
-    x ^= x >> 16;
-    return x;
-}
-
 /* Block-wide exclusive scan of one int per thread (blockDim.x == kBlock); *total gets the sum. */
 __device__ __forceinline__ int block_scan_excl(int v, int* total) {
     __shared__ int s_warp[kBlock / 32];
@@ -416,11 +430,17 @@ __device__ __forceinline__ bool colour_pass(const DevWorld& w, int nparts) {
         w.cons_colour[k] = (keep && (kept >> 7) == stamp && ((kept >> 6) & 1u) == cls) ? (int)(kept & 63u) : -1;
     }
     for (int c = gtid; c < (P + 1) * kMaxColours; c += gsize) w.col_hist[c] = 0;
+    if (gtid == 0) w.cnt[CNT_LIST] = 0;
     if (!grid_barrier(w)) return false;
-    /* the kept colours are taken at their bodies */
+    /* the kept colours are taken at their bodies; the constraints without one are listed (in s_cons, free
+     * until the slots are placed): the rounds go over the list alone, as only its members ever offer */
+    int* list = w.s_cons;
     for (int k = gtid; k < n; k += gsize) {
         const int c = w.cons_colour[k];
-        if (c < 0) continue;
+        if (c < 0) {
+            list[agg_slot(&w.cnt[CNT_LIST])] = k;
+            continue;
+        }
         const int2 bd = w.c.body[w.cons_contact[k]];
         const size_t cm = w.cons_part[k] < 0 ? bc : 0;
         const unsigned long long bit = 1ull << c;
@@ -431,20 +451,20 @@ __device__ __forceinline__ bool colour_pass(const DevWorld& w, int nparts) {
         /* two "still uncoloured" counters alternate by round parity: round r counts into
          * [r & 1] and reads the previous round's result from [(r + 1) & 1] */
         w.cnt[CNT_UNCOLOURED] = 0;
-        w.cnt[CNT_UNCOLOURED + 1] = n;
         w.cnt[CNT_ROUNDS] = 0;
         w.cnt[CNT_TAIL] = 0;
     }
     if (!grid_barrier(w)) return false;
+    const int nlist = ((volatile int*)w.cnt)[CNT_LIST];
     int round = 0;
     for (;;) {
-        const int remaining = ((volatile int*)w.cnt)[CNT_UNCOLOURED + ((round + 1) & 1)];
+        const int remaining = round == 0 ? nlist : ((volatile int*)w.cnt)[CNT_UNCOLOURED + ((round + 1) & 1)];
         if (remaining <= 0) break;
         if (remaining <= kColourTail) {
             /* Few left: list them and let one block finish the rounds with block barriers. Its
              * rounds are the same rounds (priorities, first fit, overflow colours by round). */
-            for (int k = gtid; k < n; k += gsize)
-                if (w.cons_colour[k] < 0) {
+            for (int q = gtid; q < nlist; q += gsize)
+                if (const int k = list[q]; w.cons_colour[k] < 0) {
                     const int at = atomicAdd(&w.cnt[CNT_TAIL], 1);
                     if (at < kColourTail) w.col_tail[at] = k;
                 }
@@ -455,15 +475,16 @@ __device__ __forceinline__ bool colour_pass(const DevWorld& w, int nparts) {
         }
         if (round >= kMaxColours - kFirstFitColours) {
             /* cannot happen for rounds bounded by the maximum body degree; keep the kernel finite */
-            for (int k = gtid; k < n; k += gsize)
-                if (w.cons_colour[k] < 0) w.cons_colour[k] = kMaxColours - 1;
+            for (int q = gtid; q < nlist; q += gsize)
+                if (w.cons_colour[list[q]] < 0) w.cons_colour[list[q]] = kMaxColours - 1;
             if (gtid == 0) atomicOr((unsigned*)&w.cnt[CNT_STATUS], ST_COLOUR_OVERFLOW);
             break;
         }
         unsigned long long* offer = w.b_cmin + (size_t)(round & 1) * 2 * bc;
         unsigned long long* stale = w.b_cmin + (size_t)((round + 1) & 1) * 2 * bc;
         /* A: each uncoloured constraint offers its priority to its dynamic bodies */
-        for (int k = gtid; k < n; k += gsize) {
+        for (int q = gtid; q < nlist; q += gsize) {
+            const int k = list[q];
             const int2 bd = w.c.body[w.cons_contact[k]];
             const size_t cm = w.cons_part[k] < 0 ? bc : 0;
             if (round > 0) {
@@ -478,7 +499,8 @@ __device__ __forceinline__ bool colour_pass(const DevWorld& w, int nparts) {
         if (gtid == 0) w.cnt[CNT_UNCOLOURED + (round & 1)] = 0;
         if (!grid_barrier(w)) return false;
         /* B: local minima take the lowest colour free at both bodies */
-        for (int k = gtid; k < n; k += gsize) {
+        for (int q = gtid; q < nlist; q += gsize) {
+            const int k = list[q];
             if (w.cons_colour[k] >= 0) continue;
             const int2 bd = w.c.body[w.cons_contact[k]];
             const size_t cm = w.cons_part[k] < 0 ? bc : 0;
@@ -978,23 +1000,24 @@ __device__ __forceinline__ void part_load(const PartCtx& pc, const float4* glob)
     }
 }
 
-/* Islands and the constraint list in one cooperative launch, its passes separated by grid barriers:
- * reset, union over the constraints and joints (B2world::solve's DFS, private/dynamics/
- * b2_world.rs:375-491, as connected components), each body's root and its island's awake flag,
- * the solved bodies' flags, then the constraint list in contact order (each block counts its chunk
- * of the table, the chunks' counts give each block its offset, and a block scan places the block's
- * constraints). */
-__device__ __forceinline__ bool islands_pass(const DevWorld& w, int allow_sleep) {
-    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int gsize = gridDim.x * blockDim.x;
-    const int nb = w.n_bodies;
-    for (int b = gtid; b < nb; b += gsize) {
+/* Islands and the constraint list, as passes that each need the one before: reset, union over the
+ * constraints and joints (B2world::solve's DFS, private/dynamics/b2_world.rs:375-491, as connected
+ * components), each body's root with its island's smallest body and awake flag, the solved bodies' labels
+ * and flags, then the constraint list in contact order (each block counts its chunk of the table, the
+ * chunks' counts give each block its offset, and a block scan places the block's constraints). */
+__device__ __forceinline__ void islands_reset(const DevWorld& w, int allow_sleep) {
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < w.n_bodies; b += gridDim.x * blockDim.x) {
         w.b_island[b] = b;
+        w.isl_minsep[b] = 0xffffffffu;      /* of a root: its island's smallest body */
         w.isl_minsep[w.body_cap + b] = 0u;  /* "island has an awake member" */
         w.b_flags[b] &= ~BF_ISLAND;
         if (allow_sleep) w.isl_sleep[b] = kMaxFloat;
     }
-    if (!grid_barrier(w)) return false;
+}
+
+__device__ __forceinline__ void islands_union(const DevWorld& w) {
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int gsize = gridDim.x * blockDim.x;
     const int n = w.cnt[CNT_CONTACTS];
     for (int i = gtid; i < n; i += gsize) {
         if (!contact_is_constraint(w.c.flags[i])) continue;
@@ -1008,36 +1031,56 @@ __device__ __forceinline__ bool islands_pass(const DevWorld& w, int allow_sleep)
         if (is_static(fa) || is_static(fb) || !(fa & BF_ENABLED) || !(fb & BF_ENABLED)) continue;
         uf_union(w.b_island, bd.x, bd.y);
     }
-    if (!grid_barrier(w)) return false;
-    for (int b = gtid; b < nb; b += gsize) {
-        const int r = uf_find(w.b_island, b);
+}
+
+__device__ __forceinline__ void islands_roots(const DevWorld& w) {
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < w.n_bodies; b += gridDim.x * blockDim.x) {
+        /* only b's thread writes its link here (finds through b meanwhile skip links) */
+        int r = w.b_island[b];
+        for (int p = w.b_island[r]; p != r; p = w.b_island[r]) r = p;
+        w.b_island[b] = r;
         const uint32_t f = w.b_flags[b];
+        agg_atomic_min(w.isl_minsep, r, (unsigned)b);
         agg_atomic_or(w.isl_minsep + w.body_cap, r, ((f & BF_AWAKE) && (f & BF_ENABLED) && !is_static(f)) ? 1u : 0u);
     }
-    if (!grid_barrier(w)) return false;
-    for (int b = gtid; b < nb; b += gsize) {
-        int r = w.b_island[b];
-        r = w.b_island[r];
-        while (w.b_island[r] != r) r = w.b_island[r];
-        w.b_island[b] = r;
+}
+
+__device__ __forceinline__ void islands_labels(const DevWorld& w) {
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < w.n_bodies; b += gridDim.x * blockDim.x) {
+        const int r = w.b_island[b];
+        w.b_island[b] = (int)w.isl_minsep[r];
         const uint32_t f = w.b_flags[b];
         if (!is_static(f) && (f & BF_ENABLED) && w.isl_minsep[w.body_cap + r]) w.b_flags[b] = f | BF_AWAKE | BF_ISLAND;
     }
-    if (!grid_barrier(w)) return false;
-    /* the constraint list: this block's chunk of the contact table */
+}
+
+/* whether contact i is a constraint of this step's solve */
+__device__ __forceinline__ int solved_constraint(const DevWorld& w, int i) {
+    if (!contact_is_constraint(w.c.flags[i])) return 0;
+    const int2 bd = w.c.body[i];
+    return ((w.b_flags[bd.x] & BF_ISLAND) || (w.b_flags[bd.y] & BF_ISLAND)) ? 1 : 0;
+}
+
+/* this block's chunk of the contact table */
+__device__ __forceinline__ void constraint_chunk(int n, int* c0, int* c1) {
     const int chunk = (n + (int)gridDim.x - 1) / (int)gridDim.x;
-    const int c0 = min(n, (int)blockIdx.x * chunk), c1 = min(n, c0 + chunk);
-    auto selected = [&](int i) {
-        if (!contact_is_constraint(w.c.flags[i])) return 0;
-        const int2 bd = w.c.body[i];
-        return ((w.b_flags[bd.x] & BF_ISLAND) || (w.b_flags[bd.y] & BF_ISLAND)) ? 1 : 0;
-    };
+    *c0 = min(n, (int)blockIdx.x * chunk);
+    *c1 = min(n, *c0 + chunk);
+}
+
+__device__ __forceinline__ void constraints_count(const DevWorld& w) {
+    int c0, c1;
+    constraint_chunk(w.cnt[CNT_CONTACTS], &c0, &c1);
     int mine = 0;
-    for (int i = c0 + threadIdx.x; i < c1; i += blockDim.x) mine += selected(i);
+    for (int i = c0 + threadIdx.x; i < c1; i += blockDim.x) mine += solved_constraint(w, i);
     int block_total;
     block_scan_excl(mine, &block_total);
     if (threadIdx.x == 0) w.blk_tot[blockIdx.x] = (unsigned long long)block_total;
-    if (!grid_barrier(w)) return false;
+}
+
+__device__ __forceinline__ void constraints_list(const DevWorld& w) {
+    int c0, c1;
+    constraint_chunk(w.cnt[CNT_CONTACTS], &c0, &c1);
     int before_part = 0, all_part = 0;
     for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) {
         const int t = (int)w.blk_tot[q];
@@ -1050,7 +1093,7 @@ __device__ __forceinline__ bool islands_pass(const DevWorld& w, int allow_sleep)
     int carry = 0;
     for (int base = c0; base < c1; base += blockDim.x) {
         const int i = base + threadIdx.x;
-        const int sel = i < c1 ? selected(i) : 0;
+        const int sel = i < c1 ? solved_constraint(w, i) : 0;
         int tot;
         const int ex = block_scan_excl(sel, &tot);
         if (sel) {
@@ -1066,8 +1109,21 @@ __device__ __forceinline__ bool islands_pass(const DevWorld& w, int allow_sleep)
         }
         carry += tot;
     }
-    if (gtid == 0) w.cnt[CNT_CONS] = min(all, w.cons_cap);
-    return true;
+    if (blockIdx.x == 0 && threadIdx.x == 0) w.cnt[CNT_CONS] = min(all, w.cons_cap);
+}
+
+__device__ __forceinline__ void islands_pass(const DevWorld& w, int allow_sleep) {
+    islands_reset(w, allow_sleep);
+    grid_barrier(w);
+    islands_union(w);
+    grid_barrier(w);
+    islands_roots(w);
+    grid_barrier(w);
+    islands_labels(w);
+    grid_barrier(w);
+    constraints_count(w);
+    grid_barrier(w);
+    constraints_list(w);
 }
 
 /* k_solve runs 256 or 512 threads per block (cfg_solver_block); nothing in it depends on which */
@@ -1500,12 +1556,40 @@ __device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& 
     return true;
 }
 
-__global__ void __launch_bounds__(kBlock) k_islands(DevWorld w, int allow_sleep) {
+/* Outside of a cluster the passes are kernels of their own, at full occupancy: a pass over the contacts is
+ * a handful of dependent loads each, and a persistent kernel's 8 to 24 warps an SM waited for them (100k
+ * bodies in flight 58 -> 38 us, 250k boxes 186 -> 155). */
+__global__ void __launch_bounds__(kBlock) k_islands_reset(const __grid_constant__ DevWorld w, int allow_sleep) {
+    pdl_entry();
     B2G_RETURN_IF_ABORTED(w);
     phase_stamp(w, PH_COLLIDE);
     if (blockIdx.x == 0 && threadIdx.x == 0) w.cnt[CNT_BARRIER2] = 0;  /* k_colour's */
-    grid_barrier_start();
-    islands_pass(w, allow_sleep);
+    islands_reset(w, allow_sleep);
+}
+__global__ void __launch_bounds__(kBlock) k_islands_union(const __grid_constant__ DevWorld w) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    islands_union(w);
+}
+__global__ void __launch_bounds__(kBlock) k_islands_roots(const __grid_constant__ DevWorld w) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    islands_roots(w);
+}
+__global__ void __launch_bounds__(kBlock) k_islands_labels(const __grid_constant__ DevWorld w) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    islands_labels(w);
+}
+__global__ void __launch_bounds__(kBlock) k_constraints_count(const __grid_constant__ DevWorld w) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    constraints_count(w);
+}
+__global__ void __launch_bounds__(kBlock) k_constraints_list(const __grid_constant__ DevWorld w) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    constraints_list(w);
 }
 
 __global__ void __launch_bounds__(kBlock) k_colour(DevWorld w, int nparts) {
@@ -1622,23 +1706,17 @@ int coop_blocks(const void* fn, int num_sms) {
 
 }  // namespace
 
-/* k_islands runs one block per SM for a world of up to 64k bodies and more blocks per SM for larger
- * ones (up to what can be co-resident): its passes stride over all bodies and contacts, so a large
- * batch wants more threads in flight, while a small world wants the shortest grid barriers. */
 void launch_islands_and_constraints(const DevWorld& w, const StepParams& sp, cudaStream_t s) {
-    if (w.n_bodies > 0) {
-        static int resident = 0;
-        if (!resident) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, (const void*)k_islands, kBlock, 0);
-            resident = std::max(1, std::min(resident, 8));
-        }
-        const int per_sm = std::max(1, std::min(resident, w.n_bodies / 65536));
-        DevWorld wc = w;
-        int allow_sleep = sp.allow_sleep;
-        void* args[] = {&wc, &allow_sleep};
-        cudaLaunchCooperativeKernel((const void*)k_islands, dim3(w.num_sms * per_sm), dim3(kBlock), args, 0, s);
-        B2G_LAUNCHED(1);
-    }
+    if (w.n_bodies <= 0) return;
+    const int gb = grid_for(w.n_bodies, kBlock, w.num_sms * 8);
+    const int gc = grid_for(std::max(w.contact_cap, w.n_joints), kBlock, w.num_sms * 8);  /* blk_tot holds that many */
+    launch_pdl(k_islands_reset, gb, kBlock, 0, s, w, sp.allow_sleep);
+    launch_pdl(k_islands_union, gc, kBlock, 0, s, w);
+    launch_pdl(k_islands_roots, gb, kBlock, 0, s, w);
+    launch_pdl(k_islands_labels, gb, kBlock, 0, s, w);
+    launch_pdl(k_constraints_count, gc, kBlock, 0, s, w);
+    launch_pdl(k_constraints_list, gc, kBlock, 0, s, w);
+    B2G_LAUNCHED(6);
 }
 
 /* Parts of the part-local solve: about one per 256 proxies, at most one per SM, whatever the
@@ -1663,7 +1741,7 @@ bool use_parts(const DevWorld& w, int num_sms, bool allowed) {
 }
 
 void launch_colouring(const DevWorld& w, cudaStream_t s, int num_sms, bool parts) {
-    /* more blocks per SM for large worlds (as k_islands): the colouring's passes stride over every
+    /* more blocks per SM for large worlds: the colouring's passes stride over every
      * constraint and body */
     static int resident = 0;
     if (!resident) {
