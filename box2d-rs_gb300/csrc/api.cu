@@ -1407,18 +1407,33 @@ int step(World* w, float dt, int vi, int pi) {
 World* W(void* p) { return (World*)p; }
 
 /* b2g_body_state of bodies [first, first + count); thread 0 also copies the status word to
- * *status (host memory the device writes coherently) so the caller needs no second copy */
-__global__ void k_pack_states(DevWorld d, uint32_t first, uint32_t count, b2g_body_state* out, int* status) {
+ * *status (host memory the device writes coherently) so the caller needs no second copy. The states go
+ * out through shared memory, so that a warp's store is 512 contiguous bytes (128 where out is off a
+ * 16-byte boundary): across C2C a thread's own 32 bytes in 4-byte stores ran at 20 GB/s, 1.7 M bodies
+ * now at 167 GB/s (2.78 -> 0.33 ms). */
+constexpr int kPackBlock = 256;
+__global__ void __launch_bounds__(kPackBlock) k_pack_states(DevWorld d, uint32_t first, uint32_t count, b2g_body_state* out,
+                                                            int* status) {
+    __shared__ float4 s_state[2 * kPackBlock];
+    static_assert(sizeof(b2g_body_state) == 2 * sizeof(float4), "a state is two float4");
     if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = ((volatile int*)d.cnt)[CNT_STATUS];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const float4 xf = d.b_xf[first + i], pos = d.b_pos[first + i], vel = d.b_vel[first + i];
-        b2g_body_state s;
-        s.position = b2g_vec2{xf.x, xf.y};
-        s.angle = pos.z;
-        s.linear_velocity = b2g_vec2{vel.x, vel.y};
-        s.angular_velocity = vel.z;
-        s.world_center = b2g_vec2{pos.x, pos.y};
-        out[i] = s;
+    const bool wide = ((uintptr_t)out & 15u) == 0;
+    for (uint32_t base = blockIdx.x * kPackBlock; base < count; base += gridDim.x * kPackBlock) {
+        const uint32_t i = base + threadIdx.x, m = min((uint32_t)kPackBlock, count - base);
+        if (i < count) {
+            const float4 xf = d.b_xf[first + i], pos = d.b_pos[first + i], vel = d.b_vel[first + i];
+            s_state[2 * threadIdx.x] = make_float4(xf.x, xf.y, pos.z, vel.x);
+            s_state[2 * threadIdx.x + 1] = make_float4(vel.y, vel.z, pos.x, pos.y);
+        }
+        __syncthreads();
+        if (wide) {
+            float4* o = (float4*)(out + base);
+            for (uint32_t k = threadIdx.x; k < 2 * m; k += kPackBlock) o[k] = s_state[k];
+        } else {
+            float* o = (float*)(out + base);
+            for (uint32_t k = threadIdx.x; k < 8 * m; k += kPackBlock) o[k] = ((const float*)s_state)[k];
+        }
+        __syncthreads();
     }
 }
 
@@ -2092,7 +2107,7 @@ int b2g_get_body_states_async(void* p, uint32_t first, uint32_t count, b2g_body_
      * buffer two requests ago must have finished before it is overwritten */
     if (w->ring_used[i]) CUDA_OK(w, cudaStreamWaitEvent(w->stream, w->ev_copied[i], 0));
     const int grid = grid_for((int)count, 256, w->num_sms * 8);
-    k_pack_states<<<grid, 256, 0, w->stream>>>(w->d, first, count, w->d_ring[i], nullptr);
+    k_pack_states<<<grid, kPackBlock, 0, w->stream>>>(w->d, first, count, w->d_ring[i], nullptr);
     B2G_LAUNCHED(1);
     CUDA_OK(w, cudaEventRecord(w->ev_packed[i], w->stream));
     CUDA_OK(w, cudaStreamWaitEvent(w->copy_stream, w->ev_packed[i], 0));
@@ -2132,7 +2147,7 @@ int b2g_get_body_states(void* p, uint32_t first, uint32_t count, b2g_body_state*
         const int grid = grid_for((int)count, 256, w->num_sms * 8);
         if (w->pageable) {
             int status = 0;
-            k_pack_states<<<grid, 256, 0, w->stream>>>(w->d, first, count, out, &status);
+            k_pack_states<<<grid, kPackBlock, 0, w->stream>>>(w->d, first, count, out, &status);
             B2G_LAUNCHED(1);
             CUDA_OK(w, cudaGetLastError());
             CUDA_OK(w, cudaStreamSynchronize(w->stream));
@@ -2145,7 +2160,7 @@ int b2g_get_body_states(void* p, uint32_t first, uint32_t count, b2g_body_state*
                 CUDA_OK(w, cudaMalloc((void**)&w->d_states, count * sizeof(b2g_body_state)));
                 w->d_states_cap = (int)count;
             }
-            k_pack_states<<<grid, 256, 0, w->stream>>>(w->d, first, count, w->d_states, nullptr);
+            k_pack_states<<<grid, kPackBlock, 0, w->stream>>>(w->d, first, count, w->d_states, nullptr);
             B2G_LAUNCHED(1);
             CUDA_OK(w, cudaMemcpyAsync(out, w->d_states, count * sizeof(b2g_body_state), cudaMemcpyDeviceToHost,
                                        w->stream));
