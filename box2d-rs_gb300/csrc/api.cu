@@ -84,7 +84,7 @@ struct TapeHost {
     AdjWork work{};
     std::vector<void*> work_mem;
     size_t work_bytes = 0;
-    int work_slots = 0, work_vi = 0, work_pi = 0;
+    int work_slots = 0, work_vi = 0, work_pi = 0, work_groups = 0;
     unsigned mismatches = 0;
 };
 
@@ -221,7 +221,7 @@ void tape_free_work(TapeHost* t) {
     for (void* p : t->work_mem) cudaFree(p);
     t->work_mem.clear();
     t->work_bytes = 0;
-    t->work_slots = t->work_vi = t->work_pi = 0;
+    t->work_slots = t->work_vi = t->work_pi = t->work_groups = 0;
 }
 
 void tape_free(World* w) {
@@ -3518,44 +3518,58 @@ int tape_status(World* w, TapeHost* t, long long* steps, long long* slots) {
     return B2G_OK;
 }
 
-/* work buffers for segments of ckpt_every steps with up to `slots` constraints */
-int tape_work(World* w, TapeHost* t, int slots, int vi, int pi) {
+/* Work buffers for segments of ckpt_every steps with up to `slots` constraints, `groups` of them replayed
+ * side by side, fewer where they would take more than kReplayBytes or the memory is not there. */
+constexpr size_t kReplayBytes = (size_t)8 << 30;
+
+int tape_work(World* w, TapeHost* t, int slots, int vi, int pi, int groups) {
     if (slots < 1) slots = 1;
     if (vi < 1) vi = 1;
     if (pi < 1) pi = 1;
-    if (!t->work_mem.empty() && slots <= t->work_slots && vi <= t->work_vi && pi <= t->work_pi) return B2G_OK;
-    tape_free_work(t);
-    AdjWork& a = t->work;
-    a = AdjWork{};
     const size_t nb = (size_t)t->n_bodies, seg = (size_t)t->ckpt_every, ns = (size_t)slots;
-    std::vector<void*>& m = t->work_mem;
-    size_t& by = t->work_bytes;
+    const size_t each = sizeof(float4) * (nb * (2 + 3 * seg) + ns * (1 + seg * (3 * (size_t)vi + 2 + 2 * (size_t)pi))) +
+                        ns * sizeof(adj::VC<float>);
+    groups = std::max(1, (int)std::min<size_t>((size_t)groups, kReplayBytes / std::max<size_t>(each, 1)));
+    if (!t->work_mem.empty() && slots <= t->work_slots && vi <= t->work_vi && pi <= t->work_pi && groups <= t->work_groups)
+        return B2G_OK;
+    AdjWork& a = t->work;
     int rc = B2G_OK;
-    auto A = [&](auto** ptr, size_t n) {
-        if (rc == B2G_OK) rc = talloc(w, m, by, ptr, n);
-    };
-    A(&a.cur_pos, nb);
-    A(&a.cur_vel, nb);
-    A(&a.ws_pos, seg * nb);
-    A(&a.ws_vel1, seg * nb);
-    A(&a.ws_vel2, seg * nb);
-    A(&a.vc, ns);
-    A(&a.imp, ns);
-    A(&a.wv, seg * vi * ns * 3);
-    A(&a.ww, seg * ns * 2);
-    A(&a.wp, seg * pi * ns * 2);
-    A(&a.g_pos, nb);
-    A(&a.g_vel, nb);
-    A(&a.gvc, ns);
-    A(&a.g_imp, ns);
-    A(&a.g_end[0], ns);
-    A(&a.g_end[1], ns);
-    A(&a.cnt, (size_t)CNT_SIZE);
-    A(&a.mismatch, (size_t)1);
+    for (;; groups = (groups + 1) / 2) {
+        tape_free_work(t);
+        a = AdjWork{};
+        std::vector<void*>& m = t->work_mem;
+        size_t& by = t->work_bytes;
+        rc = B2G_OK;
+        auto A = [&](auto** ptr, size_t n) {
+            if (rc == B2G_OK) rc = talloc(w, m, by, ptr, n);
+        };
+        const size_t g = (size_t)groups;
+        A(&a.cur_pos, g * nb);
+        A(&a.cur_vel, g * nb);
+        A(&a.ws_pos, g * seg * nb);
+        A(&a.ws_vel1, g * seg * nb);
+        A(&a.ws_vel2, g * seg * nb);
+        A(&a.vc, g * ns);
+        A(&a.imp, g * ns);
+        A(&a.wv, g * seg * vi * ns * 3);
+        A(&a.ww, g * seg * ns * 2);
+        A(&a.wp, g * seg * pi * ns * 2);
+        A(&a.g_pos, nb);
+        A(&a.g_vel, nb);
+        A(&a.gvc, ns);
+        A(&a.g_imp, ns);
+        A(&a.g_end[0], ns);
+        A(&a.g_end[1], ns);
+        A(&a.cnt, g * CNT_SIZE);
+        A(&a.mismatch, (size_t)1);
+        if (rc == B2G_OK || groups == 1) break;
+        cudaGetLastError();
+    }
     if (rc != B2G_OK) {
         tape_free_work(t);
         return rc;
     }
+    t->work_groups = groups;
     t->work_slots = slots;
     t->work_vi = vi;
     t->work_pi = pi;
@@ -3755,9 +3769,17 @@ int b2g_backward(void* p, const b2g_body_state* d_final, b2g_body_state* d_initi
         max_vi = std::max(max_vi, st[i].vi);
         max_pi = std::max(max_pi, st[i].pi);
     }
-    rc = tape_work(w, t, max_slots, max_vi, max_pi);
+    const int every = t->ckpt_every;
+    const int nseg = (T + every - 1) / every;
+    const int parts = use_parts(w->d, w->num_sms, w->part_solve) ? part_count(w->d, w->num_sms) : 0;
+    rc = tape_work(w, t, max_slots, max_vi, max_pi,
+                   std::min(std::max(nseg, 1), adjoint_groups(max_slots, parts, w->num_sms)));
     if (rc != B2G_OK) return rc;
+    /* (the buffers may be larger than this tape needs, so that the launch's limits are checked again) */
+    const int groups = std::max(1, std::min(t->work_groups, adjoint_groups(t->work.max_slots, parts, w->num_sms)));
     AdjWork a = t->work;
+    a.steps = T;
+    a.final_ckpt = tape_final_index(t);
     a.t = t->d;
     a.b_mass = w->d.b_mass;
     a.b_damp = w->d.b_damp;
@@ -3783,28 +3805,30 @@ int b2g_backward(void* p, const b2g_body_state* d_final, b2g_body_state* d_initi
     CUDA_OK(w, cudaMemcpyAsync(a.g_vel, gvel.data(), nb * sizeof(float4), cudaMemcpyHostToDevice, s));
     CUDA_OK(w, cudaMemsetAsync(a.g_end[0], 0, (size_t)a.max_slots * sizeof(float4), s));
     CUDA_OK(w, cudaMemsetAsync(a.g_end[1], 0, (size_t)a.max_slots * sizeof(float4), s));
-    CUDA_OK(w, cudaMemsetAsync(a.cnt, 0, CNT_SIZE * sizeof(int), s));
+    CUDA_OK(w, cudaMemsetAsync(a.cnt, 0, (size_t)t->work_groups * CNT_SIZE * sizeof(int), s));
     CUDA_OK(w, cudaMemsetAsync(a.mismatch, 0, sizeof(unsigned), s));
-    const int every = t->ckpt_every;
-    const int nseg = (T + every - 1) / every;
-    for (int g = nseg - 1; g >= 0; --g) {
-        a.t0 = g * every;
-        a.t1 = std::min(T, a.t0 + every);
-        const size_t eo = (size_t)(a.t1 == T ? tape_final_index(t) : a.t1 / every) * nb;
-        a.end_pos = t->d.ckpt_pos + eo;
-        a.end_vel = t->d.ckpt_vel + eo;
-        const int e = launch_adjoint_segment(a, s, w->num_sms);
+    std::vector<int> dcnt((size_t)t->work_groups * CNT_SIZE, 0);
+    int status = 0;
+    for (int end = nseg; end > 0; end -= groups) {
+        a.first_seg = std::max(0, end - groups);
+        int e = launch_adjoint_replay(a, end - a.first_seg, parts, s, w->num_sms);
+        for (int g = end - 1; g >= a.first_seg && e == 0; --g) e = launch_adjoint_reverse(a, g, parts, s, w->num_sms);
         if (e != 0) return fail(w, B2G_ERR_CUDA, cudaGetErrorString((cudaError_t)e));
+        if (a.first_seg > 0) {  /* the next replays reset the groups' counters */
+            CUDA_OK(w, cudaMemcpyAsync(dcnt.data(), a.cnt, dcnt.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+            CUDA_OK(w, cudaStreamSynchronize(s));
+            for (size_t g = 0; g < dcnt.size(); g += CNT_SIZE) status |= dcnt[g + CNT_STATUS];
+        }
     }
-    int dcnt[CNT_SIZE] = {};
     unsigned mism = 0;
     CUDA_OK(w, cudaMemcpyAsync(gpos.data(), a.g_pos, nb * sizeof(float4), cudaMemcpyDeviceToHost, s));
     CUDA_OK(w, cudaMemcpyAsync(gvel.data(), a.g_vel, nb * sizeof(float4), cudaMemcpyDeviceToHost, s));
     CUDA_OK(w, cudaMemcpyAsync(fpos.data(), t->d.ckpt_pos, nb * sizeof(float4), cudaMemcpyDeviceToHost, s));
-    CUDA_OK(w, cudaMemcpyAsync(dcnt, a.cnt, sizeof(dcnt), cudaMemcpyDeviceToHost, s));
+    CUDA_OK(w, cudaMemcpyAsync(dcnt.data(), a.cnt, dcnt.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
     CUDA_OK(w, cudaMemcpyAsync(&mism, a.mismatch, sizeof(mism), cudaMemcpyDeviceToHost, s));
     CUDA_OK(w, cudaStreamSynchronize(s));
-    if (dcnt[CNT_STATUS] & ST_BARRIER_TIMEOUT)
+    for (size_t g = 0; g < dcnt.size(); g += CNT_SIZE) status |= dcnt[g + CNT_STATUS];
+    if (status & ST_BARRIER_TIMEOUT)
         return fail(w, B2G_ERR_TIMEOUT, "a grid barrier of the backward pass timed out");
     t->mismatches = mism;
     /* dL/d(initial origin, angle): c0 = p0 + R(a0) lc */

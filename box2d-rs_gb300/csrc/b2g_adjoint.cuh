@@ -26,6 +26,14 @@
 #include <cmath>
 #endif
 
+/* A loop over a constraint's points, at most two: unrolled on the device, so that the arrays it indexes stay
+ * in registers (as loops over the count they were local memory: 750 bytes of it in the reverse kernel). */
+#if defined(__CUDA_ARCH__)
+#define B2G_POINTS _Pragma("unroll")
+#else
+#define B2G_POINTS
+#endif
+
 namespace b2g {
 namespace adj {
 
@@ -79,6 +87,12 @@ B2G_HD R2<double> rot_t(double a) {
     q.s = sin(a);
     q.c = cos(a);
     return q;
+}
+/* the rotations of a constraint's bodies, side by side */
+B2G_HD void rot2_t(float a, float b, R2<float>& qa, R2<float>& qb) { b2g_sincosf2(a, b, &qa.s, &qa.c, &qb.s, &qb.c); }
+B2G_HD void rot2_t(double a, double b, R2<double>& qa, R2<double>& qb) {
+    qa = rot_t(a);
+    qb = rot_t(b);
 }
 template <class T> B2G_HD P2<T> mulq(R2<T> q, P2<T> v) { return p2(q.c * v.x - q.s * v.y, q.s * v.x + q.c * v.y); }
 /* d/da of R(a) v */
@@ -171,7 +185,9 @@ B2G_HD void world_manifold(const SlotStatic& s, R2<T> qA, P2<T> pA, R2<T> qB, P2
     } else if (s.mtype == ADJ_FACE_A) {
         normal = mulq(qA, ln);
         P2<T> plane = xf_apply(qA, pA, lpt);
-        for (int j = 0; j < s.count; ++j) {
+        B2G_POINTS
+        for (int j = 0; j < 2; ++j) {
+            if (j >= s.count) break;
             P2<T> clip = xf_apply(qB, pB, lp[j]);
             P2<T> ca = clip + (rA - dot(clip - plane, normal)) * normal;
             P2<T> cb = clip - rB * normal;
@@ -180,7 +196,9 @@ B2G_HD void world_manifold(const SlotStatic& s, R2<T> qA, P2<T> pA, R2<T> qB, P2
     } else {
         normal = mulq(qB, ln);
         P2<T> plane = xf_apply(qB, pB, lpt);
-        for (int j = 0; j < s.count; ++j) {
+        B2G_POINTS
+        for (int j = 0; j < 2; ++j) {
+            if (j >= s.count) break;
             P2<T> clip = xf_apply(qA, pA, lp[j]);
             P2<T> cb = clip + (rB - dot(clip - plane, normal)) * normal;
             P2<T> ca = clip - rA * normal;
@@ -199,7 +217,8 @@ B2G_HD void init_slot(const SlotStatic& s, P2<T> cA, T aA, P2<T> cB, T aB, P2<T>
     const int fz_vcount = frozen ? vc.vcount : 0;
     const int fz_bias[2] = {frozen ? vc.bias_on[0] : 0, frozen ? vc.bias_on[1] : 0};
     const T mA = (T)s.mA, mB = (T)s.mB, iA = (T)s.iA, iB = (T)s.iB;
-    R2<T> qA = rot_t(aA), qB = rot_t(aB);
+    R2<T> qA, qB;
+    rot2_t(aA, aB, qA, qB);
     P2<T> pA = cA - mulq(qA, lcA), pB = cB - mulq(qB, lcB);
     P2<T> wp[2] = {p2((T)0, (T)0), p2((T)0, (T)0)};
     world_manifold(s, qA, pA, qB, pB, vc.n, wp);
@@ -209,7 +228,9 @@ B2G_HD void init_slot(const SlotStatic& s, P2<T> cA, T aA, P2<T> cB, T aB, P2<T>
         vc.nm[j] = vc.tm[j] = vc.bias[j] = (T)0;
         vc.bias_on[j] = 0;
     }
-    for (int j = 0; j < s.count; ++j) {
+    B2G_POINTS
+    for (int j = 0; j < 2; ++j) {
+        if (j >= s.count) break;
         vc.ra[j] = wp[j] - cA;
         vc.rb[j] = wp[j] - cB;
         T rnA = cross(vc.ra[j], vc.n), rnB = cross(vc.rb[j], vc.n);
@@ -251,7 +272,9 @@ template <class T>
 B2G_HD void warm_slot(const SlotStatic& s, const VC<T>& vc, const T ni[2], const T ti[2], P2<T>& vA, T& wA, P2<T>& vB,
                       T& wB) {
     const P2<T> t = cross_vs(vc.n, (T)1);
-    for (int j = 0; j < vc.vcount; ++j) {
+    B2G_POINTS
+    for (int j = 0; j < 2; ++j) {
+        if (j >= vc.vcount) break;
         P2<T> P = ni[j] * vc.n + ti[j] * t;
         wA -= (T)s.iA * cross(vc.ra[j], P);
         vA -= (T)s.mA * P;
@@ -273,7 +296,9 @@ B2G_HD void solve_velocity(const SlotStatic& s, const VC<T>& vc, T ni[2], T ti[2
     const T mA = (T)s.mA, mB = (T)s.mB, iA = (T)s.iA, iB = (T)s.iB;
     const P2<T> n = vc.n, t = cross_vs(vc.n, (T)1);
     const T friction = (T)s.friction;
-    for (int j = 0; j < vc.vcount; ++j) {
+    B2G_POINTS
+    for (int j = 0; j < 2; ++j) {
+        if (j >= vc.vcount) break;
         P2<T> dv = ((vB + cross_sv(wB, vc.rb[j])) - vA) - cross_sv(wA, vc.ra[j]);
         T vt = dot(dv, t) - (T)0;
         T lambda = vc.tm[j] * (-vt);
@@ -437,8 +462,11 @@ B2G_HD T solve_position(const SlotStatic& s, const P2<T>& lcA, const P2<T>& lcB,
                         unsigned char dec[2], bool frozen) {
     const T mA = (T)s.mA, mB = (T)s.mB, iA = (T)s.iA, iB = (T)s.iB;
     T minSep = (T)0;
-    for (int j = 0; j < s.count; ++j) {
-        R2<T> qA = rot_t(aA), qB = rot_t(aB);
+    B2G_POINTS
+    for (int j = 0; j < 2; ++j) {
+        if (j >= s.count) break;
+        R2<T> qA, qB;
+        rot2_t(aA, aB, qA, qB);
         P2<T> pA = cA - mulq(qA, lcA), pB = cB - mulq(qB, lcB);
         P2<T> normal, point;
         T sep;
@@ -523,7 +551,9 @@ B2G_HD void warm_slot_bwd(const SlotStatic& s, const VC<T>& vc, const T ni[2], c
                           P2<T> gvB, T gwB, T gni[2], T gti[2], VCGrad<T>& g) {
     const P2<T> t = cross_vs(vc.n, (T)1);
     P2<T> gt = p2((T)0, (T)0);
-    for (int j = 0; j < vc.vcount; ++j) {
+    B2G_POINTS
+    for (int j = 0; j < 2; ++j) {
+        if (j >= vc.vcount) break;
         P2<T> P = ni[j] * vc.n + ti[j] * t;
         P2<T> gP = p2((T)0, (T)0);
         apply_bwd((T)-1, (T)s.mA, (T)s.iA, vc.ra[j], P, gvA, gwA, gP, g.ra[j]);
@@ -559,7 +589,9 @@ B2G_HD void solve_velocity_bwd(const SlotStatic& s, const VC<T>& vc, const VelDe
     T ni[2] = {ni_in[0], ni_in[1]}, ti[2] = {ti_in[0], ti_in[1]};
     P2<T> fvA[2], fvB[2];
     T fwA[2], fwB[2], flam[2];
-    for (int j = 0; j < vc.vcount; ++j) {
+    B2G_POINTS
+    for (int j = 0; j < 2; ++j) {
+        if (j >= vc.vcount) break;
         fvA[j] = vA; fwA[j] = wA; fvB[j] = vB; fwB[j] = wB;
         P2<T> dv = ((vB + cross_sv(wB, vc.rb[j])) - vA) - cross_sv(wA, vc.ra[j]);
         T vt = dot(dv, t) - (T)0;
@@ -671,7 +703,9 @@ B2G_HD void solve_velocity_bwd(const SlotStatic& s, const VC<T>& vc, const VelDe
         gni[1] = ga.y;
     }
     /* ---- friction part, reversed ---- */
-    for (int j = vc.vcount - 1; j >= 0; --j) {
+    B2G_POINTS
+    for (int j = 1; j >= 0; --j) {
+        if (j >= vc.vcount) continue;
         const T lambda = flam[j];
         const P2<T> P = lambda * t;
         P2<T> gP = p2((T)0, (T)0);
@@ -751,7 +785,9 @@ B2G_HD void world_manifold_bwd(const SlotStatic& s, R2<T> qA, P2<T> pA, R2<T> qB
     P2<T> gnr = faceA ? gn : -gn;
     T gsR = (T)0, gcR = (T)0, gsI = (T)0, gcI = (T)0;
     P2<T> gpR = p2((T)0, (T)0), gpI = p2((T)0, (T)0), gplane = p2((T)0, (T)0);
-    for (int j = 0; j < s.count; ++j) {
+    B2G_POINTS
+    for (int j = 0; j < 2; ++j) {
+        if (j >= s.count) break;
         P2<T> clip = xf_apply(qI, pI, lp[j]);
         T u = rR - dot(clip - plane, nr);
         /* wp = 0.5 ((clip + u nr) + (clip - rI nr)) */
@@ -814,7 +850,9 @@ B2G_HD void init_slot_bwd(const SlotStatic& s, P2<T> cA, T aA, P2<T> cB, T aB, P
         cross_bwd(vc.rb[1], n, grn2B, g.rb[1], g.n);
     }
     P2<T> gwp[2] = {p2((T)0, (T)0), p2((T)0, (T)0)};
-    for (int j = s.count - 1; j >= 0; --j) {
+    B2G_POINTS
+    for (int j = 1; j >= 0; --j) {
+        if (j >= s.count) continue;
         const P2<T> ra = vc.ra[j], rb = vc.rb[j];
         if (vc.bias_on[j]) {
             P2<T> dv = ((vB + cross_sv(wB, rb)) - vA) - cross_sv(wA, ra);
@@ -842,7 +880,8 @@ B2G_HD void init_slot_bwd(const SlotStatic& s, P2<T> cA, T aA, P2<T> cB, T aB, P
         gcB -= g.rb[j];
     }
     tangent_bwd(gt, g.n);
-    R2<T> qA = rot_t(aA), qB = rot_t(aB);
+    R2<T> qA, qB;
+    rot2_t(aA, aB, qA, qB);
     P2<T> pA = cA - mulq(qA, lcA), pB = cB - mulq(qB, lcB);
     T gsA = (T)0, gcA_ = (T)0, gsB = (T)0, gcB_ = (T)0;
     P2<T> gpA = p2((T)0, (T)0), gpB = p2((T)0, (T)0);
@@ -928,10 +967,15 @@ B2G_HD void solve_position_bwd(const SlotStatic& s, const P2<T>& lcA, const P2<T
                                const unsigned char dec[2], P2<T>& gcA, T& gaA, P2<T>& gcB, T& gaB) {
     const T mA = (T)s.mA, mB = (T)s.mB, iA = (T)s.iA, iB = (T)s.iB;
     P2<T> pc[2], pcB[2];
-    T pa[2], paB[2];
-    for (int j = 0; j < s.count; ++j) {  /* forward again to get the pre-point poses */
-        pc[j] = cA; pa[j] = aA; pcB[j] = cB; paB[j] = aB;
-        R2<T> qA = rot_t(aA), qB = rot_t(aB);
+    R2<T> pq[2], pqB[2];
+    B2G_POINTS
+    for (int j = 0; j < 2; ++j) {  /* forward again to get the pre-point poses */
+        if (j >= s.count) break;
+        pc[j] = cA; pcB[j] = cB;
+        R2<T> qA, qB;
+        rot2_t(aA, aB, qA, qB);
+        pq[j] = qA; pqB[j] = qB;
+        if (j + 1 == s.count) break;  /* no point follows that would need the updated poses */
         P2<T> pA = cA - mulq(qA, lcA), pB = cB - mulq(qB, lcB);
         P2<T> normal, point;
         T sep;
@@ -948,10 +992,11 @@ B2G_HD void solve_position_bwd(const SlotStatic& s, const P2<T>& lcA, const P2<T
         cB += mB * P;
         aB += iB * cross(rb, P);
     }
-    for (int j = s.count - 1; j >= 0; --j) {
+    B2G_POINTS
+    for (int j = 1; j >= 0; --j) {
+        if (j >= s.count) continue;
         const P2<T> cA0 = pc[j], cB0 = pcB[j];
-        const T aA0 = pa[j], aB0 = paB[j];
-        R2<T> qA = rot_t(aA0), qB = rot_t(aB0);
+        const R2<T> qA = pq[j], qB = pqB[j];
         P2<T> pA = cA0 - mulq(qA, lcA), pB = cB0 - mulq(qB, lcB);
         P2<T> normal, point;
         T sep;

@@ -405,11 +405,13 @@ inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-/* The same with the whole grid as one thread-block cluster (grid_barrier is then the cluster's barrier) */
+/* The same with the grid in thread-block clusters of `blocks` (grid_barrier is the cluster's barrier in a grid
+ * of one cluster) */
 template <typename... KArgs, typename... Args>
-inline int launch_cluster(void (*kernel)(KArgs...), int blocks, int threads, size_t smem, cudaStream_t s, Args... args) {
+inline int launch_cluster(void (*kernel)(KArgs...), int grid, int blocks, int threads, size_t smem, cudaStream_t s,
+                          Args... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
+    cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;

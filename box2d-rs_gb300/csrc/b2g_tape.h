@@ -65,7 +65,8 @@ struct TapeDev {
     long long* cnt;                  /* TAPE_CNT_* */
 };
 
-/* work buffers of one backward pass (sized for one segment of `seg` steps) */
+/* work buffers of one backward pass: those of a replay (to wp) and the counters for each of `groups`
+ * segments of ckpt_every steps, replayed side by side */
 struct AdjWork {
     TapeDev t;
     const float4* b_mass;
@@ -73,7 +74,9 @@ struct AdjWork {
     const uint32_t* b_flags;
     const float2* b_lc;
     int nb;
-    int t0, t1;                      /* the segment [t0, t1) */
+    int steps, final_ckpt;           /* taped steps, the checkpoint of the final state */
+    int first_seg;                   /* the segment whose buffers come first */
+    int t0, t1;                      /* the segment [t0, t1) (set on the device) */
     int max_slots, max_vi, max_pi;
     const float4* end_pos;           /* state after the segment's last step (checkpoint or final) */
     const float4* end_vel;
@@ -93,7 +96,7 @@ struct AdjWork {
     adj::VCGrad<float>* gvc;         /* max_slots */
     float4* g_imp;                   /* max_slots */
     float4* g_end[2];                /* per step parity, max_slots: adjoint of the stored impulses */
-    int* cnt;                        /* barrier block (CNT_SIZE ints) */
+    int* cnt;                        /* barrier blocks (CNT_SIZE ints each) */
     unsigned* mismatch;              /* replayed state differing from the recorded one (bodies) */
 };
 
@@ -102,8 +105,14 @@ void launch_tape_record(const DevWorld& w, const TapeDev& t, const StepParams& s
 void launch_tape_post(const DevWorld& w, const TapeDev& t, const StepParams& sp, cudaStream_t s, int num_sms);
 /* copy the current body state into checkpoint slot `index` */
 void launch_tape_snapshot(const DevWorld& w, const TapeDev& t, int index, cudaStream_t s);
-/* one backward segment: replay [t0, t1) forward, then reverse it */
-int launch_adjoint_segment(const AdjWork& a, cudaStream_t s, int num_sms);
+/* The backward pass, `parts`: parts of the steps' part-local solves (0: none). adjoint_groups: how many
+ * segments can be replayed in one launch; replay segments [a.first_seg, a.first_seg + segments); reverse
+ * one of them. Both return a CUDA error. */
+int adjoint_groups(int max_slots, int parts, int num_sms);
+int launch_adjoint_replay(const AdjWork& a, int segments, int parts, cudaStream_t s, int num_sms);
+int launch_adjoint_reverse(const AdjWork& a, int segment, int parts, cudaStream_t s, int num_sms);
+/* parts of a world's part-local solve (k_solver.cu) */
+int part_count(const DevWorld& w, int num_sms);
 
 }  // namespace b2g
 #endif

@@ -12,7 +12,8 @@
  *                  (the per-island early exit of b2_island_private.rs:257-274).
  *   k_tape_advance one thread: step and slot counters.
  *
- * Backward, per checkpoint segment from the last to the first (one cooperative launch each):
+ * Backward, per checkpoint segment from the last to the first; the replays of several segments run in one
+ * launch, side by side:
  *   k_adj_replay   restores the segment's checkpoint and re-runs its steps with the templated
  *                  forward functions in f32 — the same IEEE operations in the same order as the
  *                  solver kernel, colour by colour — keeping every intermediate the reverse
@@ -25,6 +26,8 @@
  * the adjoints of dynamic bodies are updated without atomics; static and kinematic bodies,
  * which several slots of one colour may share, accumulate with atomicAdd.
  */
+#include <algorithm>
+
 #include "b2g_sync.cuh"
 #include "b2g_tape.h"
 
@@ -35,12 +38,48 @@ using namespace adj;
 
 constexpr int kBlock = 256;
 
-__device__ __forceinline__ bool sync_all(int* cnt) {
-    if (gridDim.x == 1) {
+/* The blocks that work on one segment: all of the grid, or one of several groups that replay a segment
+ * each. `rank` is this block's place among them. */
+struct Group {
+    int* cnt;    /* the group's counters (barrier, status) */
+    int blocks, rank;
+};
+
+__device__ __forceinline__ bool sync_all(const Group& g) {
+    __shared__ int s_ok;
+    if (g.blocks == 1) {
         __syncthreads();
         return true;
     }
-    return grid_barrier(cnt);
+    if ((int)cluster_blocks() == g.blocks) {
+        cluster_barrier();
+        return true;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_ok = grid_wait(g.cnt, grid_arrive(g.cnt, 1u) * (unsigned)g.blocks) ? 1 : 0;
+    __syncthreads();
+    return s_ok != 0;
+}
+
+/* `a` with the buffers of the group that replays segment `seg` (or reverses it), and the segment's range */
+__device__ __forceinline__ void take_segment(AdjWork& a, int seg) {
+    const size_t g = (size_t)(seg - a.first_seg), nb = (size_t)a.nb, ns = (size_t)a.max_slots, every = (size_t)a.t.ckpt_every;
+    a.t0 = seg * a.t.ckpt_every;
+    a.t1 = min(a.steps, a.t0 + a.t.ckpt_every);
+    const size_t end = (size_t)(a.t1 == a.steps ? a.final_ckpt : a.t1 / a.t.ckpt_every) * nb;
+    a.end_pos = a.t.ckpt_pos + end;
+    a.end_vel = a.t.ckpt_vel + end;
+    a.cur_pos += g * nb;
+    a.cur_vel += g * nb;
+    a.ws_pos += g * every * nb;
+    a.ws_vel1 += g * every * nb;
+    a.ws_vel2 += g * every * nb;
+    a.vc += g * ns;
+    a.imp += g * ns;
+    a.wv += g * every * a.max_vi * ns * 3;
+    a.ww += g * every * ns * 2;
+    a.wp += g * every * a.max_pi * ns * 2;
+    a.cnt += g * CNT_SIZE;
 }
 
 /* ---------------- recording ---------------- */
@@ -329,11 +368,13 @@ __device__ __forceinline__ StepOrder step_order(const AdjWork& a, int t, const T
     return o;
 }
 
-/* fn(k) for every slot in solve order, each colour complete before the next */
+/* fn(k) for every slot in solve order, each colour complete before the next. Without boundary colours
+ * (a batch of worlds, or one part) a part's blocks meet the others only at the `last` sweep before a pass
+ * over all bodies or slots. */
 template <class F>
-__device__ __forceinline__ bool sweep_forward(const StepOrder& o, int* cnt, F&& fn) {
+__device__ __forceinline__ bool sweep_forward(const StepOrder& o, const Group& g, bool last, F&& fn) {
     if (o.np > 0) {
-        for (int p = blockIdx.x; p < o.np; p += gridDim.x) {
+        for (int p = g.rank; p < o.np; p += g.blocks) {
             const int* row = o.pool + o.rows[p];
             const int nc = row[0];
             for (int c = 0; c < nc; ++c) {
@@ -341,42 +382,46 @@ __device__ __forceinline__ bool sweep_forward(const StepOrder& o, int* cnt, F&& 
                 __syncthreads();
             }
         }
-        if (!sync_all(cnt)) return false;
+        if ((last || o.ncol > 0) && !sync_all(g)) return false;
     }
-    const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsize = gridDim.x * blockDim.x;
+    const int gtid = g.rank * blockDim.x + threadIdx.x, gsize = g.blocks * blockDim.x;
     for (int c = 0; c < o.ncol; ++c) {
         for (int k = o.co[c] + gtid; k < o.co[c + 1]; k += gsize) fn(k);
-        if (!sync_all(cnt)) return false;
+        if (!sync_all(g)) return false;
     }
     return true;
 }
 
 /* the same colours in the reverse order */
 template <class F>
-__device__ __forceinline__ bool sweep_reverse(const StepOrder& o, int* cnt, F&& fn) {
-    const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsize = gridDim.x * blockDim.x;
+__device__ __forceinline__ bool sweep_reverse(const StepOrder& o, const Group& g, bool last, F&& fn) {
+    const int gtid = g.rank * blockDim.x + threadIdx.x, gsize = g.blocks * blockDim.x;
     for (int c = o.ncol - 1; c >= 0; --c) {
         for (int k = o.co[c] + gtid; k < o.co[c + 1]; k += gsize) fn(k);
-        if (!sync_all(cnt)) return false;
+        if (!sync_all(g)) return false;
     }
     if (o.np > 0) {
-        for (int p = blockIdx.x; p < o.np; p += gridDim.x) {
+        for (int p = g.rank; p < o.np; p += g.blocks) {
             const int* row = o.pool + o.rows[p];
             for (int c = row[0] - 1; c >= 0; --c) {
                 for (int k = row[1 + c] + threadIdx.x; k < row[2 + c]; k += blockDim.x) fn(k);
                 __syncthreads();
             }
         }
-        if (!sync_all(cnt)) return false;
+        if ((last || o.ncol > 0) && !sync_all(g)) return false;
     }
     return true;
 }
 
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_adj_replay(AdjWork a) {
+/* The segments from a.first_seg on, a group of blocks each: a replay needs its checkpoint alone, so they
+ * run side by side. */
+__global__ void __launch_bounds__(kBlock) k_adj_replay(AdjWork a, int blocks) {
+    pdl_entry();
     grid_barrier_start();
-    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int gsize = gridDim.x * blockDim.x;
+    take_segment(a, a.first_seg + (int)blockIdx.x / blocks);
+    const Group group{a.cnt, blocks, (int)blockIdx.x % blocks};
+    const int gtid = group.rank * blockDim.x + threadIdx.x;
+    const int gsize = blocks * blockDim.x;
     const int nb = a.nb;
     {
         const size_t o = (size_t)(a.t0 / a.t.ckpt_every) * nb;
@@ -385,7 +430,7 @@ __global__ void __launch_bounds__(BLOCK) k_adj_replay(AdjWork a) {
             a.cur_vel[b] = a.t.ckpt_vel[o + b];
         }
     }
-    if (!sync_all(a.cnt)) return;
+    if (!sync_all(group)) return;
     for (int t = a.t0; t < a.t1; ++t) {
         const int s = t - a.t0;
         const TapeStep st = a.t.steps[t];
@@ -411,7 +456,7 @@ __global__ void __launch_bounds__(BLOCK) k_adj_replay(AdjWork a) {
             }
             wv1[b] = v;
         }
-        if (!sync_all(a.cnt)) return;
+        if (!sync_all(group)) return;
         /* constraint initialisation and warm-start impulses */
         for (int k = gtid; k < ns; k += gsize) {
             const TapeSlot ts = sl[k];
@@ -433,9 +478,9 @@ __global__ void __launch_bounds__(BLOCK) k_adj_replay(AdjWork a) {
             }
             a.imp[k] = im;
         }
-        if (!sync_all(a.cnt)) return;
+        if (!sync_all(group)) return;
         if (st.warm) {
-            const bool ok = sweep_forward(order, a.cnt, [&](int k) {
+            const bool ok = sweep_forward(order, group, st.vi == 0, [&](int k) {
                     const SlotStatic ss = slot_static(sl[k]);
                     const float4 vA = a.cur_vel[ss.a], vB = a.cur_vel[ss.b];
                     float4* rec = a.ww + ((size_t)s * a.max_slots + k) * 2;
@@ -454,7 +499,7 @@ __global__ void __launch_bounds__(BLOCK) k_adj_replay(AdjWork a) {
         }
         /* velocity iterations */
         for (int it = 0; it < st.vi; ++it) {
-            const bool ok = sweep_forward(order, a.cnt, [&](int k) {
+            const bool ok = sweep_forward(order, group, it == st.vi - 1, [&](int k) {
                     const SlotStatic ss = slot_static(sl[k]);
                     const float4 vA = a.cur_vel[ss.a], vB = a.cur_vel[ss.b];
                     const float4 im = a.imp[k];
@@ -489,10 +534,10 @@ __global__ void __launch_bounds__(BLOCK) k_adj_replay(AdjWork a) {
             a.cur_pos[b] = make_float4(c.x, c.y, ang, p.w);
             a.cur_vel[b] = make_float4(vv.x, vv.y, w, v.w);
         }
-        if (!sync_all(a.cnt)) return;
+        if (!sync_all(group)) return;
         /* position iterations, each island for the number of iterations it ran */
         for (int it = 0; it < st.pi; ++it) {
-            const bool ok = sweep_forward(order, a.cnt, [&](int k) {
+            const bool ok = sweep_forward(order, group, it == st.pi - 1, [&](int k) {
                     const TapeSlot ts = sl[k];
                     if (it >= __float_as_int(ts.rad.w)) return;
                     const SlotStatic ss = slot_static(ts);
@@ -521,9 +566,11 @@ __global__ void __launch_bounds__(BLOCK) k_adj_replay(AdjWork a) {
     }
 }
 
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_adj_reverse(AdjWork a) {
+__global__ void __launch_bounds__(kBlock) k_adj_reverse(AdjWork a, int seg) {
+    pdl_entry();
     grid_barrier_start();
+    take_segment(a, seg);
+    const Group group{a.cnt, (int)gridDim.x, (int)blockIdx.x};
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int gsize = gridDim.x * blockDim.x;
     const int nb = a.nb;
@@ -542,7 +589,7 @@ __global__ void __launch_bounds__(BLOCK) k_adj_reverse(AdjWork a) {
         float4* gend_prev = a.g_end[(t + 1) & 1];
         /* position iterations, last to first */
         for (int it = st.pi - 1; it >= 0; --it) {
-            const bool ok = sweep_reverse(order, a.cnt, [&](int k) {
+            const bool ok = sweep_reverse(order, group, it == 0, [&](int k) {
                     const TapeSlot ts = sl[k];
                     if (it >= __float_as_int(ts.rad.w)) return;
                     const SlotStatic ss = slot_static(ts);
@@ -591,10 +638,10 @@ __global__ void __launch_bounds__(BLOCK) k_adj_reverse(AdjWork a) {
             a.g_imp[k] = gend_cur[k];
         }
         for (int k = gtid; k < nprev; k += gsize) gend_prev[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (!sync_all(a.cnt)) return;
+        if (!sync_all(group)) return;
         /* velocity iterations, last to first */
         for (int it = st.vi - 1; it >= 0; --it) {
-            const bool ok = sweep_reverse(order, a.cnt, [&](int k) {
+            const bool ok = sweep_reverse(order, group, it == 0, [&](int k) {
                     const SlotStatic ss = slot_static(sl[k]);
                     const float4* rec = wv_rec(a, s, it, k);
                     const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2];
@@ -660,10 +707,10 @@ __global__ void __launch_bounds__(BLOCK) k_adj_reverse(AdjWork a) {
                 }
             }
         }
-        if (!sync_all(a.cnt)) return;
+        if (!sync_all(group)) return;
         /* constraint initialisation, colour by colour */
         {
-            const bool ok = sweep_reverse(order, a.cnt, [&](int k) {
+            const bool ok = sweep_reverse(order, group, true, [&](int k) {
                 const TapeSlot ts = sl[k];
                 const SlotStatic ss = slot_static(ts);
                 const float4 pA = wsp[ss.a], pB = wsp[ss.b];
@@ -695,16 +742,8 @@ __global__ void __launch_bounds__(BLOCK) k_adj_reverse(AdjWork a) {
             integrate_velocity_bwd(bs, h, gvv, gw);
             a.g_vel[b] = make_float4(gvv.x, gvv.y, gw, 0.0f);
         }
-        if (!sync_all(a.cnt)) return;
+        if (!sync_all(group)) return;
     }
-}
-
-/* one block per SM, like the forward solver: the sweeps are bound by grid-barrier latency, which
- * grows with the number of arriving blocks */
-int coop_blocks_for(const void* fn, int block, int num_sms) {
-    (void)fn;
-    (void)block;
-    return num_sms;
 }
 
 }  // namespace
@@ -725,31 +764,61 @@ void launch_tape_snapshot(const DevWorld& w, const TapeDev& t, int index, cudaSt
     B2G_LAUNCHED(1);
 }
 
-/* Small problems run in one block (block-level barriers); larger ones as a cooperative grid of
- * at most two blocks per SM. */
-int launch_adjoint_segment(const AdjWork& a, cudaStream_t s, int num_sms) {
-    AdjWork ac = a;
-    void* args[] = {&ac};
-    const bool single = a.max_slots <= 4096 && a.nb <= 16384;
-    cudaError_t e;
-    int* bar = a.cnt + CNT_BARRIER;
-    if (single) {
-        e = cudaLaunchCooperativeKernel((const void*)k_adj_replay<512>, dim3(1), dim3(512), args, 0, s);
-        if (e == cudaSuccess)
-            e = cudaLaunchCooperativeKernel((const void*)k_adj_reverse<512>, dim3(1), dim3(512), args, 0, s);
-    } else {
-        static int br = 0, bv = 0;
-        if (!br) br = coop_blocks_for((const void*)k_adj_replay<kBlock>, kBlock, num_sms);
-        if (!bv) bv = coop_blocks_for((const void*)k_adj_reverse<kBlock>, kBlock, num_sms);
-        e = cudaMemsetAsync(bar, 0, sizeof(int), s);
-        if (e == cudaSuccess)
-            e = cudaLaunchCooperativeKernel((const void*)k_adj_replay<kBlock>, dim3(br), dim3(kBlock), args, 0, s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(bar, 0, sizeof(int), s);
-        if (e == cudaSuccess)
-            e = cudaLaunchCooperativeKernel((const void*)k_adj_reverse<kBlock>, dim3(bv), dim3(kBlock), args, 0, s);
+/* How a backward pass is launched, from the slots of its largest step and the parts of its solves: on
+ * clusters of up to 16 blocks (one block for a small world) where a step fits 512 slots a block, else on a
+ * cooperative grid of a block for each part or 256 slots. (One block for up to 4096 slots took 110 ms for
+ * 128 steps of 10 throw-and-stack worlds, whose 1000 slots in two parts it swept one after the other; the
+ * cluster of two takes 31. 128 steps of one world: 34.7 -> 18.5 ms, 64 steps of 512 worlds: 42.7 -> 28 ms,
+ * replays side by side and local memory gone.) */
+static int adjoint_blocks(int max_slots, int parts, int num_sms, bool* cluster) {
+    *cluster = max_slots <= 512 * kClusterMaxBlocks && parts <= kClusterMaxBlocks;
+    if (*cluster) {
+        int c = 1;
+        while (c < kClusterMaxBlocks && (c < parts || 512 * c < max_slots)) c <<= 1;
+        static const bool big = cudaFuncSetAttribute((const void*)k_adj_replay, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                                     1) == cudaSuccess &&
+                                cudaFuncSetAttribute((const void*)k_adj_reverse, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                                     1) == cudaSuccess;
+        if (c <= 8 || big) return c;
+        *cluster = false;
     }
-    B2G_LAUNCHED(2);
-    return (int)e;
+    return std::max(1, std::min(num_sms, std::max(parts, (max_slots + kBlock - 1) / kBlock)));
+}
+
+/* Segments whose replays can run side by side: any number on clusters, and what is co-resident of a
+ * cooperative grid. */
+int adjoint_groups(int max_slots, int parts, int num_sms) {
+    bool cluster;
+    const int blocks = adjoint_blocks(max_slots, parts, num_sms, &cluster);
+    if (cluster) return 1 << 20;
+    int per_sm = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_adj_replay, kBlock, 0);
+    return std::max(1, per_sm * num_sms / blocks);
+}
+
+int launch_adjoint_replay(const AdjWork& a, int segments, int parts, cudaStream_t s, int num_sms) {
+    AdjWork ac = a;
+    bool cluster;
+    int blocks = adjoint_blocks(a.max_slots, parts, num_sms, &cluster);
+    B2G_LAUNCHED(1);
+    if (cluster) return launch_cluster(k_adj_replay, blocks * segments, blocks, kBlock, 0, s, ac, blocks);
+    const cudaError_t e = cudaMemsetAsync(a.cnt, 0, (size_t)segments * CNT_SIZE * sizeof(int), s);
+    if (e != cudaSuccess) return (int)e;
+    void* args[] = {&ac, &blocks};
+    return (int)cudaLaunchCooperativeKernel((const void*)k_adj_replay, dim3(blocks * segments), dim3(kBlock), args, 0, s);
+}
+
+int launch_adjoint_reverse(const AdjWork& a, int segment, int parts, cudaStream_t s, int num_sms) {
+    AdjWork ac = a;
+    bool cluster;
+    const int blocks = adjoint_blocks(a.max_slots, parts, num_sms, &cluster);
+    B2G_LAUNCHED(1);
+    if (cluster) return launch_cluster(k_adj_reverse, blocks, blocks, kBlock, 0, s, ac, segment);
+    int* bar = a.cnt + (size_t)(segment - a.first_seg) * CNT_SIZE + CNT_BARRIER;
+    const cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(int), s);
+    if (e != cudaSuccess) return (int)e;
+    void* args[] = {&ac, &segment};
+    return (int)cudaLaunchCooperativeKernel((const void*)k_adj_reverse, dim3(blocks), dim3(kBlock), args, 0, s);
 }
 
 }  // namespace b2g

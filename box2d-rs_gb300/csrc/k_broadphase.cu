@@ -944,7 +944,7 @@ int launch_back(const DevWorld& w, const StepParams& sp, cudaStream_t s) {
         cudaFuncSetAttribute((const void*)k_back, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     (void)allowed;
     B2G_LAUNCHED(1);
-    return launch_cluster(k_back, cluster_size(w), kBlock, 0, s, w, sp);
+    return launch_cluster(k_back, cluster_size(w), cluster_size(w), kBlock, 0, s, w, sp);
 }
 
 /* Runs update_pairs + add_pair and merges: the caller swaps w.c and w.c_alt afterwards. */

@@ -1853,7 +1853,7 @@ int launch_front(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool p
     const bool local = use_parts(w, w.num_sms, parts);
     const size_t smem = local && (passes & FRONT_SOLVE) ? part_smem(spc, kPartSmemOne) : 0;
     B2G_LAUNCHED(1);
-    return launch_cluster(k_front, cluster_size(w), kBlock, smem, s, w, spc, local ? part_count(w, w.num_sms) : 0, passes);
+    return launch_cluster(k_front, cluster_size(w), cluster_size(w), kBlock, smem, s, w, spc, local ? part_count(w, w.num_sms) : 0, passes);
 }
 
 void launch_phase_stamp(const DevWorld& w, int phase, cudaStream_t s) {
