@@ -1224,12 +1224,7 @@ void issue_step(World* w, const StepParams& sp, float dt) {
     if (dt > 0.0f) {
         const bool taping = w->tape && w->tape->recording;
         if (cluster_world(w->d)) {
-            launch_front(w->d, sp, s, w->part_solve, taping ? FRONT_ISLANDS | FRONT_COLOUR : FRONT_ALL);
-            if (taping) {
-                launch_tape_record(w->d, w->tape->d, sp, s, w->num_sms);
-                launch_front(w->d, sp, s, w->part_solve, FRONT_SOLVE);
-                launch_tape_post(w->d, w->tape->d, sp, s, w->num_sms);
-            }
+            launch_front(w->d, sp, s, w->part_solve, taping ? &w->tape->d : nullptr);
         } else {
             launch_islands_and_constraints(w->d, sp, s);
             launch_colouring(w->d, s, w->num_sms, w->part_solve);

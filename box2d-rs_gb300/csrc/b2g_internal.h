@@ -445,15 +445,15 @@ void launch_touch_all_proxies(const DevWorld& w, cudaStream_t s);
 void launch_flag_joint_contacts(const DevWorld& w, cudaStream_t s, int num_sms);
 void launch_islands_and_constraints(const DevWorld& w, const StepParams& sp, cudaStream_t s);
 /* Worlds of up to kClusterMaxProxies proxies (and twice as many bodies) run the whole of islands,
- * colouring and solver (`passes`: FRONT_* bits) as one kernel on one thread-block cluster, and the whole
+ * colouring and solver, and of a taped step's recording (tape), as one kernel on one thread-block cluster, and the whole
  * broadphase and contact merge as another (launch_back): cluster_world says whether a world does, given
  * the device's largest cluster. */
-enum { FRONT_ISLANDS = 1, FRONT_COLOUR = 2, FRONT_SOLVE = 4, FRONT_ALL = 7 };
 constexpr int kClusterMaxBlocks = 16;
 constexpr int kClusterMaxProxies = kClusterMaxBlocks * 256;
 bool cluster_world(const DevWorld& w);
 int cluster_size(const DevWorld& w);
-int launch_front(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool parts, int passes);
+struct TapeDev;
+int launch_front(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool parts, const TapeDev* tape);
 int launch_back(const DevWorld& w, const StepParams& sp, cudaStream_t s);
 /* a stamp on its own (a step that ends with a phase no kernel follows) */
 void launch_phase_stamp(const DevWorld& w, int phase, cudaStream_t s);

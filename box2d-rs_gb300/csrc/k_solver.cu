@@ -36,6 +36,7 @@
 #include "b2g_joint.cuh"
 #include "b2g_solver_math.cuh"
 #include "b2g_sync.cuh"
+#include "b2g_tape_record.cuh"
 
 namespace b2g {
 
@@ -1642,29 +1643,33 @@ __global__ void __launch_bounds__(kBlock) k_solve_fixtures(const __grid_constant
     finish_fixtures(w);
 }
 
-/* Islands, colouring and solver of a world of a few thousand bodies as one kernel on one cluster of up
- * to 16 blocks (passes: FRONT_*; a taped step stops after the colouring to record it). Such a step is
+/* Islands, colouring and solver of a world of a few thousand bodies, and the recording of a taped step, as
+ * one kernel on one cluster of up to 16 blocks. Such a step is
  * bound by the latency of its barriers and launches, not by work: three cooperative launches of 152
  * blocks took 20 + 22 + 56 us for a 16-body world (each launch a memset of its counter besides) and
  * every barrier of their sweeps 1.4 us; here a barrier takes 0.3 us (one block: a __syncthreads) and the
  * passes follow each other without a launch. */
 __global__ void __launch_bounds__(kBlock, 1) k_front(const __grid_constant__ DevWorld w, const __grid_constant__ StepParams sp,
-                                                  int nparts, int passes) {
+                                                  int nparts, const __grid_constant__ TapeDev t, int taped) {
     pdl_entry();
     if (cluster_leaves(w)) return;
-    if (passes & FRONT_ISLANDS) {
-        phase_stamp(w, PH_COLLIDE);
-        islands_pass(w, sp.allow_sleep);
-    }
-    if (passes & FRONT_COLOUR) {
+    phase_stamp(w, PH_COLLIDE);
+    islands_pass(w, sp.allow_sleep);
+    grid_barrier(w);
+    phase_stamp(w, PH_ISLANDS);
+    colour_pass(w, nparts);
+    grid_barrier(w);
+    if (taped) {
+        tape_record(w, t, sp);
         grid_barrier(w);
-        phase_stamp(w, PH_ISLANDS);
-        colour_pass(w, nparts);
     }
-    if (passes & FRONT_SOLVE) {
+    phase_stamp(w, PH_COLOURING);
+    solve_pass<true>(w, sp);
+    if (taped) {
         grid_barrier(w);
-        phase_stamp(w, PH_COLOURING);
-        solve_pass<true>(w, sp);
+        tape_post(w, t, sp);
+        grid_barrier(w);
+        if (blockIdx.x == 0 && threadIdx.x == 0) tape_advance(w, t);
     }
 }
 
@@ -1846,14 +1851,15 @@ bool cluster_world(const DevWorld& w) {
            cluster_size(w) <= max_cluster();
 }
 
-int launch_front(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool parts, int passes) {
+int launch_front(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool parts, const TapeDev* tape) {
     StepParams spc = sp;
     spc.part_bodies = 0;
     spc.part_slot_bytes = 0;
     const bool local = use_parts(w, w.num_sms, parts);
-    const size_t smem = local && (passes & FRONT_SOLVE) ? part_smem(spc, kPartSmemOne) : 0;
+    const size_t smem = local ? part_smem(spc, kPartSmemOne) : 0;
     B2G_LAUNCHED(1);
-    return launch_cluster(k_front, cluster_size(w), cluster_size(w), kBlock, smem, s, w, spc, local ? part_count(w, w.num_sms) : 0, passes);
+    return launch_cluster(k_front, cluster_size(w), cluster_size(w), kBlock, smem, s, w, spc,
+                          local ? part_count(w, w.num_sms) : 0, tape ? *tape : TapeDev{}, tape ? 1 : 0);
 }
 
 void launch_phase_stamp(const DevWorld& w, int phase, cudaStream_t s) {
