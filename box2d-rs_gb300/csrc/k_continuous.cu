@@ -46,7 +46,10 @@
  *     synchronisation, with the moved proxies' LBVH leaves updated in place and their ancestors'
  *     boxes grown to cover them
  *   7 pairs of the moved proxies on the LBVH (skip itself, skip a moved partner with a larger proxy
- *     id); new contacts are appended to the table
+ *     id), one warp per proxy; new contacts are appended to the table. A walk by one thread is a chain
+ *     of a fetch for each node it visits and was the longest phase: with a warp's walk the pass and the
+ *     merge before it take 154 us instead of 230 for 1000 fast bodies, 299 instead of 391 for 4000,
+ *     and 1.38 ms instead of 1.96 ms for 512 worlds of 200 (tens of thousands of moved proxies)
  * After the loop the appended contacts are merged into the key-sorted table.
  */
 #include <climits>
@@ -55,6 +58,7 @@
 #include "b2g_solver_math.cuh"
 #include "b2g_sync.cuh"
 #include "b2g_toi.cuh"
+#include "b2g_walk.cuh"
 
 namespace b2g {
 namespace {
@@ -67,7 +71,6 @@ constexpr float kToiBaumgarte = 0.75f;     /* B2_TOI_BAUMGARTE, src/b2_common.rs
 constexpr int kIslBodies = 64;             /* the TOI island's body capacity, 2 x B2_MAX_TOICONTACTS */
 constexpr int kIslContacts = kToiCand + 1;
 constexpr int kMaxIters = 1 << 16;         /* iterations of one pass */
-constexpr int kStack = 64;
 constexpr uint32_t kNoAlpha = 0xffffffffu;
 /* 1 - 10 eps: the largest alpha that is still an event (private/dynamics/b2_world.rs:697) */
 constexpr float kEventMax = 1.0f - 10.0f * kEpsilon;
@@ -200,13 +203,6 @@ __device__ __forceinline__ void mark_complex(const DevWorld& w, int i, int epoch
     if (xa && dynamic_body(fb)) w.b_cx[bd.y] = epoch;
 }
 
-__device__ __forceinline__ bool box_overlap(const float4 a, const float4 b) {
-    /* b2_test_overlap, src/b2_collision.rs:355-368 (closed boxes) */
-    if (b.x - a.z > 0.0f || b.y - a.w > 0.0f) return false;
-    if (a.x - b.z > 0.0f || a.y - b.w > 0.0f) return false;
-    return true;
-}
-
 __device__ __forceinline__ void atomic_min_float(float* p, float v) {
     int old = __float_as_int(*(volatile float*)p);
     while (v < __int_as_float(old)) {
@@ -315,6 +311,8 @@ __device__ __forceinline__ ConstraintIn island_constraint(const DevWorld& w, int
     in.qB = qB;
     return in;
 }
+
+constexpr int max_of(int a, int b) { return a > b ? a : b; }
 
 struct IslandScratch {
     int body[kIslBodies];
@@ -834,33 +832,12 @@ __global__ void __launch_bounds__(kTBlock) k_continuous(DevWorld w, StepParams s
         /* 7: find_new_contacts for the proxies this iteration moved */
         if (gtid == 0) vcnt[CNT_TOI_NEV] = 0;
         const int nm = min(vcnt[CNT_TOI_MOVED], w.fix_cap);
-        for (int qi = gtid; qi < nm; qi += gstride) {
+        int* pend = reinterpret_cast<int*>(smem) + warp * kPendMax;
+        for (int qi = gtid >> 5; qi < nm; qi += gstride >> 5) {
             const int q = w.t_moved[qi];
-            const uint32_t wd = w.b_world[w.f_body[q]];
-            const float4 box = w.f_fat[q];
-            for (int h = 0; h < 2; ++h) {
-                const int root = w.bp_world_root[wd + (h ? (uint32_t)w.num_worlds : 0u)];
-                if (root == INT_MIN) continue;
-                if (root < 0) {
-                    if (box_overlap(w.bp_leaf[~root], box)) toi_pair(w, q, (int)w.bp_val[~root], n_tab, n_all, epoch);
-                    continue;
-                }
-                int stack[kStack];
-                int top = 0;
-                stack[top++] = root;
-                while (top > 0) {
-                    const int node = stack[--top];
-                    const int2 ch = w.bp_node_child[node];
-                    const float4 bx[2] = {w.bp_node_b0[node], w.bp_node_b1[node]};
-                    const int kids[2] = {ch.x, ch.y};
-                    for (int c = 0; c < 2; ++c) {
-                        if (!box_overlap(bx[c], box)) continue;
-                        if (kids[c] < 0) toi_pair(w, q, (int)w.bp_val[~kids[c]], n_tab, n_all, epoch);
-                        else if (top < kStack) stack[top++] = kids[c];
-                        else atomicOr((unsigned*)&w.cnt[CNT_STATUS], ST_STACK_OVERFLOW);
-                    }
-                }
-            }
+            walk_box(w, w.f_fat[q], w.b_world[w.f_body[q]], pend, [&](bool ok, int p) {
+                if (ok) toi_pair(w, q, (int)w.bp_val[p], n_tab, n_all, epoch);
+            });
         }
         if (!grid_barrier(w)) return;
     }
@@ -903,7 +880,8 @@ __global__ void __launch_bounds__(kTBlock) k_continuous(DevWorld w, StepParams s
 
 int launch_continuous(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms) {
     static bool configured = false;
-    const int smem = kIslWarps * (int)sizeof(IslandScratch);
+    /* the islands' scratch, and after them the walks' pending nodes */
+    constexpr int smem = max_of(kIslWarps * (int)sizeof(IslandScratch), kTBlock / 32 * kPendMax * (int)sizeof(int));
     if (!configured) {
         cudaFuncSetAttribute((const void*)k_continuous, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         configured = true;
