@@ -137,6 +137,7 @@ enum {
     CNT_BP_WARP_VISITS = 57, /* the most node fetches one warp of the last traversal made */
     CNT_BP_WARP_CHECKS = 58, /* the most leaf checks one warp of the last traversal made */
     CNT_LIST = 59,           /* colouring: constraints that keep no colour of the previous colouring */
+    CNT_BP_LIST = 60,        /* leaves of moved proxies listed for this pass's traversal (in bp_val_alt) */
     CNT_SIZE = 64
 };
 

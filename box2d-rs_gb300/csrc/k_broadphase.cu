@@ -21,8 +21,8 @@
  *      internal node stores both children's boxes, and after the refit a four-way record of
  *      its grandchildren, so a traversal step is one 80-byte fetch and four overlap tests,
  *   4. bottom-up refit with per-node arrival counters,
- *   5. one thread per moved proxy walks its world's two subtrees with a short stack and
- *      applies the reference's rule: skip itself; skip a moved partner whose proxy id is
+ *   5. the moved proxies' leaves are listed, and a thread per listed leaf walks its world's two
+ *      subtrees with a short stack and applies the reference's rule: skip itself; skip a moved partner whose proxy id is
  *      larger (that partner reports the pair); emit (min id, max id).
  * Which pass rebuilds changes only how many nodes a query visits: boxes of internal nodes only
  * have to contain their leaves, and leaves hold the exact fat AABBs.
@@ -84,6 +84,7 @@ __device__ __forceinline__ void bp_decide(const DevWorld& w, int mode) {
     c[CNT_BP_CANDIDATES] = 0;
     c[CNT_BP_WARP_VISITS] = 0;
     c[CNT_BP_WARP_CHECKS] = 0;
+    c[CNT_BP_LIST] = 0;
     if (mode == BP_REPEAT) return;
     const int moved = c[CNT_BP_MOVED];
     const long long drift = (long long)c[CNT_BP_DRIFT] + moved;
@@ -442,9 +443,26 @@ __device__ __forceinline__ void bp_update_leaves(const DevWorld& w) {
         }
     }
 }
+/* The leaves of the moved proxies, in bp_val_alt (free once the keys are sorted): a block's in order, the
+ * blocks' in any. */
+__device__ __forceinline__ void bp_list_moved(const DevWorld& w) {
+    const int n = w.n_fixtures;
+    __shared__ int s_at;
+    for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+        const int p = base + threadIdx.x;
+        const bool moved = p < n && w.f_moved[w.bp_val[p]] != 0;
+        if (!__syncthreads_or(moved)) continue;
+        uint32_t total;
+        const uint32_t r = block_exclusive_scan(moved ? 1u : 0u, &total);
+        if (threadIdx.x == 0) s_at = atomicAdd(&w.cnt[CNT_BP_LIST], (int)total);
+        __syncthreads();
+        if (moved) w.bp_val_alt[s_at + r] = (uint32_t)p;
+    }
+}
 __global__ void k_bp_update(DevWorld w) {
     pdl_entry();
     B2G_RETURN_IF_ABORTED(w);
+    bp_list_moved(w);
     bp_rows(w);
     if (!bp_rebuilding(w)) bp_update_leaves(w);
 }
@@ -576,13 +594,20 @@ __device__ __forceinline__ unsigned check_batch(const DevWorld& w, const StepPar
     return n;
 }
 
-/* One lane per moved proxy starts a walk of the hierarchies, and a warp walks in step:
+/* The listed moved proxies are dealt out evenly, as many to a warp (one to a lane, at most 32) as the
+ * resident warps need to hold them all: a pass moves few of a world's proxies or half of them, and the
+ * chain of the longest warp is what it takes. A warp walks in step:
  *  - a lane only queues the leaves its query box overlaps (in shared memory), and whenever a warp
  *    has 32 or more queued the whole warp checks them, one leaf per lane (the partner rules, the
  *    existing-contact row scan and add_pair's filters are chains of dependent loads);
  *  - a lane whose walk is done takes over the oldest pending node of a lane with two or more,
  *    with that lane's query box, so a warp's rounds follow its total work rather than its longest
  *    walk. */
+/* Threads of an SM, the four blocks its registers allow: 100k bodies in flight (55k moved proxies) take
+ * 99 us, and took 146 with a warp for every 32 proxies, moved or not; 120 and 162 with three and two blocks,
+ * 116 with a second wave, 120 with five blocks of 48 registers. 10k bodies: 34 (100) us, a 250k pile of 14k
+ * moved ones: 52 (104). */
+constexpr int kTraverseThreads = 1024;
 constexpr int kLeafQueue = 224;  /* 31 left over + 32 lanes x 4 leaves in one round, or the setup's
                                     2 single-proxy roots per lane */
 
@@ -591,21 +616,19 @@ __device__ __forceinline__ void bp_traverse(const DevWorld& w, const StepParams&
     __shared__ int s_give_node[kBlock / 32][32];
     __shared__ int s_give_f[kBlock / 32][32];
     __shared__ float4 s_give_q[kBlock / 32][32];
-    const int n = w.n_fixtures;
+    const int n = w.cnt[CNT_BP_LIST];
     const int n_contacts = w.cnt[CNT_CONTACTS];
     const uint32_t nw = (uint32_t)w.num_worlds;
     const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    const int per = max(1, min(32, (n + warps - 1) / warps));  /* queries a warp starts with */
     const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
     uint2* queue = s_queue[wq];
-    const int stride = gridDim.x * blockDim.x;
     unsigned visits = 0, candidates = 0;  /* this lane's node fetches and leaf checks (traffic counters) */
-    for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
-        const int p = base + lane;
-        int f = -1;
-        if (p < n) {
-            f = (int)w.bp_val[p];
-            if (!w.f_moved[f]) f = -1;
-        }
+    for (int base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per; base < n; base += warps * per) {
+        const bool mine = lane < per && base + lane < n;
+        const int p = mine ? (int)w.bp_val_alt[base + lane] : 0;
+        int f = mine ? (int)w.bp_val[p] : -1;
         int stack[kStack];
         int bot = 0, top = 0;  /* pending nodes [bot, top) of the current query */
         int found[6];
@@ -871,6 +894,7 @@ __global__ void __launch_bounds__(kBlock) k_back(const __grid_constant__ DevWorl
         phase_stamp(w, PH_SORT);
         bp_update_leaves(w);
     }
+    bp_list_moved(w);
     grid_barrier(w);
     phase_stamp(w, PH_HIERARCHY);
     bp_traverse(w, sp);
@@ -967,7 +991,7 @@ void launch_broadphase(const DevWorld& w, const StepParams& sp, cudaStream_t s, 
         launch_pdl(k_bp_update, grid_for(std::max(n, w.contact_cap), kBlock, num_sms * 8), kBlock, 0, s, w);
         B2G_LAUNCHED(1);
         const int tb = w.cfg_traverse_block;
-        launch_pdl(k_bp_traverse, grid_for(n, tb, num_sms * 2048 / tb), tb, 0, s, w, sp); B2G_LAUNCHED(1);
+        launch_pdl(k_bp_traverse, grid_for(n, tb / 32, num_sms * kTraverseThreads / tb), tb, 0, s, w, sp); B2G_LAUNCHED(1);
         launch_pdl(k_bp_clear_moved, gf, kBlock, 0, s, w); B2G_LAUNCHED(1);
     }
     if (n == 0) cudaMemsetAsync(w.sort_hist, 0, kSortRankWords * sizeof(uint32_t), s);
