@@ -1227,9 +1227,9 @@ void issue_step(World* w, const StepParams& sp, float dt) {
             launch_front(w->d, sp, s, w->part_solve, taping ? &w->tape->d : nullptr);
         } else {
             launch_islands_and_constraints(w->d, sp, s);
-            launch_colouring(w->d, s, w->num_sms, w->part_solve);
+            launch_colouring(w->d, s, w->num_sms, w->part_solve, taping);
             if (taping) launch_tape_record(w->d, w->tape->d, sp, s, w->num_sms);
-            launch_solver(w->d, sp, s, w->num_sms, w->part_solve);
+            launch_solver(w->d, sp, s, w->num_sms, w->part_solve, taping);
             if (taping) launch_tape_post(w->d, w->tape->d, sp, s, w->num_sms);
         }
         /* a host contact filter is asked about the new pairs between the traversal and the merge */

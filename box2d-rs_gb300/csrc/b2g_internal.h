@@ -97,7 +97,7 @@ enum {
     CNT_COLOURINGS = 19,  /* colourings done so far: the stamp of colours kept in contacts (mids.w) */
     CNT_DYN_EXTENT = 20,  /* largest half-extent of a dynamic body's fat AABB (float bits), this pass */
     CNT_INTERIOR = 21,    /* constraint slots solved part-locally this step (slots [0, n)) */
-    CNT_PARTS = 22,       /* parts of this step's colouring (at most the solver's blocks), 0 if off */
+    CNT_PARTS = 22,       /* parts of this step's colouring, 0 if off */
     CNT_PART_NCACHE = 23, /* constraint bodies of the current partition (entries of cache_body) */
     CNT_PART_P = 24,      /* parts of the current partition (0: none) */
     CNT_PART_NF = 25,     /* proxies when the current partition was made */
@@ -138,13 +138,14 @@ enum {
     CNT_BP_WARP_CHECKS = 58, /* the most leaf checks one warp of the last traversal made */
     CNT_LIST = 59,           /* colouring: constraints that keep no colour of the previous colouring */
     CNT_BP_LIST = 60,        /* leaves of moved proxies listed for this pass's traversal (in bp_val_alt) */
+    CNT_PART_SPLIT = 61,     /* a kept partition of more parts than SMs has split a world */
     CNT_SIZE = 64
 };
 
 constexpr int kMaxColours = 256;   /* first-fit colours 0..63, then one per colouring round */
 constexpr int kFirstFitColours = 64;
 constexpr int kColourTail = 256;   /* uncoloured constraints one block finishes colouring (one per thread) */
-constexpr int kMaxParts = 1024;    /* body parts of the part-local solve (at most one per solver block) */
+constexpr int kMaxParts = 1024;    /* body parts of the part-local solve (more than one per SM only in a large batch) */
 /* default of cfg_collide_group: one lane per pair (measured on GB300 at least as fast as the 8-lane
  * segments on the mixed 100k scene, the 4096-world batch and the 250k-box pile) */
 constexpr int kCollideGroup = 0;
@@ -459,8 +460,8 @@ int launch_back(const DevWorld& w, const StepParams& sp, cudaStream_t s);
 /* a stamp on its own (a step that ends with a phase no kernel follows) */
 void launch_phase_stamp(const DevWorld& w, int phase, cudaStream_t s);
 /* parts: allow the part-local solve (used where the world's size suits it) */
-void launch_colouring(const DevWorld& w, cudaStream_t s, int num_sms, bool parts);
-int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms, bool parts);
+void launch_colouring(const DevWorld& w, cudaStream_t s, int num_sms, bool parts, bool taped);
+int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms, bool parts, bool taped);
 /* time of impact of n shape pairs; every pointer is memory the device reaches. A definition that is no
  * circle, polygon or edge sets *bad, and no result is written then */
 void launch_time_of_impact(const b2g_fixture_def* da, const b2g_sweep* swa, const b2g_fixture_def* db,

@@ -284,7 +284,7 @@ __device__ __forceinline__ bool colour_pass(const DevWorld& w, int nparts) {
     const int gsize = gridDim.x * blockDim.x;
     const int n = w.cnt[CNT_CONS];
     const int nf = w.n_fixtures;
-    const int P = (nf > 0 && nparts <= kMaxParts && nparts <= (int)gridDim.x) ? nparts : 0;
+    const int P = (nf > 0 && nparts <= kMaxParts) ? nparts : 0;
     const size_t bc = (size_t)w.body_cap;
     const unsigned long long kNone = ~0ull;
     const uint32_t stamp = (uint32_t)w.cnt[CNT_COLOURINGS] & kStampMask;  /* the previous colouring's */
@@ -301,138 +301,146 @@ __device__ __forceinline__ bool colour_pass(const DevWorld& w, int nparts) {
     /* the partition is made afresh every 4th colouring (and when the part or proxy count changed)
      * and kept in between: a body stays in its part, and a body outside the partition goes to the
      * part whose rank range its Morton rank falls in. (Kept colours stay proper across a new
-     * partition: interior constraints that share a body are always in the same part.) */
-    const bool rebalance = P > 0 && ((stamp & 3u) == 0u || w.cnt[CNT_PART_P] != P || w.cnt[CNT_PART_NF] != nf);
+     * partition: interior constraints that share a body are always in the same part.) More parts than
+     * SMs, a batch's, have a solver without boundary sweeps: should a kept partition have put a world's
+     * bodies into two parts (Morton ranks move when a large static proxy changes hierarchies), it is made
+     * afresh after all, which puts every world into one part. */
+    bool rebalance = P > 0 && ((stamp & 3u) == 0u || w.cnt[CNT_PART_P] != P || w.cnt[CNT_PART_NF] != nf);
     int ncache = w.cnt[CNT_PART_NCACHE];  /* read before any barrier; a rebalance rewrites it below */
-    if (rebalance) {
-        /* Parts of equal work: weigh each Morton rank by the constraint endpoints of its body and
-         * cut the weight prefix into P equal ranges. rank_x was zeroed by the broadphase. */
-        for (int k = gtid; k < n; k += gsize) {
-            const int2 bd = w.c.body[w.cons_contact[k]];
-            if (is_dynamic(w.b_flags[bd.x]) && w.b_rank[bd.x] < nf) atomicAdd(&w.rank_x[w.b_rank[bd.x]], 1ull << 32);
-            if (is_dynamic(w.b_flags[bd.y]) && w.b_rank[bd.y] < nf) atomicAdd(&w.rank_x[w.b_rank[bd.y]], 1ull << 32);
-        }
-        for (int q = gtid; q < P; q += gsize) {
-            w.part_cbeg[q] = 0;
-            w.part_cend[q] = 0;
-            w.part_rbeg[q] = INT_MAX;
-        }
-        if (!grid_barrier(w)) return false;
-        /* each block scans its chunk of ranks: (weight << 32 | has weight), exclusive */
-        const int chunk = (nf + (int)gridDim.x - 1) / (int)gridDim.x;
-        const int r0 = min(nf, (int)blockIdx.x * chunk), r1 = min(nf, r0 + chunk);
-        unsigned long long carry = 0;
-        for (int base = r0; base < r1; base += blockDim.x) {
-            const int r = base + threadIdx.x;
-            unsigned long long v = r < r1 ? w.rank_x[r] : 0ull;
-            v += v ? 1ull : 0ull;
-            unsigned long long tot;
-            const unsigned long long ex = block_scan_excl64(v, &tot);
-            if (r < r1) w.rank_x[r] = carry + ex;
-            carry += tot;
-        }
-        if (threadIdx.x == 0) w.blk_tot[blockIdx.x] = carry;
-        if (!grid_barrier(w)) return false;
-        unsigned long long before = 0, all = 0;
-        {
-            unsigned long long mine = 0, every = 0;
-            for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) {
-                const unsigned long long t = w.blk_tot[q];
-                if (q < (int)blockIdx.x) mine += t;
-                every += t;
+    for (;;) {
+        if (rebalance) {
+            /* Parts of equal work: weigh each Morton rank by the constraint endpoints of its body and
+             * cut the weight prefix into P equal ranges. rank_x was zeroed by the broadphase. */
+            for (int k = gtid; k < n; k += gsize) {
+                const int2 bd = w.c.body[w.cons_contact[k]];
+                if (is_dynamic(w.b_flags[bd.x]) && w.b_rank[bd.x] < nf) atomicAdd(&w.rank_x[w.b_rank[bd.x]], 1ull << 32);
+                if (is_dynamic(w.b_flags[bd.y]) && w.b_rank[bd.y] < nf) atomicAdd(&w.rank_x[w.b_rank[bd.y]], 1ull << 32);
             }
-            block_scan_excl64(mine, &before);
-            block_scan_excl64(every, &all);
-        }
-        const unsigned long long wtot = all >> 32;
-        /* A batch of worlds cuts only at world boundaries: a world's bodies all take the part of the
-         * weight prefix at the world's first rank (ranks are grouped by world), so no constraint
-         * joins two parts, there are no boundary colours, and the parts never wait for each other.
-         * That needs the prefix at any rank: the chunks' prefixes are made global first. */
-        const bool aligned = w.num_worlds > 1;
-        if (aligned) {
-            for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) w.rank_x[r] += before;
+            for (int q = gtid; q < P; q += gsize) {
+                w.part_cbeg[q] = 0;
+                w.part_cend[q] = 0;
+                w.part_rbeg[q] = INT_MAX;
+            }
             if (!grid_barrier(w)) return false;
-        }
-        const unsigned long long base_x = aligned ? 0ull : before;
-        for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-            const unsigned long long x = base_x + w.rank_x[r];
-            const unsigned long long x1 = r + 1 < r1 ? base_x + w.rank_x[r + 1] : before + carry;
-            if ((uint32_t)x1 == (uint32_t)x || wtot == 0ull) continue;  /* no constraint at this rank */
-            unsigned long long px = x;
-            if (aligned) {
-                const int first = w.bp_world_first[(uint32_t)(w.bp_key[r] >> kKeyMortonBits)];
-                if (first >= 0 && first <= r) px = w.rank_x[first];
+            /* each block scans its chunk of ranks: (weight << 32 | has weight), exclusive */
+            const int chunk = (nf + (int)gridDim.x - 1) / (int)gridDim.x;
+            const int r0 = min(nf, (int)blockIdx.x * chunk), r1 = min(nf, r0 + chunk);
+            unsigned long long carry = 0;
+            for (int base = r0; base < r1; base += blockDim.x) {
+                const int r = base + threadIdx.x;
+                unsigned long long v = r < r1 ? w.rank_x[r] : 0ull;
+                v += v ? 1ull : 0ull;
+                unsigned long long tot;
+                const unsigned long long ex = block_scan_excl64(v, &tot);
+                if (r < r1) w.rank_x[r] = carry + ex;
+                carry += tot;
             }
-            const int part = min(P - 1, (int)(((px >> 32) * (unsigned long long)P) / wtot));
-            const int c = (int)(uint32_t)x;
-            if (c >= nf) continue;  /* cannot happen: at most one constraint body per rank */
-            const int b = w.f_body[w.bp_val[r]];
-            w.b_part[b] = part;
-            w.b_cidx[b] = c;
-            w.cache_body[c] = b;
-        }
-        if (!grid_barrier(w)) return false;
-        /* each part's range of constraint bodies */
-        ncache = min(nf, (int)(uint32_t)all);
-        for (int c = gtid; c < ncache; c += gsize) {
-            const int part = w.b_part[w.cache_body[c]];
-            if (c == 0 || w.b_part[w.cache_body[c - 1]] != part) {
-                w.part_cbeg[part] = c;
-                int rb = w.b_rank[w.cache_body[c]];
-                if (w.num_worlds > 1) {  /* whole worlds: the range starts at the world's first rank */
-                    const int first = w.bp_world_first[(uint32_t)(w.bp_key[rb] >> kKeyMortonBits)];
-                    if (first >= 0 && first <= rb) rb = first;
+            if (threadIdx.x == 0) w.blk_tot[blockIdx.x] = carry;
+            if (!grid_barrier(w)) return false;
+            unsigned long long before = 0, all = 0;
+            {
+                unsigned long long mine = 0, every = 0;
+                for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) {
+                    const unsigned long long t = w.blk_tot[q];
+                    if (q < (int)blockIdx.x) mine += t;
+                    every += t;
                 }
-                if (part > 0) w.part_rbeg[part] = rb;
+                block_scan_excl64(mine, &before);
+                block_scan_excl64(every, &all);
             }
-            if (c == ncache - 1 || w.b_part[w.cache_body[c + 1]] != part) w.part_cend[part] = c + 1;
-        }
-        if (gtid == 0) {
-            w.cnt[CNT_PART_NCACHE] = ncache;
-            w.cnt[CNT_PART_NF] = nf;
-            w.cnt[CNT_PART_P] = P;
-        }
-    }
-    if (gtid == 0 && P == 0) w.cnt[CNT_PART_P] = 0;
-    /* a body's part: its own if the partition holds it, else the part whose rank range its
-     * current Morton rank falls in (the block of that part then reads it in global memory) */
-    auto part_of = [&](int b) {
-        const int c = w.b_cidx[b];
-        if (c >= 0 && c < ncache && w.cache_body[c] == b) return w.b_part[b];
-        const int r = w.b_rank[b];
-        if (r >= nf) return -2;
-        int lo = 0, hi = P - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (w.part_rbeg[mid] <= r) lo = mid;
-            else hi = mid - 1;
-        }
-        return lo;
-    };
-    for (int k = gtid; k < n; k += gsize) {
-        const int ci = w.cons_contact[k];
-        int part = -1;
-        if (P > 0) {
-            const int2 bd = w.c.body[ci];
-            const bool da = is_dynamic(w.b_flags[bd.x]), db = is_dynamic(w.b_flags[bd.y]);
-            if (P == 1) {
-                part = 0;  /* one part holds everything; bodies outside its cache stay in global memory */
-            } else {
-                const int pa = !da ? -1 : part_of(bd.x);
-                const int pb = !db ? -1 : part_of(bd.y);
-                part = !da ? pb : (!db ? pa : (pa == pb ? pa : -1));
-                if (part < 0) part = -1;
+            const unsigned long long wtot = all >> 32;
+            /* A batch of worlds cuts only at world boundaries: a world's bodies all take the part of the
+             * weight prefix at the world's first rank (ranks are grouped by world), so no constraint
+             * joins two parts, there are no boundary colours, and the parts never wait for each other.
+             * That needs the prefix at any rank: the chunks' prefixes are made global first. */
+            const bool aligned = w.num_worlds > 1;
+            if (aligned) {
+                for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) w.rank_x[r] += before;
+                if (!grid_barrier(w)) return false;
+            }
+            const unsigned long long base_x = aligned ? 0ull : before;
+            for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
+                const unsigned long long x = base_x + w.rank_x[r];
+                const unsigned long long x1 = r + 1 < r1 ? base_x + w.rank_x[r + 1] : before + carry;
+                if ((uint32_t)x1 == (uint32_t)x || wtot == 0ull) continue;  /* no constraint at this rank */
+                unsigned long long px = x;
+                if (aligned) {
+                    const int first = w.bp_world_first[(uint32_t)(w.bp_key[r] >> kKeyMortonBits)];
+                    if (first >= 0 && first <= r) px = w.rank_x[first];
+                }
+                const int part = min(P - 1, (int)(((px >> 32) * (unsigned long long)P) / wtot));
+                const int c = (int)(uint32_t)x;
+                if (c >= nf) continue;  /* cannot happen: at most one constraint body per rank */
+                const int b = w.f_body[w.bp_val[r]];
+                w.b_part[b] = part;
+                w.b_cidx[b] = c;
+                w.cache_body[c] = b;
+            }
+            if (!grid_barrier(w)) return false;
+            /* each part's range of constraint bodies */
+            ncache = min(nf, (int)(uint32_t)all);
+            for (int c = gtid; c < ncache; c += gsize) {
+                const int part = w.b_part[w.cache_body[c]];
+                if (c == 0 || w.b_part[w.cache_body[c - 1]] != part) {
+                    w.part_cbeg[part] = c;
+                    int rb = w.b_rank[w.cache_body[c]];
+                    if (w.num_worlds > 1) {  /* whole worlds: the range starts at the world's first rank */
+                        const int first = w.bp_world_first[(uint32_t)(w.bp_key[rb] >> kKeyMortonBits)];
+                        if (first >= 0 && first <= rb) rb = first;
+                    }
+                    if (part > 0) w.part_rbeg[part] = rb;
+                }
+                if (c == ncache - 1 || w.b_part[w.cache_body[c + 1]] != part) w.part_cend[part] = c + 1;
+            }
+            if (gtid == 0) {
+                w.cnt[CNT_PART_NCACHE] = ncache;
+                w.cnt[CNT_PART_NF] = nf;
+                w.cnt[CNT_PART_P] = P;
             }
         }
-        w.cons_part[k] = part;
-        const uint32_t cls = part < 0 ? 1u : 0u;
-        const uint32_t kept = w.c.mids[ci].w;
-        w.cons_colour[k] = (keep && (kept >> 7) == stamp && ((kept >> 6) & 1u) == cls) ? (int)(kept & 63u) : -1;
+        if (gtid == 0 && P == 0) w.cnt[CNT_PART_P] = 0;
+        /* a body's part: its own if the partition holds it, else the part whose rank range its
+         * current Morton rank falls in (the block of that part then reads it in global memory) */
+        auto part_of = [&](int b) {
+            const int c = w.b_cidx[b];
+            if (c >= 0 && c < ncache && w.cache_body[c] == b) return w.b_part[b];
+            const int r = w.b_rank[b];
+            if (r >= nf) return -2;
+            int lo = 0, hi = P - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (w.part_rbeg[mid] <= r) lo = mid;
+                else hi = mid - 1;
+            }
+            return lo;
+        };
+        for (int k = gtid; k < n; k += gsize) {
+            const int ci = w.cons_contact[k];
+            int part = -1;
+            if (P > 0) {
+                const int2 bd = w.c.body[ci];
+                const bool da = is_dynamic(w.b_flags[bd.x]), db = is_dynamic(w.b_flags[bd.y]);
+                if (P == 1) {
+                    part = 0;  /* one part holds everything; bodies outside its cache stay in global memory */
+                } else {
+                    const int pa = !da ? -1 : part_of(bd.x);
+                    const int pb = !db ? -1 : part_of(bd.y);
+                    part = !da ? pb : (!db ? pa : (pa == pb ? pa : -1));
+                    if (part < 0 && P > w.num_sms) w.cnt[CNT_PART_SPLIT] = 1;
+                    if (part < 0) part = -1;
+                }
+            }
+            w.cons_part[k] = part;
+            const uint32_t cls = part < 0 ? 1u : 0u;
+            const uint32_t kept = w.c.mids[ci].w;
+            w.cons_colour[k] = (keep && (kept >> 7) == stamp && ((kept >> 6) & 1u) == cls) ? (int)(kept & 63u) : -1;
+        }
+        for (int c = gtid; c < (P + 1) * kMaxColours; c += gsize) w.col_hist[c] = 0;
+        if (gtid == 0) w.cnt[CNT_LIST] = 0;
+        if (!grid_barrier(w)) return false;
+        if (P <= w.num_sms || rebalance || ((volatile int*)w.cnt)[CNT_PART_SPLIT] == 0) break;
+        rebalance = true;
     }
-    for (int c = gtid; c < (P + 1) * kMaxColours; c += gsize) w.col_hist[c] = 0;
-    if (gtid == 0) w.cnt[CNT_LIST] = 0;
-    if (!grid_barrier(w)) return false;
     /* the kept colours are taken at their bodies; the constraints without one are listed (in s_cons, free
      * until the slots are placed): the rounds go over the list alone, as only its members ever offer */
     int* list = w.s_cons;
@@ -594,7 +602,10 @@ __device__ __forceinline__ bool colour_pass(const DevWorld& w, int nparts) {
         w.s_contact[slot] = ci;
         w.s_cons[slot] = k;
     }
-    if (gtid == 0) w.cnt[CNT_COLOURINGS] = (int)next;
+    if (gtid == 0) {
+        w.cnt[CNT_COLOURINGS] = (int)next;
+        w.cnt[CNT_PART_SPLIT] = 0;
+    }
     return true;
 }
 
@@ -1129,6 +1140,7 @@ __device__ __forceinline__ void islands_pass(const DevWorld& w, int allow_sleep)
 
 /* k_solve runs 256 or 512 threads per block (cfg_solver_block); nothing in it depends on which */
 constexpr int kSolveMaxBlock = 512;
+constexpr int kBatchPerSm = 4;  /* resident blocks of a large batch's sweeps, 64 registers a thread */
 
 /* phase 0: integrate velocities (b2_island_private.rs:136-170) */
 __device__ __forceinline__ void integrate_velocities(const DevWorld& w, const StepParams& sp) {
@@ -1246,16 +1258,59 @@ __device__ __forceinline__ void finish_fixtures(const DevWorld& w) {
     if ((threadIdx.x & 31) == 0 && moved) atomicAdd(&w.cnt[CNT_BP_MOVED], (int)moved);
 }
 
+/* phase 4: store impulses (:585-598) and integrate positions (:222-252) */
+__device__ __forceinline__ void store_and_integrate(const DevWorld& w, const StepParams& sp, int ncons) {
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int gsize = gridDim.x * blockDim.x;
+    const float h = sp.dt;
+    for (int k = gtid; k < ncons; k += gsize) {
+        const int ci = w.s_contact[k];
+        const int4 idx = w.vc_idx[k];
+        const float4 imp = w.vc_imp[k];
+        float4 m = w.c.mimp[ci];
+        m.x = imp.x;
+        m.y = imp.y;
+        if (idx.z > 1) {
+            m.z = imp.z;
+            m.w = imp.w;
+        }
+        w.c.mimp[ci] = m;
+    }
+    for (int b = gtid; b < w.n_bodies; b += gsize) {
+        const uint32_t f = w.b_flags[b];
+        if (!(f & BF_ISLAND)) continue;
+        float4 p = w.b_pos[b];
+        float4 v = w.b_vel[b];
+        V2 vv = mk(v.x, v.y);
+        float wv = v.z;
+        V2 translation = scale(h, vv);
+        if (dot(translation, translation) > kMaxTranslationSquared) {
+            float ratio = fdiv(kMaxTranslation, length(translation));
+            vv.x *= ratio;
+            vv.y *= ratio;
+        }
+        float rotation = h * wv;
+        if (rotation * rotation > kMaxRotationSquared) {
+            float ratio = fdiv(kMaxRotation, fabsr(rotation));
+            wv *= ratio;
+        }
+        p.x += h * vv.x;
+        p.y += h * vv.y;
+        p.z += h * wv;
+        w.b_pos[b] = p;
+        w.b_vel[b] = make_float4(vv.x, vv.y, wv, v.w);
+        for (int j = 0; j < sp.pi; ++j) w.isl_minsep[(size_t)j * w.body_cap + b] = 0u;
+    }
+}
+
 /* WHOLE: the solver from the velocities' integration to the fixtures' synchronisation (one cluster); else
  * the sweeps between them, whose kernels before and after it spread over more threads */
 template <bool WHOLE>
 __device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& sp) {
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int gsize = gridDim.x * blockDim.x;
-    const int nb = w.n_bodies;
     const int ncons = w.cnt[CNT_CONS];
     const int ncol = w.cnt[CNT_COLOURS];
-    const float h = sp.dt;
     if (WHOLE) {
         integrate_velocities(w, sp);
         if (!grid_barrier(w)) return false;
@@ -1409,45 +1464,7 @@ __device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& 
             }
         }
     }
-    /* phase 4: store impulses (:585-598) and integrate positions (:222-252) */
-    for (int k = gtid; k < ncons; k += gsize) {
-        const int ci = w.s_contact[k];
-        const int4 idx = w.vc_idx[k];
-        const float4 imp = w.vc_imp[k];
-        float4 m = w.c.mimp[ci];
-        m.x = imp.x;
-        m.y = imp.y;
-        if (idx.z > 1) {
-            m.z = imp.z;
-            m.w = imp.w;
-        }
-        w.c.mimp[ci] = m;
-    }
-    for (int b = gtid; b < nb; b += gsize) {
-        const uint32_t f = w.b_flags[b];
-        if (!(f & BF_ISLAND)) continue;
-        float4 p = w.b_pos[b];
-        float4 v = w.b_vel[b];
-        V2 vv = mk(v.x, v.y);
-        float wv = v.z;
-        V2 translation = scale(h, vv);
-        if (dot(translation, translation) > kMaxTranslationSquared) {
-            float ratio = fdiv(kMaxTranslation, length(translation));
-            vv.x *= ratio;
-            vv.y *= ratio;
-        }
-        float rotation = h * wv;
-        if (rotation * rotation > kMaxRotationSquared) {
-            float ratio = fdiv(kMaxRotation, fabsr(rotation));
-            wv *= ratio;
-        }
-        p.x += h * vv.x;
-        p.y += h * vv.y;
-        p.z += h * wv;
-        w.b_pos[b] = p;
-        w.b_vel[b] = make_float4(vv.x, vv.y, wv, v.w);
-        for (int j = 0; j < sp.pi; ++j) w.isl_minsep[(size_t)j * w.body_cap + b] = 0u;
-    }
+    store_and_integrate(w, sp, ncons);
     if (!grid_barrier(w)) return false;
     /* phase 5: position iterations with the per-island early exit (:257-274).
      * Iteration j accumulates max(-separation) of each island into its own buffer j (all
@@ -1606,6 +1623,114 @@ __global__ void __launch_bounds__(kSolveMaxBlock) k_solve(DevWorld w, StepParams
     solve_pass<false>(w, sp);
 }
 
+/* A large batch's sweeps. Its parts are whole worlds, so nothing waits for another part: a block takes
+ * one part from the warm start to the last velocity iteration, and after the integration one from the first
+ * position iteration to the last. A colour of a part is a few hundred slots and a chain of a microsecond, so
+ * what counts is how many parts an SM works on at once, and L1: the bodies alone are kept in shared memory,
+ * the slots come from L1 and L2 (a part's worth for each resident block stays there between sweeps), one for
+ * each thread. 1.7 M bodies of 4096 worlds, solver: 3640 us with one part for each SM in k_solve; 1855 with
+ * these kernels, four blocks of 256 threads and 32 KB each; 2300 with 52 KB each, which leaves L1 the
+ * smallest share; 2390 with two blocks and registers for two slots a thread, 2320 with one slot, 2290 with
+ * three blocks, 2290 with five; 2160 with two blocks of 512, 2320 with one of 1024. */
+constexpr int kBatchBodies = 2048;  /* cached; a part's others are read in global memory */
+
+/* this block's part, false if it has no constraint */
+__device__ __forceinline__ bool batch_part(const DevWorld& w, PartCtx& pc, int* s_off) {
+    extern __shared__ float4 s_part[];
+    const int p = blockIdx.x;
+    if (w.cnt[CNT_CONS] == 0) return false;
+    if (w.cnt[CNT_COLOURS] != 0 || w.cnt[CNT_PARTS] != (int)gridDim.x) {  /* a boundary constraint: cannot happen */
+        if (threadIdx.x == 0) atomicOr((unsigned*)&w.cnt[CNT_STATUS], ST_PART_MISMATCH);
+        return false;
+    }
+    pc.ncol = w.part_ncol[p];
+    if (pc.ncol == 0) return false;
+    for (int i = threadIdx.x; i <= pc.ncol; i += blockDim.x) s_off[i] = w.part_off[(size_t)p * (kMaxColours + 1) + i];
+    pc.cbeg = w.part_cbeg[p];
+    pc.nloc = max(0, min(w.part_cend[p] - pc.cbeg, kBatchBodies));
+    pc.off = s_off;
+    pc.state = s_part;
+    pc.body = w.cache_body + pc.cbeg;
+    return true;
+}
+
+__global__ void __launch_bounds__(kBlock, kBatchPerSm) k_batch_velocities(const __grid_constant__ DevWorld w,
+                                                                          const __grid_constant__ StepParams sp) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    __shared__ int s_off[kMaxColours + 1];
+    PartCtx pc{};
+    if (!batch_part(w, pc, s_off)) return;
+    part_load(pc, w.b_vel);
+    __syncthreads();
+    for (int k = s_off[0] + threadIdx.x; k < s_off[pc.ncol]; k += blockDim.x) {
+        const int4 idx = w.vc_idx[k];
+        w.vc_code[k] = make_int2(body_code(w, pc, idx.x, (idx.w & 1) != 0), body_code(w, pc, idx.y, (idx.w & 2) != 0));
+    }
+    __syncthreads();
+    if (sp.warm)
+        for (int c = 0; c < pc.ncol; ++c) {
+            for (int k = s_off[c] + threadIdx.x; k < s_off[c + 1]; k += blockDim.x) {
+                const VelSlot sl = coded_vel_slot(w, k);
+                float4 va = ld_body(pc.state, w.b_vel, sl.idx.x), vb = ld_body(pc.state, w.b_vel, sl.idx.y);
+                float4 imp;
+                part_vel_solve(sl, true, va, vb, imp);
+                if (sl.idx.w & 1) st_body(pc.state, w.b_vel, sl.idx.x, va);
+                if (sl.idx.w & 2) st_body(pc.state, w.b_vel, sl.idx.y, vb);
+            }
+            __syncthreads();
+        }
+    for (int it = 0; it < sp.vi; ++it)
+        for (int c = 0; c < pc.ncol; ++c) {
+            for (int k = s_off[c] + threadIdx.x; k < s_off[c + 1]; k += blockDim.x) {
+                const VelSlot sl = coded_vel_slot(w, k);
+                float4 va = ld_body(pc.state, w.b_vel, sl.idx.x), vb = ld_body(pc.state, w.b_vel, sl.idx.y);
+                float4 imp;
+                part_vel_solve(sl, false, va, vb, imp);
+                w.vc_imp[k] = imp;
+                if (sl.idx.w & 1) st_body(pc.state, w.b_vel, sl.idx.x, va);
+                if (sl.idx.w & 2) st_body(pc.state, w.b_vel, sl.idx.y, vb);
+            }
+            __syncthreads();
+        }
+    part_store(pc, w.b_vel);
+}
+
+__global__ void __launch_bounds__(kBlock) k_batch_integrate(const __grid_constant__ DevWorld w,
+                                                            const __grid_constant__ StepParams sp) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    store_and_integrate(w, sp, w.cnt[CNT_CONS]);
+}
+
+__global__ void __launch_bounds__(kBlock, kBatchPerSm) k_batch_positions(const __grid_constant__ DevWorld w,
+                                                                         const __grid_constant__ StepParams sp) {
+    pdl_entry();
+    B2G_RETURN_IF_ABORTED(w);
+    __shared__ int s_off[kMaxColours + 1];
+    PartCtx pc{};
+    if (!batch_part(w, pc, s_off)) return;
+    part_load(pc, w.b_pos);
+    __syncthreads();
+    const float tol = 3.0f * kLinearSlop;
+    for (int it = 0; it < sp.pi; ++it) {
+        uint32_t* cur = w.isl_minsep + (size_t)it * w.body_cap;
+        for (int c = 0; c < pc.ncol; ++c) {
+            for (int k = s_off[c] + threadIdx.x; k < s_off[c + 1]; k += blockDim.x) {
+                const PosSlot sl = coded_pos_slot(w, k);
+                if (island_done(w, sl.island, it, tol)) continue;
+                float4 pa = ld_body(pc.state, w.b_pos, sl.idx.x), pb = ld_body(pc.state, w.b_pos, sl.idx.y);
+                const float ms = solve_position_math(sl, pa, pb);
+                if (sl.idx.w & 1) st_body(pc.state, w.b_pos, sl.idx.x, pa);
+                if (sl.idx.w & 2) st_body(pc.state, w.b_pos, sl.idx.y, pb);
+                agg_atomic_max(cur, sl.island, ms < 0.0f ? __float_as_uint(-ms) : 0u);
+            }
+            __syncthreads();
+        }
+    }
+    part_store(pc, w.b_pos);
+}
+
 /* The passes before and after the sweeps, each a thread for every body, slot or fixture: long chains of
  * gathers, which the persistent kernel's 8 warps an SM left waiting for memory (of the 250k-box pile's solve
  * 1306 us: initialisation 270, bodies and fixtures 60; the solve takes 1020 us with these kernels, that of
@@ -1731,6 +1856,16 @@ int part_count(const DevWorld& w, int num_sms) {
     return std::max(1, std::min(std::min(num_sms, kMaxParts), w.n_fixtures / 256));
 }
 
+/* Parts of a batch large enough for the kernels of its own (0: it is not): one per 512 proxies, from 1024
+ * proxies per SM. Solver, us, with these parts and with one per SM in k_solve: 107k bodies 447 and 408 (whose
+ * bodies and slots nearly fit the shared memory), 250k 491 and 649, 490k 569 and 857, 630k 759 and 1343, 1.7 M
+ * 1855 and 3640. A tape keeps the schedule of at most one part per SM, which its backward pass replays. */
+constexpr int kBatchPart = 512, kBatchMinProxiesPerSm = 1024;
+int batch_parts(const DevWorld& w, int num_sms, bool taped) {
+    const bool large = w.num_worlds > 1 && (long long)w.n_fixtures > (long long)num_sms * kBatchMinProxiesPerSm;
+    return large && !taped ? std::min(kMaxParts, w.n_fixtures / kBatchPart) : 0;
+}
+
 /* In one world the part-local solve pays off while a part's bodies and constraints fit its block's
  * shared memory; a larger world (thousands of proxies per SM) keeps the grid-wide colour sweeps,
  * which spread each colour over every thread of the GPU. A batch of worlds is cut at world
@@ -1745,7 +1880,7 @@ bool use_parts(const DevWorld& w, int num_sms, bool allowed) {
            (w.num_worlds > 1 || (long long)w.n_fixtures <= (long long)num_sms * kPartMaxProxiesPerSm);
 }
 
-void launch_colouring(const DevWorld& w, cudaStream_t s, int num_sms, bool parts) {
+void launch_colouring(const DevWorld& w, cudaStream_t s, int num_sms, bool parts, bool taped) {
     /* more blocks per SM for large worlds: the colouring's passes stride over every
      * constraint and body */
     static int resident = 0;
@@ -1757,6 +1892,8 @@ void launch_colouring(const DevWorld& w, cudaStream_t s, int num_sms, bool parts
     const int blocks = coop_blocks((const void*)k_colour, num_sms) * per_sm;
     DevWorld wc = w;
     int nparts = use_parts(w, num_sms, parts) ? part_count(w, num_sms) : 0;
+    if (nparts > 0)
+        if (const int many = batch_parts(w, num_sms, taped)) nparts = many;
     void* args[] = {&wc, &nparts};
     cudaLaunchCooperativeKernel((const void*)k_colour, dim3(blocks), dim3(kBlock), args, 0, s);
     B2G_LAUNCHED(1);
@@ -1767,6 +1904,7 @@ void launch_colouring(const DevWorld& w, cudaStream_t s, int num_sms, bool parts
  * one part per SM. */
 constexpr int kPartSmemOne = 200 * 1024;
 constexpr int kPartSmemTwo = 96 * 1024;
+constexpr int kBatchSmem = kBatchBodies * (int)sizeof(float4);
 
 /* the solver's shared memory for the part-local solve, set in the parameters it is launched with */
 size_t part_smem(StepParams& sp, int budget) {
@@ -1778,10 +1916,12 @@ size_t part_smem(StepParams& sp, int budget) {
     return (size_t)(budget > 0 ? body_bytes + sp.part_slot_bytes : 0);
 }
 
-int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms, bool parts) {
+int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms, bool parts, bool taped) {
     static bool attr_set = false;
     if (!attr_set) {
         cudaFuncSetAttribute((const void*)k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kPartSmemOne);
+        cudaFuncSetAttribute((const void*)k_batch_velocities, cudaFuncAttributeMaxDynamicSharedMemorySize, kBatchSmem);
+        cudaFuncSetAttribute((const void*)k_batch_positions, cudaFuncAttributeMaxDynamicSharedMemorySize, kBatchSmem);
         attr_set = true;
     }
     const int blocks = coop_blocks((const void*)k_solve, num_sms) * w.cfg_coop_per_sm;
@@ -1796,8 +1936,17 @@ int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int n
     const int gb = grid_for(w.n_bodies, kBlock, num_sms * 8), gc = grid_for(w.cons_cap, kBlock, num_sms * 8);
     launch_pdl(k_solve_velocities, gb, kBlock, 0, s, w, spc);
     launch_pdl(k_solve_init, gc, kBlock, 0, s, w, spc);
-    const int threads = w.cfg_coop_per_sm == 1 && w.cfg_solver_block == kSolveMaxBlock ? kSolveMaxBlock : kBlock;
-    const int rc = (int)cudaLaunchCooperativeKernel((const void*)k_solve, dim3(blocks), dim3(threads), args, smem, s);
+    int rc = 0;
+    const int many = use_parts(w, num_sms, parts) ? batch_parts(w, num_sms, taped) : 0;
+    if (many > 0) {
+        launch_pdl(k_batch_velocities, many, kBlock, kBatchSmem, s, w, spc);
+        launch_pdl(k_batch_integrate, gc, kBlock, 0, s, w, spc);
+        launch_pdl(k_batch_positions, many, kBlock, kBatchSmem, s, w, spc);
+        B2G_LAUNCHED(2);
+    } else {
+        const int threads = w.cfg_coop_per_sm == 1 && w.cfg_solver_block == kSolveMaxBlock ? kSolveMaxBlock : kBlock;
+        rc = (int)cudaLaunchCooperativeKernel((const void*)k_solve, dim3(blocks), dim3(threads), args, smem, s);
+    }
     launch_pdl(k_solve_bodies, gb, kBlock, 0, s, w, spc);
     if (sp.allow_sleep) launch_pdl(k_solve_sleep, gb, kBlock, 0, s, w, spc);
     launch_pdl(k_solve_fixtures, grid_for(w.n_fixtures, kBlock, num_sms * 8), kBlock, 0, s, w);
