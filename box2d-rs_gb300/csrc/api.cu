@@ -197,6 +197,16 @@ int size_bucket(const World* w) {
     return b * 2 + (w->num_worlds > 1 ? 1 : 0);
 }
 
+/* whether circles and polygons both are an eighth of the fixtures or more */
+int mixed_shapes(const World* w) {
+    size_t circles = 0, polygons = 0;
+    for (const ShapeRec& s : w->h_shape) {
+        circles += shape_type(s) == SHAPE_CIRCLE ? 1 : 0;
+        polygons += shape_type(s) == SHAPE_POLYGON ? 1 : 0;
+    }
+    return 8 * std::min(circles, polygons) >= w->h_shape.size() ? 1 : 0;
+}
+
 void apply_launch_config(World* w) {
     if (!w->cfg_set) {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
@@ -562,6 +572,7 @@ int upload(World* w) {
         U(d.f_shape, w->h_shape); U(d.f_body, w->h_fbody); U(d.f_mat, w->h_fmat); U(d.f_filter, w->h_filter);
         U(d.f_group, w->h_group); U(d.f_refid, w->h_refid); U(d.f_fat, w->h_fat); U(d.f_moved, w->h_moved);
         launch_shape_rows(d, nf, s);  /* the narrowphase's structure-of-arrays copy of f_shape */
+        d.mixed_shapes = mixed_shapes(w);
     }
     /* body -> fixtures (the continuous pass synchronises an island body's proxies) */
     w->h_fix_off.assign((size_t)nb + 1, 0);
@@ -2625,6 +2636,7 @@ int load_host_state(World* w, const unsigned char* src, const unsigned char* end
         D(d.f_shape, w->h_shape, nf); D(d.f_body, w->h_fbody, nf); D(d.f_mat, w->h_fmat, nf);
         D(d.f_filter, w->h_filter, nf); D(d.f_group, w->h_group, nf); D(d.f_refid, w->h_refid, nf);
         D(d.f_fat, w->h_fat, nf); D(d.f_moved, w->h_moved, nf);
+        d.mixed_shapes = mixed_shapes(w);
     }
 #undef D
     /* fixture lists, newest first (fixtures are appended in creation order) */

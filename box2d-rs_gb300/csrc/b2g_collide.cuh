@@ -21,6 +21,12 @@
 
 #include "b2g_math.cuh"
 
+#ifdef __CUDA_ARCH__
+#define B2G_UNROLL _Pragma("unroll")
+#else
+#define B2G_UNROLL
+#endif
+
 namespace b2g {
 
 enum { SHAPE_CIRCLE = 0, SHAPE_EDGE = 1, SHAPE_POLYGON = 2 };
@@ -112,15 +118,16 @@ B2G_HD void shape_aabb(const ShapeRec& s, const Xf& xf, AABB& out) {
 }
 
 B2G_HD int clip_segment(ClipV out[2], const ClipV in[2], V2 normal, float offset, int vertex_index_a) {
-    int count = 0;
     float d0 = dot(normal, in[0].v) - offset;
     float d1 = dot(normal, in[1].v) - offset;
-    if (d0 <= 0.0f) out[count++] = in[0];
-    if (d1 <= 0.0f) out[count++] = in[1];
+    /* the points behind the plane in order, then the crossing: d0 d1 < 0 leaves it one of the two */
+    int count = (d0 <= 0.0f ? 1 : 0) + (d1 <= 0.0f ? 1 : 0);
+    out[0] = d0 <= 0.0f ? in[0] : in[1];
+    out[1] = in[1];
     if (d0 * d1 < 0.0f) {
         float interp = fdiv(d0, d0 - d1);
-        out[count].v = add(in[0].v, scale(interp, sub(in[1].v, in[0].v)));
-        out[count].id = feature((uint32_t)vertex_index_a, (in[0].id >> 8) & 0xffu, FEATURE_VERTEX, FEATURE_FACE);
+        out[1].v = add(in[0].v, scale(interp, sub(in[1].v, in[0].v)));
+        out[1].id = feature((uint32_t)vertex_index_a, (in[0].id >> 8) & 0xffu, FEATURE_VERTEX, FEATURE_FACE);
         ++count;
     }
     return count;
@@ -197,19 +204,35 @@ B2G_HD void collide_polygon_circle(Manifold& m, const S& poly, const Xf& xfA, co
     }
 }
 
+/* poly2's vertices are read once, into registers (a shape holds eight rows, used or not): read again for
+ * each edge of poly1 they were most of the pass's L1 traffic, 16 bytes of another line in every lane. */
 template <class S>
 B2G_HD float find_max_separation(int& edgeIndex, const S& p1, const Xf& xf1, const S& p2, const Xf& xf2) {
     Xf xf = mul_t(xf2, xf1);
     int n1 = sh_count(p1), n2 = sh_count(p2);
+    V2 w[kMaxPolygonVertices];
+    const bool wide = n2 > 4;
+    B2G_UNROLL
+    for (int j = 0; j < 4; ++j) w[j] = sh_v(p2, j);
+    B2G_UNROLL
+    for (int j = 4; j < kMaxPolygonVertices; ++j) w[j] = wide ? sh_v(p2, j) : w[0];
     int best = 0;
     float maxSep = -kMaxFloat;
     for (int i = 0; i < n1; ++i) {
         V2 n = mul(xf.q, sh_n(p1, i));
         V2 v1 = mul(xf, sh_v(p1, i));
         float si = kMaxFloat;
-        for (int j = 0; j < n2; ++j) {
-            float sij = dot(n, sub(sh_v(p2, j), v1));
-            if (sij < si) si = sij;
+        B2G_UNROLL
+        for (int j = 0; j < 4; ++j) {
+            float sij = dot(n, sub(w[j], v1));
+            if (j < n2 && sij < si) si = sij;
+        }
+        if (wide) {
+            B2G_UNROLL
+            for (int j = 4; j < kMaxPolygonVertices; ++j) {
+                float sij = dot(n, sub(w[j], v1));
+                if (j < n2 && sij < si) si = sij;
+            }
         }
         if (si > maxSep) {
             maxSep = si;
@@ -232,8 +255,8 @@ B2G_HD void collide_polygons(Manifold& m, const S& A, const Xf& xfA, const S& B,
     if (sepB > totalRadius) return;
     const float kTol = 0.1f * kLinearSlop;
     const bool flip = sepB > sepA + kTol;
-    const S& poly1 = flip ? B : A;
-    const S& poly2 = flip ? A : B;
+    const S poly1 = flip ? B : A;
+    const S poly2 = flip ? A : B;
     const Xf xf1 = flip ? xfB : xfA;
     const Xf xf2 = flip ? xfA : xfB;
     const int edge1 = flip ? edgeB : edgeA;
@@ -280,16 +303,19 @@ B2G_HD void collide_polygons(Manifold& m, const S& A, const Xf& xfA, const S& B,
     if (clip_segment(cp2, cp1, tangent, sideOffset2, iv2) < 2) return;
     m.ln = localNormal;
     m.lp = planePoint;
-    int pc = 0;
-    for (int i = 0; i < 2; ++i) {
-        float separation = dot(normal, cp2[i].v) - frontOffset;
-        if (separation <= totalRadius) {
-            m.p[pc] = mul_t(xf2, cp2[i].v);
-            m.id[pc] = flip ? feature_swap(cp2[i].id) : cp2[i].id;
-            ++pc;
-        }
+    const bool keep0 = dot(normal, cp2[0].v) - frontOffset <= totalRadius;
+    const bool keep1 = dot(normal, cp2[1].v) - frontOffset <= totalRadius;
+    const V2 q0 = mul_t(xf2, cp2[0].v), q1 = mul_t(xf2, cp2[1].v);
+    const uint32_t id0 = flip ? feature_swap(cp2[0].id) : cp2[0].id, id1 = flip ? feature_swap(cp2[1].id) : cp2[1].id;
+    if (keep0 || keep1) {
+        m.p[0] = keep0 ? q0 : q1;
+        m.id[0] = keep0 ? id0 : id1;
     }
-    m.count = pc;
+    if (keep0 && keep1) {
+        m.p[1] = q1;
+        m.id[1] = id1;
+    }
+    m.count = (keep0 ? 1 : 0) + (keep1 ? 1 : 0);
 }
 
 template <class S>
@@ -502,21 +528,21 @@ B2G_HD void collide_edge_polygon(Manifold& m, const S& edge, const Xf& xfA, cons
         m.ln = sh_n(poly, ri1);
         m.lp = sh_v(poly, ri1);
     }
-    int pc = 0;
-    for (int i = 0; i < 2; ++i) {
-        float separation = dot(rnormal, sub(cp2[i].v, rv1));
-        if (separation <= radius) {
-            if (primaryType == 0) {
-                m.p[pc] = mul_t(xf, cp2[i].v);
-                m.id[pc] = cp2[i].id;
-            } else {
-                m.p[pc] = cp2[i].v;
-                m.id[pc] = feature_swap(cp2[i].id);
-            }
-            ++pc;
-        }
+    const bool keep0 = dot(rnormal, sub(cp2[0].v, rv1)) <= radius;
+    const bool keep1 = dot(rnormal, sub(cp2[1].v, rv1)) <= radius;
+    const V2 q0 = primaryType == 0 ? mul_t(xf, cp2[0].v) : cp2[0].v;
+    const V2 q1 = primaryType == 0 ? mul_t(xf, cp2[1].v) : cp2[1].v;
+    const uint32_t id0 = primaryType == 0 ? cp2[0].id : feature_swap(cp2[0].id);
+    const uint32_t id1 = primaryType == 0 ? cp2[1].id : feature_swap(cp2[1].id);
+    if (keep0 || keep1) {
+        m.p[0] = keep0 ? q0 : q1;
+        m.id[0] = keep0 ? id0 : id1;
     }
-    m.count = pc;
+    if (keep0 && keep1) {
+        m.p[1] = q1;
+        m.id[1] = id1;
+    }
+    m.count = (keep0 ? 1 : 0) + (keep1 ? 1 : 0);
 }
 
 template <class S>
@@ -640,16 +666,19 @@ __device__ __forceinline__ void collide_polygons_group(Manifold& m, int lane, fl
     if (clip_segment(cp2, cp1, tangent, sideOffset2, iv2) < 2) return;
     m.ln = localNormal;
     m.lp = planePoint;
-    int pc = 0;
-    for (int i = 0; i < 2; ++i) {
-        float separation = dot(normal, cp2[i].v) - frontOffset;
-        if (separation <= totalRadius) {
-            m.p[pc] = mul_t(xf2, cp2[i].v);
-            m.id[pc] = flip ? feature_swap(cp2[i].id) : cp2[i].id;
-            ++pc;
-        }
+    const bool keep0 = dot(normal, cp2[0].v) - frontOffset <= totalRadius;
+    const bool keep1 = dot(normal, cp2[1].v) - frontOffset <= totalRadius;
+    const V2 q0 = mul_t(xf2, cp2[0].v), q1 = mul_t(xf2, cp2[1].v);
+    const uint32_t id0 = flip ? feature_swap(cp2[0].id) : cp2[0].id, id1 = flip ? feature_swap(cp2[1].id) : cp2[1].id;
+    if (keep0 || keep1) {
+        m.p[0] = keep0 ? q0 : q1;
+        m.id[0] = keep0 ? id0 : id1;
     }
-    m.count = pc;
+    if (keep0 && keep1) {
+        m.p[1] = q1;
+        m.id[1] = id1;
+    }
+    m.count = (keep0 ? 1 : 0) + (keep1 ? 1 : 0);
 }
 
 /* Which pair of a batch this lane's segment takes: of the lanes in `todo` (a warp-uniform mask of

@@ -80,7 +80,9 @@ __device__ __forceinline__ bool contact_finish(const DevWorld& w, bool record_ev
     const int old_count = (int)((ids.z >> 8) & 0xffu);
     flags |= CF_ENABLED | set_flags;
     float ni[2] = {0.0f, 0.0f}, ti[2] = {0.0f, 0.0f};
-    for (int p = 0; p < m.count; ++p) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        if (p >= m.count) break;
         if (old_count > 0 && ids.x == m.id[p]) {
             ni[p] = oldimp.x;
             ti[p] = oldimp.y;

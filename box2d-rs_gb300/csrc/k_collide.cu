@@ -18,7 +18,8 @@
  *   - otherwise evaluate the manifold with the routine of the contact's kind, carry
  *     normal/tangent impulses from old points with the same feature id, update the
  *     touching flag, wake both bodies when it changes, and emit begin/end events.
- * Then the batch's manifolds: one lane per pair, or, for a batch with at most cfg_collide_group
+ * Then the manifolds. Small worlds and large worlds of mixed shapes list a block's contacts by kind first
+ * (k_collide_tiles); else a batch's manifolds as they come (k_collide): one lane per pair, or, for a batch with at most cfg_collide_group
  * polygon pairs, those pairs four at a time, eight lanes to a pair (collide_polygons_group: lane k
  * holds row k of both polygons; the default, 0, keeps one lane per pair, which measured at least as
  * fast on GB300). Shapes are read from the structure-of-arrays rows (f_vn, f_hdr): a polygon's used
@@ -166,7 +167,8 @@ __device__ __forceinline__ bool warp_aborted(const DevWorld& w) {
 
 }  // namespace
 
-__global__ void __launch_bounds__(256, 4) k_collide(DevWorld w, StepParams sp, int deferred, int starts_step) {
+__global__ void __launch_bounds__(256, 4) k_collide(const __grid_constant__ DevWorld w, const __grid_constant__ StepParams sp,
+                                                    int deferred, int starts_step) {
     pdl_entry();
     if (warp_aborted(w)) return;
     if (starts_step) phase_stamp(w, PH_START);
@@ -182,6 +184,108 @@ __global__ void __launch_bounds__(256, 4) k_collide(DevWorld w, StepParams sp, i
         const int state = i < n ? collide_head(w, sp, i, deferred != 0, h) : HEAD_SKIPPED;
         if (deferred && i < n) w.c_done[i] = state != HEAD_SKIPPED ? 1 : 0;
         collide_batch(w, sp, i, state, h, deferred != 0);
+    }
+}
+
+/* The pass by tiles: a block takes the heads of up to kTile consecutive contacts, lists those to evaluate
+ * by kind, and its warps take 32 of one kind at a time: neighbours in the table are of all kinds, and a warp
+ * that evaluates one contact per lane runs the routine of every kind it holds one after another (seven lanes
+ * of 32 at work on average, twelve here). A block with few polygon pairs takes them four to a warp, eight
+ * lanes to a pair, and the kinds run side by side in its warps. Bound by instruction issue and by L1 (each
+ * lane reads rows of its own shapes); 8.0 M contacts of 4096 worlds 609 us, 780 in k_collide (1031 before the
+ * polygon routine kept its vertices in registers). */
+constexpr int kTile = 512;
+constexpr int kKinds = 5;
+constexpr int kKindsSmall = 2048, kKindsProxiesPerSm = 1024;
+
+__global__ void __launch_bounds__(256, 4) k_collide_tiles(const __grid_constant__ DevWorld w,
+                                                          const __grid_constant__ StepParams sp, int deferred,
+                                                          int starts_step) {
+    pdl_entry();
+    if (warp_aborted(w)) return;
+    if (starts_step) phase_stamp(w, PH_START);
+    phase_stamp(w, PH_INITIAL);
+    if (blockIdx.x == 0 && threadIdx.x < 3) w.cnt[CNT_CASCADE + threadIdx.x] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) w.cnt[CNT_BARRIER] = w.cnt[CNT_BARRIER2] = 0;
+    __shared__ uint16_t s_list[kKinds][kTile];
+    __shared__ int s_count[kKinds];
+    const int n = w.cnt[CNT_CONTACTS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const bool rec = sp.record_events != 0;
+    const uint32_t set_flags = sp.pre_solve ? CF_UPDATED : 0u;
+    const int share = (n + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int tile = max(32, min(kTile, (share + 31) & ~31));
+    for (int t0 = blockIdx.x * tile; t0 < n; t0 += gridDim.x * tile) {
+        if (threadIdx.x < kKinds) s_count[threadIdx.x] = 0;
+        __syncthreads();
+        for (int j = threadIdx.x; j < tile; j += blockDim.x) {
+            const int i = t0 + j;
+            Head h;
+            const int state = i < n ? collide_head(w, sp, i, deferred != 0, h) : HEAD_SKIPPED;
+            if (deferred && i < n) w.c_done[i] = state != HEAD_SKIPPED ? 1 : 0;
+            const int kind = state == HEAD_EVALUATE ? min((int)((h.flags >> CF_KIND_SHIFT) & 7u), kKinds - 1) : -1;
+            const unsigned same = __match_any_sync(kFullWarp, kind);
+            const int first = __ffs((int)same) - 1;
+            int at = 0;
+            if (lane == first && kind >= 0) at = atomicAdd(&s_count[kind], __popc(same));
+            at = __shfl_sync(kFullWarp, at, first) + __popc(same & ((1u << lane) - 1u));
+            if (kind >= 0) s_list[kind][at] = (uint16_t)j;
+        }
+        __syncthreads();
+        const int np = s_count[KIND_POLYGONS];
+        const bool segments = np <= 8 * warps;
+        if (segments) {
+            const int seg = lane >> 3, row = lane & 7;
+            for (int p0 = 4 * warp; p0 < np; p0 += 4 * warps) {
+                const bool mine = p0 + seg < np;
+                const int i = mine ? t0 + s_list[KIND_POLYGONS][p0 + seg] : 0;
+                float4 la = make_float4(0.0f, 0.0f, 0.0f, 0.0f), lb = la, ha = la, hb = la;
+                Xf xa, xb;
+                xa.p = xb.p = mk(0.0f, 0.0f);
+                xa.q.s = xb.q.s = 0.0f;
+                xa.q.c = xb.q.c = 1.0f;
+                int2 fx = make_int2(0, 0), bd = fx;
+                if (mine) {
+                    fx = w.c.fix[i];
+                    bd = w.c.body[i];
+                    ha = w.f_hdr[fx.x];
+                    hb = w.f_hdr[fx.y];
+                    la = w.f_vn[(size_t)fx.x * kMaxPolygonVertices + row];
+                    lb = w.f_vn[(size_t)fx.y * kMaxPolygonVertices + row];
+                    xa = load_xf(w, bd.x);
+                    xb = load_xf(w, bd.y);
+                }
+                Manifold m;
+                manifold_init(m);
+                collide_polygons_group(m, row, la, (__float_as_int(ha.w) >> 8) & 0xff, ha.z, xa, lb,
+                                       (__float_as_int(hb.w) >> 8) & 0xff, hb.z, xb);
+                if (mine && row == 0)
+                    contact_finish(w, rec, i, w.c.flags[i], fx, bd, w.c.mids[i], w.c.mimp[i], m, deferred ? i : -1, set_flags);
+            }
+        }
+        /* the other kinds (and many polygon pairs) from the last warp down: few pairs leave those idle */
+        int g = warps - 1 - warp;
+#pragma unroll 1
+        for (int kk = 0; kk < kKinds; ++kk) {
+            const int kind = kk == 0 ? KIND_POLYGONS : kk <= KIND_POLYGONS ? kk - 1 : kk;
+            const int count = s_count[kind], groups = kind == KIND_POLYGONS && segments ? 0 : (count + 31) >> 5;
+            for (; g < groups; g += warps) {
+                const int q = 32 * g + lane;
+                if (q >= count) continue;
+                const int i = t0 + s_list[kind][q];
+                const uint32_t flags = w.c.flags[i];
+                const int2 fx = w.c.fix[i];
+                const int2 bd = w.c.body[i];
+                const uint4 ids = w.c.mids[i];
+                const float4 imp = w.c.mimp[i];
+                Manifold m;
+                manifold_init(m);
+                evaluate(kind, m, shape_rows(w, fx.x), load_xf(w, bd.x), shape_rows(w, fx.y), load_xf(w, bd.y));
+                contact_finish(w, rec, i, flags, fx, bd, ids, imp, m, deferred ? i : -1, set_flags);
+            }
+            g -= groups;
+        }
+        __syncthreads();
     }
 }
 
@@ -322,10 +426,19 @@ void launch_shape_rows(const DevWorld& w, int n_fixtures, cudaStream_t s) {
     B2G_LAUNCHED(1);
 }
 
+/* k_collide_tiles or k_collide, us: 42 contacts 7.5 and 10.7, 1200 7.9 and 10.3, 5000 8.9 and 9.6, 16.5k 10.3
+ * both, 25k 10.2 and 9.3, 164k 25.7 and 21.9 (a block's tile is a part of a warp's worth of each kind), 440k
+ * 37 and 34; mixed shapes in larger worlds, 1.2 M 102 and 122, 2.9 M 235 and 296, 8.0 M 609 and 780; 2.9 M
+ * contacts of boxes alone 197 and 174. */
+static bool by_kind(const DevWorld& w) {
+    return w.n_fixtures <= kKindsSmall || (w.mixed_shapes && w.n_fixtures > kKindsProxiesPerSm * w.num_sms);
+}
+
 void launch_collide(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool may_sleep, int num_sms,
                     bool starts_step) {
     const int block = w.cfg_collide_block;
-    launch_pdl(k_collide, grid_for(w.contact_cap, block, w.num_sms * 2048 / block), block, 0, s, w, sp, may_sleep ? 1 : 0,
+    const auto kernel = w.cfg_collide_group > 0 || !by_kind(w) ? k_collide : k_collide_tiles;
+    launch_pdl(kernel, grid_for(w.contact_cap, block, w.num_sms * 2048 / block), block, 0, s, w, sp, may_sleep ? 1 : 0,
                starts_step ? 1 : 0);
     B2G_LAUNCHED(1);
     if (!may_sleep) return;
