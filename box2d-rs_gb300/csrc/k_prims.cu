@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kSortBlock) k_radix_coop(unsigned long long* k
     grid_barrier_start(barrier_word);
     const int n = load_n(d_n, max_n);
     if (n > kSortTile && n <= kRankSort && max_n > kSortTile) return;  /* the rank count sorted it */
-    radix_sort_grid(ka, va, kb, vb, n, bits, hist, cnt);
+    radix_sort_grid(ka, va, kb, vb, n, bits, hist, cnt, sort_hist_tiles(max_n));
 }
 
 __global__ void k_copy_pairs(const unsigned long long* __restrict__ kin, const uint32_t* __restrict__ vin,
