@@ -268,7 +268,7 @@ struct DevWorld {
     unsigned long long* rank_x;  /* per Morton rank: constraint endpoints << 32 | has-any, then
                                     its exclusive prefix within the scanning block's chunk */
     unsigned long long* blk_tot; /* per block of a cooperative launch (at least kMaxParts and 8 per SM): chunk
-                                    totals of that scan and of k_islands' constraint count */
+                                    totals of that scan, of the constraint count and of the merge's count */
     int* cache_body;             /* constraint bodies in rank order */
     int* part_cbeg;              /* kMaxParts: each part's first entry of cache_body */
     int* part_cend;              /* kMaxParts: one past its last */

@@ -19,10 +19,12 @@
  *               one colour per round). Constraints of one colour share no dynamic body, so
  *               each colour is solved in parallel with results identical to any sequential
  *               order.
- *   solver      one persistent cooperative kernel: integrate velocities, initialise
- *               constraints, warm start, velocity iterations, store impulses, integrate
- *               positions, position iterations with the per-island early exit, write
- *               back transforms, sleep, synchronise fixtures (fat AABB + moved flag).
+ *   solver      integrate velocities, initialise constraints, warm start, velocity
+ *               iterations, store impulses, integrate positions, position iterations with the
+ *               per-island early exit, write back transforms, sleep, synchronise fixtures (fat
+ *               AABB + moved flag): the sweeps as one persistent cooperative kernel with
+ *               full-occupancy kernels before and after it, as kernels of a block per part
+ *               (large batches), or with islands and colouring on one cluster (small worlds).
  *               Colour sweeps are separated by a grid barrier whose wait is bounded:
  *               on timeout it sets ST_BARRIER_TIMEOUT and the kernel returns.
  * The host reference solved in the GPU's colour order (the oracle's ordering hook)

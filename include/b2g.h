@@ -175,7 +175,7 @@ typedef struct b2g_body_state {
     b2g_vec2 world_center;     /* m_sweep.c (get_world_center)  */
 } b2g_body_state;
 
-/* B2Profile, src/b2_time_step.rs:5-14; milliseconds measured with CUDA events. */
+/* B2Profile, src/b2_time_step.rs:5-14; milliseconds between time stamps that the step's kernels leave in device memory. */
 typedef struct b2g_profile {
     float step, collide, solve, solve_init, solve_velocity, solve_position, broadphase, solve_toi;
 } b2g_profile;
@@ -355,7 +355,7 @@ int b2g_state_load(void* world, const void* in, uint64_t bytes);
 /* Continuous physics: solid time-of-impact events solved since the world was made, the
  * iterations of the last step's pass, and the passes restarted one event at a time. */
 int b2g_get_toi_stats(void* world, int32_t* events, int32_t* last_iterations, int32_t* restarts);
-/* Device times (ms, CUDA events) of the last step's phases, n >= 7: initial broadphase (only
+/* Device times (ms, from time stamps of the step's kernels) of the last step's phases, n >= 7: initial broadphase (only
  * after fixtures were added), collide, islands + constraint list, colouring, solver kernel,
  * broadphase tree pass (keys, sort, hierarchy, traversal), contact merge (with the continuous
  * pass when it runs); with n >= 10 also the tree pass in three: keys + sort, hierarchy (build,
@@ -590,10 +590,12 @@ typedef struct b2g_launch_config {
     int32_t traverse_block;       /* broadphase traversal threads per block: 32..256, power of two */
     int32_t tuning_steps;         /* out: steps the world's last b2g_autotune ran (ignored on set) */
     int32_t solver_block;         /* solver threads per block: 256, or 512 with one block per SM (more
-                                     loads in flight on large worlds and batches); 0 on set: 256 */
+                                     loads in flight on large worlds); 0 on set: 256. The sweeps of a
+                                     large batch have block sizes of their own */
     int32_t collide_group;        /* narrowphase pairs per warp: a warp's batch of 32 contacts with at
                                      most this many polygon pairs evaluates each of them on 8 lanes (4
-                                     pairs at a time); more, one lane per pair. 0..32, default 0 */
+                                     pairs at a time); more, one lane per pair. 0..32, default 0: one
+                                     lane per pair, contacts listed by kind first where that is faster */
 } b2g_launch_config;
 int b2g_get_launch_config(void* world, b2g_launch_config* out);
 int b2g_set_launch_config(void* world, const b2g_launch_config* config);
