@@ -208,16 +208,21 @@ int mixed_shapes(const World* w) {
 }
 
 void apply_launch_config(World* w) {
+    bool chosen = w->cfg_set;
     if (!w->cfg_set) {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         const int b = size_bucket(w);
         for (auto& e : g_tuned)
-            if (e.first == b) w->cfg = e.second;
+            if (e.first == b) {
+                w->cfg = e.second;
+                chosen = true;
+            }
     }
     w->d.cfg_coop_per_sm = w->cfg.coop_per_sm;
     w->d.cfg_collide_block = w->cfg.collide_block;
     w->d.cfg_traverse_block = w->cfg.traverse_block;
     w->d.cfg_solver_block = w->cfg.coop_per_sm == 1 ? w->cfg.solver_block : 256;
+    w->d.cfg_solver_auto = chosen ? 0 : 1;
     w->d.cfg_collide_group = w->cfg.collide_group;
 }
 

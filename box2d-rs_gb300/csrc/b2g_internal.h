@@ -198,6 +198,7 @@ struct DevWorld {
     int cfg_collide_block;    /* threads per block of the narrowphase */
     int cfg_traverse_block;   /* threads per block of the broadphase traversal */
     int cfg_solver_block;     /* threads per block of the persistent solver (256, or 512 at one block per SM) */
+    int cfg_solver_auto;      /* nobody chose it: by the world's size */
     int mixed_shapes;         /* circles and polygons are both a good share of the fixtures */
     int cfg_collide_group;    /* narrowphase: a warp batch with at most this many polygon pairs evaluates
                                  them eight lanes to a pair (collide_polygons_group); more, a lane each */

@@ -1918,6 +1918,17 @@ size_t part_smem(StepParams& sp, int budget) {
     return (size_t)(budget > 0 ? body_bytes + sp.part_slot_bytes : 0);
 }
 
+/* 512 threads for k_solve where no configuration says otherwise: in a batch, whose parts are solved without
+ * waiting for each other, and in a world whose parts have more slots than their caches hold; more barrier
+ * arrivals are all that a small world gets from them. Solver, us, with 256 and 512: batches of 64 worlds of up
+ * to 2048 bodies 351 and 311, 256 such 420 and 365, 2048 of up to 128 175 and 161, 512 of up to 128 91 and
+ * 92; piles of 50k boxes 575 and 583, 100k 712 and 713, 150k 787 and 759, 250k 1118 and 1056; 30k bodies 421
+ * and 429. */
+constexpr int kWideProxiesPerSm = 896;
+static bool wide_solver(const DevWorld& w, int num_sms) {
+    return w.num_worlds > 1 || (long long)w.n_fixtures > (long long)num_sms * kWideProxiesPerSm;
+}
+
 int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms, bool parts, bool taped) {
     static bool attr_set = false;
     if (!attr_set) {
@@ -1946,7 +1957,8 @@ int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int n
         launch_pdl(k_batch_positions, many, kBlock, kBatchSmem, s, w, spc);
         B2G_LAUNCHED(2);
     } else {
-        const int threads = w.cfg_coop_per_sm == 1 && w.cfg_solver_block == kSolveMaxBlock ? kSolveMaxBlock : kBlock;
+        const bool wide = w.cfg_solver_auto ? wide_solver(w, num_sms) : w.cfg_solver_block == kSolveMaxBlock;
+        const int threads = w.cfg_coop_per_sm == 1 && wide ? kSolveMaxBlock : kBlock;
         rc = (int)cudaLaunchCooperativeKernel((const void*)k_solve, dim3(blocks), dim3(threads), args, smem, s);
     }
     launch_pdl(k_solve_bodies, gb, kBlock, 0, s, w, spc);

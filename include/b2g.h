@@ -590,8 +590,10 @@ typedef struct b2g_launch_config {
     int32_t traverse_block;       /* broadphase traversal threads per block: 32..256, power of two */
     int32_t tuning_steps;         /* out: steps the world's last b2g_autotune ran (ignored on set) */
     int32_t solver_block;         /* solver threads per block: 256, or 512 with one block per SM (more
-                                     loads in flight on large worlds); 0 on set: 256. The sweeps of a
-                                     large batch have block sizes of their own */
+                                     loads in flight on large worlds); 0 on set: 256. A world that no
+                                     configuration was set for or tuned to reads 256 and takes 512
+                                     where it is larger or a batch; a large batch's sweeps have block
+                                     sizes of their own */
     int32_t collide_group;        /* narrowphase pairs per warp: a warp's batch of 32 contacts with at
                                      most this many polygon pairs evaluates each of them on 8 lanes (4
                                      pairs at a time); more, one lane per pair. 0..32, default 0: one
