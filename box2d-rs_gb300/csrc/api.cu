@@ -79,6 +79,7 @@ struct TapeHost {
     int ckpt_every = 16;
     int steps = 0;                 /* steps with dt > 0 issued while recording */
     int n_bodies = 0;
+    int contact_cap = 0;           /* entries of the contact maps */
     size_t bytes = 0;
     /* backward work buffers and the sizes they were made for */
     AdjWork work{};
@@ -3515,6 +3516,21 @@ int talloc(World* w, std::vector<void*>& mem, size_t& bytes, T** p, size_t n) {
     return B2G_OK;
 }
 
+/* recording begins on t's buffers */
+int tape_start(World* w, TapeHost* t) {
+    TapeDev& d = t->d;
+    t->valid = true;
+    t->steps = 0;
+    t->mismatches = 0;
+    cudaMemsetAsync(d.cnt, 0, TAPE_CNT_SIZE * sizeof(long long), w->stream);
+    cudaMemsetAsync(d.cmap[0], 0, (size_t)w->d.contact_cap * sizeof(unsigned long long), w->stream);
+    cudaMemsetAsync(d.cmap[1], 0, (size_t)w->d.contact_cap * sizeof(unsigned long long), w->stream);
+    CUDA_OK(w, cudaGetLastError());
+    t->recording = true;
+    drop_graphs(w);  /* the step graphs gain the recording kernels */
+    return B2G_OK;
+}
+
 int tape_final_index(const TapeHost* t) { return t->step_cap / t->ckpt_every + 1; }
 
 int tape_status(World* w, TapeHost* t, long long* steps, long long* slots) {
@@ -3604,12 +3620,22 @@ int b2g_tape_begin(void* p, int32_t max_steps, int32_t every, int64_t max_slots)
     if (!w->joints.empty()) return fail(w, B2G_ERR_UNSUPPORTED, "the tape does not record joints");
     int rc = prepare(w);
     if (rc != B2G_OK) return rc;
+    const int interval = every > 0 ? every : 16;
+    const long long slot_cap = max_slots > 0 ? (long long)max_slots : (long long)max_steps * (4LL * w->d.n_fixtures + 1024);
+    /* the last tape's buffers serve a new one of the same sizes (an optimisation records the same steps each
+     * iteration): 4 ms of allocation for 64 steps of 512 worlds */
+    if (TapeHost* t = w->tape) {
+        if (t->step_cap == max_steps && t->slot_cap == slot_cap && t->ckpt_every == interval &&
+            t->n_bodies == w->d.n_bodies && t->contact_cap == w->d.contact_cap)
+            return tape_start(w, t);
+    }
     tape_free(w);
     TapeHost* t = new TapeHost;
-    t->ckpt_every = every > 0 ? every : 16;
+    t->ckpt_every = interval;
     t->step_cap = max_steps;
-    t->slot_cap = max_slots > 0 ? (long long)max_slots : (long long)max_steps * (4LL * w->d.n_fixtures + 1024);
+    t->slot_cap = slot_cap;
     t->n_bodies = w->d.n_bodies;
+    t->contact_cap = w->d.contact_cap;
     const size_t nck = (size_t)(max_steps / t->ckpt_every + 2) * t->n_bodies;
     TapeDev& d = t->d;
     auto A = [&](auto** ptr, size_t n) {
@@ -3638,14 +3664,8 @@ int b2g_tape_begin(void* p, int32_t max_steps, int32_t every, int64_t max_slots)
     d.step_cap = max_steps;
     d.ckpt_every = t->ckpt_every;
     d.n_bodies = t->n_bodies;
-    cudaMemsetAsync(d.cnt, 0, TAPE_CNT_SIZE * sizeof(long long), w->stream);
-    cudaMemsetAsync(d.cmap[0], 0, (size_t)w->d.contact_cap * sizeof(unsigned long long), w->stream);
-    cudaMemsetAsync(d.cmap[1], 0, (size_t)w->d.contact_cap * sizeof(unsigned long long), w->stream);
-    CUDA_OK(w, cudaGetLastError());
-    t->recording = true;
     w->tape = t;
-    drop_graphs(w);  /* the step graphs gain the recording kernels */
-    return B2G_OK;
+    return tape_start(w, t);
 }
 
 int b2g_tape_end(void* p) {
