@@ -292,7 +292,7 @@ struct DevWorld {
     float4* bp_node_b1;          /* internal node: child 1 box */
     int2* bp_node_child;         /* child indices; leaves encoded as ~leaf */
     int* bp_parent;              /* parent of internal nodes [0,n-1) and leaves [n-1, 2n-1) */
-    uint32_t* bp_flag;           /* refit arrival counters */
+    uint32_t* bp_flag;           /* no longer used: its place in the layout of saved states */
     float4* bp_quad_box;         /* internal node: its grandchildren's boxes (4 per node; a leaf child
                                     stands for itself), so a walk descends two levels per fetch */
     int4* bp_quad_child;         /* the 4 entries (encoded like children; INT_MIN: none) */
