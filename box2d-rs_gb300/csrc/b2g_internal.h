@@ -139,6 +139,7 @@ enum {
     CNT_LIST = 59,           /* colouring: constraints that keep no colour of the previous colouring */
     CNT_BP_LIST = 60,        /* leaves of moved proxies listed for this pass's traversal (in bp_val_alt) */
     CNT_PART_SPLIT = 61,     /* a kept partition of more parts than SMs has split a world */
+    CNT_ISLAND_SPAN = 62,    /* a kinematic body may have made an island of several parts */
     CNT_SIZE = 64
 };
 

@@ -305,8 +305,9 @@ __device__ __forceinline__ bool colour_pass(const DevWorld& w, int nparts) {
      * part whose rank range its Morton rank falls in. (Kept colours stay proper across a new
      * partition: interior constraints that share a body are always in the same part.) More parts than
      * SMs, a batch's, have a solver without boundary sweeps: should a kept partition have put a world's
-     * bodies into two parts (Morton ranks move when a large static proxy changes hierarchies), it is made
-     * afresh after all, which puts every world into one part. */
+     * bodies into two parts (Morton ranks move when a large static proxy changes hierarchies), which a
+     * constraint between the parts or one at a kinematic body shows, it is made afresh after all, which puts
+     * every world into one part. */
     bool rebalance = P > 0 && ((stamp & 3u) == 0u || w.cnt[CNT_PART_P] != P || w.cnt[CNT_PART_NF] != nf);
     int ncache = w.cnt[CNT_PART_NCACHE];  /* read before any barrier; a rebalance rewrites it below */
     for (;;) {
@@ -403,11 +404,7 @@ __device__ __forceinline__ bool colour_pass(const DevWorld& w, int nparts) {
         if (gtid == 0 && P == 0) w.cnt[CNT_PART_P] = 0;
         /* a body's part: its own if the partition holds it, else the part whose rank range its
          * current Morton rank falls in (the block of that part then reads it in global memory) */
-        auto part_of = [&](int b) {
-            const int c = w.b_cidx[b];
-            if (c >= 0 && c < ncache && w.cache_body[c] == b) return w.b_part[b];
-            const int r = w.b_rank[b];
-            if (r >= nf) return -2;
+        auto part_of_rank = [&](int r) {
             int lo = 0, hi = P - 1;
             while (lo < hi) {
                 const int mid = (lo + hi + 1) >> 1;
@@ -415,6 +412,25 @@ __device__ __forceinline__ bool colour_pass(const DevWorld& w, int nparts) {
                 else hi = mid - 1;
             }
             return lo;
+        };
+        auto part_of = [&](int b) {
+            const int c = w.b_cidx[b];
+            if (c >= 0 && c < ncache && w.cache_body[c] == b) return w.b_part[b];
+            const int r = w.b_rank[b];
+            return r >= nf ? -2 : part_of_rank(r);
+        };
+        /* A kinematic body is in no part and joins every body it touches in one island (islands cross all
+         * but static bodies), so interior constraints at it may make an island of several parts without
+         * any boundary constraint. In one world of several parts that is taken for granted; in a batch a
+         * new partition holds a world in the part of the world's first rank, and a body elsewhere shows
+         * that a kept one no longer does. */
+        auto may_span = [&](int dynamic, int part) {
+            if (w.num_worlds <= 1) return true;
+            if (rebalance) return false;
+            const int r = w.b_rank[dynamic];
+            if (r >= nf) return true;
+            const int first = w.bp_world_first[(uint32_t)(w.bp_key[r] >> kKeyMortonBits)];
+            return part_of_rank(first >= 0 && first <= r ? first : r) != part;
         };
         for (int k = gtid; k < n; k += gsize) {
             const int ci = w.cons_contact[k];
@@ -428,7 +444,12 @@ __device__ __forceinline__ bool colour_pass(const DevWorld& w, int nparts) {
                     const int pa = !da ? -1 : part_of(bd.x);
                     const int pb = !db ? -1 : part_of(bd.y);
                     part = !da ? pb : (!db ? pa : (pa == pb ? pa : -1));
-                    if (part < 0 && P > w.num_sms) w.cnt[CNT_PART_SPLIT] = 1;
+                    bool split = part < 0;
+                    if (da != db && part >= 0 && !is_static(w.b_flags[da ? bd.y : bd.x]) && may_span(da ? bd.x : bd.y, part)) {
+                        w.cnt[CNT_ISLAND_SPAN] = 1;
+                        split = true;
+                    }
+                    if (split && P > w.num_sms) w.cnt[CNT_PART_SPLIT] = 1;
                     if (part < 0) part = -1;
                 }
             }
@@ -1020,6 +1041,7 @@ __device__ __forceinline__ void part_load(const PartCtx& pc, const float4* glob)
  * and flags, then the constraint list in contact order (each block counts its chunk of the table, the
  * chunks' counts give each block its offset, and a block scan places the block's constraints). */
 __device__ __forceinline__ void islands_reset(const DevWorld& w, int allow_sleep) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) w.cnt[CNT_ISLAND_SPAN] = 0;  /* for the colouring */
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < w.n_bodies; b += gridDim.x * blockDim.x) {
         w.b_island[b] = b;
         w.isl_minsep[b] = 0xffffffffu;      /* of a root: its island's smallest body */
@@ -1496,13 +1518,15 @@ __device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& 
         __syncthreads();
     }
     const int nbnd = parts ? min(s_boff[ncol], pc.bcap) : 0;
+    const bool span = parts && ncol == 0 && nparts > 1 && w.cnt[CNT_ISLAND_SPAN] != 0;
     for (int it = 0; it < sp.pi; ++it) {
         uint32_t* cur = w.isl_minsep + (size_t)it * w.body_cap;
         if (parts) {
             /* the interior colours, then a barrier: islands span parts, and the next iteration's
-             * early exit reads this iteration's buffer. Without boundary constraints (a batch cut at
-             * world boundaries) no island spans two parts: each part's islands are written by its
-             * own block alone, so the iterations need no grid barrier until the positions go back. */
+             * early exit reads this iteration's buffer. Without boundary constraints only a kinematic
+             * body makes an island of several parts (span). Without either, as in a batch cut at world
+             * boundaries, each part's islands are written by its own block alone, so the iterations need
+             * no grid barrier until the positions go back. */
             if (it > 0) {
                 part_done_flags(w, pc, nbnd, it, tol);
                 __syncthreads();
@@ -1531,6 +1555,8 @@ __device__ __forceinline__ bool solve_pass(const DevWorld& w, const StepParams& 
                 }
             } else if (it == sp.pi - 1) {
                 part_store(pc, w.b_pos);
+                if (!grid_barrier(w)) return false;
+            } else if (span) {
                 if (!grid_barrier(w)) return false;
             }
             continue;
