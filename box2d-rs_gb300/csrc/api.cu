@@ -37,6 +37,7 @@
 
 #include "../../include/b2g.h"
 #include "b2g_internal.h"
+#include "b2g_lists.h"
 #include "b2g_shape.cuh"
 #include "b2g_tape.h"
 
@@ -3210,11 +3211,17 @@ int b2g_get_solver_order(void* p, uint32_t* out, int32_t cap, int32_t* n) {
 
 namespace {
 
+/* what a query's kernels tell the host */
+struct QueryResult {
+    int status, unsorted;               /* the write's flag */
+    unsigned long long total, counter;  /* the find's counter */
+};
+
 /* Device buffers of one query call, pieces of an allocation the world keeps for the next call (it is freed
  * with the world; a call that needed more than kQueryKeep bytes leaves none). The arrays themselves only
  * where the device cannot reach the caller's. */
 struct QueryBuffers {
-    int* result;       /* status, total, the find's counter, the write's flag */
+    QueryResult* result;
     int2* lists;
     uint32_t* found;
     float* query;
@@ -3224,7 +3231,7 @@ struct QueryBuffers {
 constexpr size_t kQueryKeep = 64u << 20;
 
 int query_buffers(World* w, QueryBuffers& b, const float* query, const uint32_t* world, int n, int found, size_t out_bytes) {
-    const size_t size[6] = {4 * sizeof(int), found > 0 ? n * sizeof(int2) : 0, (size_t)found * sizeof(uint32_t),
+    const size_t size[6] = {sizeof(QueryResult), found > 0 ? n * sizeof(int2) : 0, (size_t)found * sizeof(uint32_t),
                             query ? n * 4 * sizeof(float) : 0, world ? n * sizeof(uint32_t) : 0, out_bytes};
     size_t at[6], total = 0;
     for (int k = 0; k < 6; ++k) {
@@ -3244,7 +3251,7 @@ int query_buffers(World* w, QueryBuffers& b, const float* query, const uint32_t*
         w->query_bytes = total;
     }
     unsigned char* m = w->query_mem;
-    b = {(int*)(m + at[0]), (int2*)(m + at[1]), (uint32_t*)(m + at[2]), (float*)(m + at[3]), world ? (uint32_t*)(m + at[4]) : nullptr,
+    b = {(QueryResult*)(m + at[0]), (int2*)(m + at[1]), (uint32_t*)(m + at[2]), (float*)(m + at[3]), world ? (uint32_t*)(m + at[4]) : nullptr,
          m + at[5]};
     if (query) CUDA_OK(w, cudaMemcpyAsync(b.query, query, size[3], cudaMemcpyHostToDevice, w->stream));
     if (world) CUDA_OK(w, cudaMemcpyAsync(b.world, world, size[4], cudaMemcpyHostToDevice, w->stream));
@@ -3286,9 +3293,9 @@ int b2g_ray_cast_closest(void* p, const float* rays, const uint32_t* world_index
     QueryBuffers b;
     int rc = query_buffers(w, b, rays, world_index, n, 0, (size_t)n * sizeof(b2g_ray_hit));
     if (rc != B2G_OK) return rc;
-    launch_ray_cast(w->d, b.query, b.world, n, (b2g_ray_hit*)b.out, b.result, s);
+    launch_ray_cast(w->d, b.query, b.world, n, (b2g_ray_hit*)b.out, &b.result->status, s);
     CUDA_OK(w, cudaGetLastError());
-    CUDA_OK(w, cudaMemcpyAsync(&status, b.result, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CUDA_OK(w, cudaMemcpyAsync(&status, &b.result->status, sizeof(int), cudaMemcpyDeviceToHost, s));
     CUDA_OK(w, cudaStreamSynchronize(s));
     if (!(status & ~ST_STACK_OVERFLOW))
         CUDA_OK(w, cudaMemcpy(out, b.out, (size_t)n * sizeof(b2g_ray_hit), cudaMemcpyDeviceToHost));
@@ -3311,20 +3318,23 @@ int b2g_query_aabb(void* p, const float* boxes, const uint32_t* world_index, int
         QueryBuffers b;
         int rc = query_buffers(w, b, direct ? nullptr : boxes, direct ? nullptr : world_index, n, room, 0);
         if (rc != B2G_OK) return rc;
-        int got[2] = {0, 0};  /* status, total */
-        CUDA_OK(w, cudaMemsetAsync(b.result, 0, 4 * sizeof(int), s));
+        QueryResult got{};
+        CUDA_OK(w, cudaMemsetAsync(b.result, 0, sizeof(QueryResult), s));
         launch_query_find(w->d, direct ? boxes : b.query, direct ? world_index : b.world, n, b.found, room, b.lists,
-                          b.result + 2, direct ? got : b.result, s);
+                          &b.result->counter, direct ? &got.status : &b.result->status,
+                          direct ? &got.total : &b.result->total, s);
         CUDA_OK(w, cudaGetLastError());
-        if (!direct) CUDA_OK(w, cudaMemcpyAsync(got, b.result, sizeof(got), cudaMemcpyDeviceToHost, s));
+        if (!direct) CUDA_OK(w, cudaMemcpyAsync(&got, b.result, sizeof(got), cudaMemcpyDeviceToHost, s));
         CUDA_OK(w, cudaStreamSynchronize(s));
-        const int status = ((volatile int*)got)[0], total = ((volatile int*)got)[1];
+        const int status = ((volatile QueryResult&)got).status;
+        const unsigned long long all = ((volatile QueryResult&)got).total;
         if (status & ~ST_STACK_OVERFLOW) return status_error(w, status);
-        *out_count = total;
-        if (total > capacity) {
+        *out_count = saturated_count(all);
+        if (!within_capacity(all, capacity)) {
             status_error(w, status);
             return fail(w, B2G_ERR_CAPACITY, "more overlaps than capacity; *out_count holds the total");
         }
+        const int total = (int)all;  /* at most capacity */
         if (total > room) {
             room = total;
             continue;
@@ -3340,8 +3350,8 @@ int b2g_query_aabb(void* p, const float* boxes, const uint32_t* world_index, int
         } else if (total > 0) {
             uint32_t* pairs = nullptr;
             CUDA_OK(w, cudaMalloc((void**)&pairs, bytes));
-            launch_query_write(w->d, n, b.found, b.lists, pairs, b.result + 3, s);
-            cudaError_t e = cudaMemcpyAsync(&unsorted, b.result + 3, sizeof(int), cudaMemcpyDeviceToHost, s);
+            launch_query_write(w->d, n, b.found, b.lists, pairs, &b.result->unsorted, s);
+            cudaError_t e = cudaMemcpyAsync(&unsorted, &b.result->unsorted, sizeof(int), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
             if (e == cudaSuccess) e = cudaMemcpy(out_pairs, pairs, bytes, cudaMemcpyDeviceToHost);
             cudaFree(pairs);

@@ -486,13 +486,13 @@ void launch_collide_pairs(const ShapeRec* a, const float4* xa, const ShapeRec* b
                           int n, float4* geo, float4* pts, uint4* ids, cudaStream_t s);
 
 /* World queries on the last step's LBVH (k_query.cu). Every pointer is memory the device reaches; the
- * last kernel of a call writes the world's status word (and the total) to status / status_total. */
+ * last kernel of a call writes the world's status word to *status (and the total to *total_out). */
 void launch_ray_cast(const DevWorld& w, const float* rays, const uint32_t* ray_world, int n, b2g_ray_hit* out, int* status,
                      cudaStream_t s);
 /* found: the boxes' fixtures, box by box in no order, lists[i] = (first entry, entries) of box i; written only
  * while they fit cap. *total (zero before) counts all */
 void launch_query_find(const DevWorld& w, const float* boxes, const uint32_t* box_world, int n, uint32_t* found, int cap,
-                       int2* lists, int* total, int* status_total, cudaStream_t s);
+                       int2* lists, unsigned long long* total, int* status, unsigned long long* total_out, cudaStream_t s);
 /* out: (box, fixture) pairs sorted by box then fixture, but for lists of more than 1024 fixtures, which
  * are left as found (*unsorted is then set) */
 void launch_query_write(const DevWorld& w, int n, const uint32_t* found, const int2* lists, uint32_t* out, int* unsorted,

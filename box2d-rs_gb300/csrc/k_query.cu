@@ -18,6 +18,7 @@
 #include <climits>
 
 #include "b2g_internal.h"
+#include "b2g_lists.h"
 #include "b2g_walk.cuh"
 
 namespace b2g {
@@ -195,13 +196,14 @@ __global__ void __launch_bounds__(kBlock) k_ray_cast(DevWorld w, const float* ra
  * for its box (up to 32 pending nodes a round, from a stack in shared memory) and keeps what it finds in shared
  * memory; the box's list then goes to a piece of `found` that it reserves with one atomic (a longer list
  * than fits is written by a second walk). lists[i] = (first entry, entries); *total counts all of them,
- * written or not. k_query_write: the lists in the order of the boxes, each by fixture. */
+ * written or not, in 64 bits: boxes over a whole world of 250k fixtures pass 31 bits at 8600 of them. k_query_write: the lists in the order of the boxes, each by fixture. */
 constexpr int kBoxWarps = 4;
 constexpr int kFoundMax = 256;   /* a box's fixtures kept in shared memory */
 constexpr int kRankMax = 1024;   /* longer lists are left to the host to sort */
 
 __global__ void __launch_bounds__(32 * kBoxWarps) k_query_find(DevWorld w, const float* boxes, const uint32_t* box_world,
-                                                               int n, uint32_t* found, int cap, int2* lists, int* total) {
+                                                               int n, uint32_t* found, int cap, int2* lists,
+                                                               unsigned long long* total) {
     if (((volatile int*)w.cnt)[CNT_STATUS] & ~ST_STACK_OVERFLOW) return;
     __shared__ int s_pend[kBoxWarps][kPendMax];
     __shared__ uint32_t s_found[kBoxWarps][kFoundMax];
@@ -221,13 +223,12 @@ __global__ void __launch_bounds__(32 * kBoxWarps) k_query_find(DevWorld w, const
                 count += __popc(who);
             });
         __syncwarp();
-        int first = 0;
-        if (lane == 0) {
-            first = count > 0 ? atomicAdd(total, count) : 0;
-            lists[i] = make_int2(first, count);
-        }
-        first = __shfl_sync(0xffffffffu, first, 0);
-        if (first > cap - count) continue;  /* the caller learns the total and asks again with room for it */
+        unsigned long long place = 0;
+        if (lane == 0 && count > 0) place = atomicAdd(total, (unsigned long long)count);
+        place = __shfl_sync(0xffffffffu, place, 0);
+        if (!list_fits(place, count, cap)) continue;  /* the caller learns the total and asks again with room for it */
+        const int first = (int)place;
+        if (lane == 0) lists[i] = make_int2(first, count);
         if (count <= kFoundMax) {
             for (int k = lane; k < count; k += 32) found[first + k] = s_found[wid][k];
         } else {
@@ -282,9 +283,9 @@ __global__ void __launch_bounds__(256) k_query_write(int n, const uint32_t* foun
 }
 
 /* the status word, and a count if there is one, where the host reads them */
-__global__ void k_query_end(DevWorld w, const int* total, int* out) {
-    out[0] = ((volatile int*)w.cnt)[CNT_STATUS];
-    if (total) out[1] = *total;
+__global__ void k_query_end(DevWorld w, const unsigned long long* total, int* status, unsigned long long* total_out) {
+    *status = ((volatile int*)w.cnt)[CNT_STATUS];
+    if (total) *total_out = *total;
 }
 
 }  // namespace
@@ -293,15 +294,15 @@ void launch_ray_cast(const DevWorld& w, const float* rays, const uint32_t* ray_w
                      cudaStream_t s) {
     const int per = lanes_for(n, w.num_sms);
     k_ray_cast<<<grid_for(n, kBlock / 32 * per, w.num_sms * 16), kBlock, 0, s>>>(w, rays, ray_world, n, per, out);
-    k_query_end<<<1, 1, 0, s>>>(w, nullptr, status);
+    k_query_end<<<1, 1, 0, s>>>(w, nullptr, status, nullptr);
     B2G_LAUNCHED(2);
 }
 
 void launch_query_find(const DevWorld& w, const float* boxes, const uint32_t* box_world, int n, uint32_t* found, int cap,
-                       int2* lists, int* total, int* status_total, cudaStream_t s) {
+                       int2* lists, unsigned long long* total, int* status, unsigned long long* total_out, cudaStream_t s) {
     k_query_find<<<grid_for(n, kBoxWarps, w.num_sms * 16), 32 * kBoxWarps, 0, s>>>(w, boxes, box_world, n, found, cap,
                                                                                   lists, total);
-    k_query_end<<<1, 1, 0, s>>>(w, total, status_total);
+    k_query_end<<<1, 1, 0, s>>>(w, total, status, total_out);
     B2G_LAUNCHED(2);
 }
 

@@ -577,8 +577,8 @@ typedef struct b2g_ray_hit {
 int b2g_ray_cast_closest(void* world, const float* rays, const uint32_t* world_index, int32_t n, b2g_ray_hit* out);
 /* Fixtures whose fat AABB overlaps each box (boxes: n x (lower.x, lower.y, upper.x, upper.y)), as
  * (box index, fixture) pairs sorted by box then fixture (the reference reports the same set per
- * box through its query callback, in tree order). *out_count = total pairs; at most capacity are
- * written (B2G_ERR_CAPACITY if more exist). */
+ * box through its query callback, in tree order). *out_count = total pairs (INT32_MAX if there are more
+ * than that); at most capacity are written (B2G_ERR_CAPACITY if more exist). */
 int b2g_query_aabb(void* world, const float* boxes, const uint32_t* world_index, int32_t n, uint32_t* out_pairs,
                    int32_t capacity, int32_t* out_count);
 
