@@ -26,6 +26,7 @@
 
 #include "b2g.h"
 #include "b2g_collide.cuh"
+#include "b2g_launch.h"
 
 namespace b2g {
 
@@ -431,6 +432,33 @@ inline int launch_cluster(void (*kernel)(KArgs...), int grid, int blocks, int th
     return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+inline int current_device() {
+    int dev = -1;
+    return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
+}
+
+/* Lets a kernel run as clusters of up to kClusterMaxBlocks blocks on the current device, and says whether one
+ * of `blocks` blocks fits it: 16 blocks need as many free SMs in one GPC. */
+template <typename... KArgs>
+inline bool cluster_fits(void (*kernel)(KArgs...), int blocks, int threads, size_t smem) {
+    cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (smem > 0) cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    const bool fits = cudaOccupancyMaxActiveClusters(&n, (const void*)kernel, &cfg) == cudaSuccess && n > 0;
+    if (!fits) cudaGetLastError();
+    return fits;
+}
+
 /* kernel-file launchers */
 /* may_sleep: some body may be asleep (sleeping allowed, or a body made asleep): contacts then see
  * the bodies woken by contacts before them in the table's key order, as in the reference's list */
@@ -453,13 +481,14 @@ void launch_islands_and_constraints(const DevWorld& w, const StepParams& sp, cud
  * colouring and solver, and of a taped step's recording (tape), as one kernel on one thread-block cluster, and the whole
  * broadphase and contact merge as another (launch_back): cluster_world says whether a world does, given
  * the device's largest cluster. */
-constexpr int kClusterMaxBlocks = 16;
 constexpr int kClusterMaxProxies = kClusterMaxBlocks * 256;
 bool cluster_world(const DevWorld& w);
 int cluster_size(const DevWorld& w);
 struct TapeDev;
 int launch_front(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool parts, const TapeDev* tape);
 int launch_back(const DevWorld& w, const StepParams& sp, cudaStream_t s);
+/* whether launch_back's kernel fits the current device as one cluster of that many blocks (and may be launched so) */
+bool back_cluster_fits(int blocks);
 /* a stamp on its own (a step that ends with a phase no kernel follows) */
 void launch_phase_stamp(const DevWorld& w, int phase, cudaStream_t s);
 /* parts: allow the part-local solve (used where the world's size suits it) */

@@ -622,10 +622,11 @@ static int adjoint_blocks(int max_slots, int parts, int num_sms, bool* cluster) 
     if (*cluster) {
         int c = 1;
         while (c < kClusterMaxBlocks && (c < parts || 512 * c < max_slots)) c <<= 1;
-        static const bool big = cudaFuncSetAttribute((const void*)k_adj_replay, cudaFuncAttributeNonPortableClusterSizeAllowed,
-                                                     1) == cudaSuccess &&
-                                cudaFuncSetAttribute((const void*)k_adj_reverse, cudaFuncAttributeNonPortableClusterSizeAllowed,
-                                                     1) == cudaSuccess;
+        static PerDevice<bool> allowed;
+        const bool big = allowed.at(current_device(), [] {
+            return cudaFuncSetAttribute((const void*)k_adj_replay, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                   cudaFuncSetAttribute((const void*)k_adj_reverse, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        });
         if (c <= 8 || big) return c;
         *cluster = false;
     }

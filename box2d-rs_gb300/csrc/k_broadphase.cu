@@ -1018,10 +1018,9 @@ void launch_touch_all_proxies(const DevWorld& w, cudaStream_t s) {
     B2G_LAUNCHED(1);
 }
 
+bool back_cluster_fits(int blocks) { return cluster_fits(k_back, blocks, kBlock, 0); }
+
 int launch_back(const DevWorld& w, const StepParams& sp, cudaStream_t s) {
-    static const cudaError_t allowed =
-        cudaFuncSetAttribute((const void*)k_back, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    (void)allowed;
     B2G_LAUNCHED(1);
     return launch_cluster(k_back, cluster_size(w), cluster_size(w), kBlock, 0, s, w, sp);
 }

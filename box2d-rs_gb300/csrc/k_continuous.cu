@@ -879,13 +879,12 @@ __global__ void __launch_bounds__(kTBlock) k_continuous(DevWorld w, StepParams s
 }  // namespace
 
 int launch_continuous(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms) {
-    static bool configured = false;
+    static PerDevice<bool> shared_memory;
     /* the islands' scratch, and after them the walks' pending nodes */
     constexpr int smem = max_of(kIslWarps * (int)sizeof(IslandScratch), kTBlock / 32 * kPendMax * (int)sizeof(int));
-    if (!configured) {
-        cudaFuncSetAttribute((const void*)k_continuous, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        configured = true;
-    }
+    shared_memory.at(current_device(), [] {
+        return cudaFuncSetAttribute((const void*)k_continuous, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+    });
     DevWorld wc = w;
     StepParams p = sp;
     void* args[] = {&wc, &p};

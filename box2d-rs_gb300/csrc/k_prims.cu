@@ -283,13 +283,7 @@ void scan_exclusive_u32(const uint32_t* in, uint32_t* out, const int* d_n, int m
 void radix_sort_pairs_coop(unsigned long long* key_a, uint32_t* val_a, unsigned long long* key_b, uint32_t* val_b,
                            const int* d_n, int max_n, int bits, uint32_t* hist, int* cnt, cudaStream_t s, int num_sms,
                            int barrier_word, bool zero_or_max) {
-    static int per_sm = 0;
-    if (!per_sm) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_radix_coop, kSortBlock, 0);
-        if (per_sm < 1) per_sm = 1;
-        if (per_sm > 2) per_sm = 2;
-    }
-    /* one block per SM keeps the grid barrier short; per_sm only guards co-residency */
+    /* one block per SM keeps the grid barrier short */
     const int blocks = num_sms;
     if (max_n > kSortTile && (!zero_or_max || max_n <= kRankSort)) {
         /* the rank count for inputs between one tile and kRankSort keys (each kernel checks n) */

@@ -31,8 +31,6 @@
  * gives bit-identical bodies, because each operation is the same IEEE f32 operation.
  */
 #include <algorithm>
-#include <mutex>
-#include <vector>
 
 #include "b2g_internal.h"
 #include "b2g_joint.cuh"
@@ -1911,11 +1909,12 @@ bool use_parts(const DevWorld& w, int num_sms, bool allowed) {
 void launch_colouring(const DevWorld& w, cudaStream_t s, int num_sms, bool parts, bool taped) {
     /* more blocks per SM for large worlds: the colouring's passes stride over every
      * constraint and body */
-    static int resident = 0;
-    if (!resident) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, (const void*)k_colour, kBlock, 0);
-        resident = std::max(1, std::min(resident, 8));
-    }
+    static PerDevice<int> blocks_per_sm;
+    const int resident = blocks_per_sm.at(current_device(), [] {
+        int n = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, (const void*)k_colour, kBlock, 0);
+        return std::max(1, std::min(n, 8));
+    });
     const int per_sm = std::max(w.cfg_coop_per_sm, std::min(resident, w.n_bodies / 65536));
     const int blocks = coop_blocks((const void*)k_colour, num_sms) * per_sm;
     DevWorld wc = w;
@@ -1956,13 +1955,13 @@ static bool wide_solver(const DevWorld& w, int num_sms) {
 }
 
 int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms, bool parts, bool taped) {
-    static bool attr_set = false;
-    if (!attr_set) {
+    static PerDevice<bool> shared_memory;
+    shared_memory.at(current_device(), [] {
         cudaFuncSetAttribute((const void*)k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kPartSmemOne);
         cudaFuncSetAttribute((const void*)k_batch_velocities, cudaFuncAttributeMaxDynamicSharedMemorySize, kBatchSmem);
         cudaFuncSetAttribute((const void*)k_batch_positions, cudaFuncAttributeMaxDynamicSharedMemorySize, kBatchSmem);
-        attr_set = true;
-    }
+        return true;
+    });
     const int blocks = coop_blocks((const void*)k_solve, num_sms) * w.cfg_coop_per_sm;
     DevWorld wc = w;
     StepParams spc = sp;
@@ -1994,36 +1993,14 @@ int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int n
     return rc;
 }
 
-/* The largest cluster k_front and k_back can run as on the current device (0: none), found once per
- * device: 16 blocks need the non-portable size and as many free SMs in one GPC. */
+/* the largest cluster that k_front and k_back can both run as on the current device (0: none) */
 static int max_cluster() {
-    static std::mutex m;
-    static std::vector<int> found;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 0;
-    std::lock_guard<std::mutex> lock(m);
-    if ((int)found.size() <= dev) found.resize((size_t)dev + 1, -1);
-    if (found[dev] >= 0) return found[dev];
-    int best = 0;
-    cudaFuncSetAttribute((const void*)k_front, cudaFuncAttributeMaxDynamicSharedMemorySize, kPartSmemOne);
-    cudaFuncSetAttribute((const void*)k_front, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    for (int c = kClusterMaxBlocks; c >= 1 && best == 0; c >>= 1) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(c);
-        cfg.blockDim = dim3(kBlock);
-        cfg.dynamicSmemBytes = kPartSmemOne;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = c;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, (const void*)k_front, &cfg) == cudaSuccess && n > 0) best = c;
-        else cudaGetLastError();
-    }
-    found[dev] = best;
-    return best;
+    static PerDevice<int> largest;
+    const int dev = current_device();
+    if (dev < 0) return 0;
+    return largest.at(dev, [] {
+        return largest_cluster([](int c) { return cluster_fits(k_front, c, kBlock, kPartSmemOne) && back_cluster_fits(c); });
+    });
 }
 
 /* One block of 256 threads for each 128 proxies, a power of two up to 16: at least as many blocks as the
