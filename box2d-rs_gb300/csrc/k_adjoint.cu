@@ -611,45 +611,30 @@ void launch_tape_snapshot(const DevWorld& w, const TapeDev& t, int index, cudaSt
     B2G_LAUNCHED(1);
 }
 
-/* How a backward pass is launched, from the slots of its largest step and the parts of its solves: on
- * clusters of up to 16 blocks (one block for a small world) where a step fits 512 slots a block, else on a
- * cooperative grid of a block for each part or 256 slots. (One block for up to 4096 slots took 110 ms for
- * 128 steps of 10 throw-and-stack worlds, whose 1000 slots in two parts it swept one after the other; the
- * cluster of two takes 31. 128 steps of one world: 34.7 -> 18.5 ms, 64 steps of 512 worlds: 42.7 -> 28 ms,
- * replays side by side and local memory gone.) */
-static int adjoint_blocks(int max_slots, int parts, int num_sms, bool* cluster) {
-    *cluster = max_slots <= 512 * kClusterMaxBlocks && parts <= kClusterMaxBlocks;
-    if (*cluster) {
-        int c = 1;
-        while (c < kClusterMaxBlocks && (c < parts || 512 * c < max_slots)) c <<= 1;
-        static PerDevice<bool> allowed;
-        const bool big = allowed.at(current_device(), [] {
-            return cudaFuncSetAttribute((const void*)k_adj_replay, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                   cudaFuncSetAttribute((const void*)k_adj_reverse, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-        });
-        if (c <= 8 || big) return c;
-        *cluster = false;
-    }
-    return std::max(1, std::min(num_sms, std::max(parts, (max_slots + kBlock - 1) / kBlock)));
+static AdjointBlocks device_adjoint_blocks(int max_slots, int parts, int num_sms) {
+    static PerDevice<int> largest;
+    const int most = largest.at(current_device(), [] {
+        return largest_cluster([](int c) { return cluster_fits(k_adj_replay, c, kBlock, 0) && cluster_fits(k_adj_reverse, c, kBlock, 0); });
+    });
+    return adjoint_blocks(max_slots, parts, num_sms, most);
 }
 
 /* Segments whose replays can run side by side: any number on clusters, and what is co-resident of a
  * cooperative grid. */
 int adjoint_groups(int max_slots, int parts, int num_sms) {
-    bool cluster;
-    const int blocks = adjoint_blocks(max_slots, parts, num_sms, &cluster);
-    if (cluster) return 1 << 20;
+    const AdjointBlocks on = device_adjoint_blocks(max_slots, parts, num_sms);
+    if (on.cluster) return 1 << 20;
     int per_sm = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_adj_replay, kBlock, 0);
-    return std::max(1, per_sm * num_sms / blocks);
+    return std::max(1, per_sm * num_sms / on.blocks);
 }
 
 int launch_adjoint_replay(const AdjWork& a, int segments, int parts, cudaStream_t s, int num_sms) {
     AdjWork ac = a;
-    bool cluster;
-    int blocks = adjoint_blocks(a.max_slots, parts, num_sms, &cluster);
+    const AdjointBlocks on = device_adjoint_blocks(a.max_slots, parts, num_sms);
+    int blocks = on.blocks;
     B2G_LAUNCHED(1);
-    if (cluster) return launch_cluster(k_adj_replay, blocks * segments, blocks, kBlock, 0, s, ac, blocks);
+    if (on.cluster) return launch_cluster(k_adj_replay, blocks * segments, blocks, kBlock, 0, s, ac, blocks);
     const cudaError_t e = cudaMemsetAsync(a.cnt, 0, (size_t)segments * CNT_SIZE * sizeof(int), s);
     if (e != cudaSuccess) return (int)e;
     void* args[] = {&ac, &blocks};
@@ -658,10 +643,10 @@ int launch_adjoint_replay(const AdjWork& a, int segments, int parts, cudaStream_
 
 int launch_adjoint_reverse(const AdjWork& a, int segment, int parts, cudaStream_t s, int num_sms) {
     AdjWork ac = a;
-    bool cluster;
-    const int blocks = adjoint_blocks(a.max_slots, parts, num_sms, &cluster);
+    const AdjointBlocks on = device_adjoint_blocks(a.max_slots, parts, num_sms);
+    const int blocks = on.blocks;
     B2G_LAUNCHED(1);
-    if (cluster) return launch_cluster(k_adj_reverse, blocks, blocks, kBlock, 0, s, ac, segment);
+    if (on.cluster) return launch_cluster(k_adj_reverse, blocks, blocks, kBlock, 0, s, ac, segment);
     int* bar = a.cnt + (size_t)(segment - a.first_seg) * CNT_SIZE + CNT_BARRIER;
     const cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(int), s);
     if (e != cudaSuccess) return (int)e;
