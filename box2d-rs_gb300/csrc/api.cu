@@ -86,7 +86,8 @@ struct TapeHost {
     AdjWork work{};
     std::vector<void*> work_mem;
     size_t work_bytes = 0;
-    int work_slots = 0, work_vi = 0, work_pi = 0, work_groups = 0;
+    WorkSizes work_for;
+    int work_groups = 0;
     unsigned mismatches = 0;
 };
 
@@ -238,7 +239,8 @@ void tape_free_work(TapeHost* t) {
     for (void* p : t->work_mem) cudaFree(p);
     t->work_mem.clear();
     t->work_bytes = 0;
-    t->work_slots = t->work_vi = t->work_pi = t->work_groups = 0;
+    t->work_for = WorkSizes{};
+    t->work_groups = 0;
 }
 
 void tape_free(World* w) {
@@ -3556,32 +3558,32 @@ int tape_status(World* w, TapeHost* t, long long* steps, long long* slots) {
     return B2G_OK;
 }
 
-/* Work buffers for segments of ckpt_every steps with up to `slots` constraints, `groups` of them replayed
- * side by side, fewer where they would take more than kReplayBytes or the memory is not there. */
-constexpr size_t kReplayBytes = (size_t)8 << 30;
-
-int tape_work(World* w, TapeHost* t, int slots, int vi, int pi, int groups) {
+/* Work buffers for segments of ckpt_every steps with up to `slots` constraints, `wanted` of them replayed
+ * side by side if the memory is there (replay_groups, allocate_groups). */
+int tape_work(World* w, TapeHost* t, int slots, int vi, int pi, int wanted) {
     if (slots < 1) slots = 1;
     if (vi < 1) vi = 1;
     if (pi < 1) pi = 1;
+    if (wanted < 1) wanted = 1;
+    if (t->work_for.serve(slots, vi, pi, wanted)) return B2G_OK;
+    tape_free_work(t);
     const size_t nb = (size_t)t->n_bodies, seg = (size_t)t->ckpt_every, ns = (size_t)slots;
     const size_t each = sizeof(float4) * (nb * (2 + 3 * seg) + ns * (1 + seg * (3 * (size_t)vi + 2 + 2 * (size_t)pi))) +
                         ns * sizeof(adj::VC<float>);
-    groups = std::max(1, (int)std::min<size_t>((size_t)groups, kReplayBytes / std::max<size_t>(each, 1)));
-    if (!t->work_mem.empty() && slots <= t->work_slots && vi <= t->work_vi && pi <= t->work_pi && groups <= t->work_groups)
-        return B2G_OK;
+    size_t free_bytes = 0, device_bytes = 0;
+    CUDA_OK(w, cudaMemGetInfo(&free_bytes, &device_bytes));
     AdjWork& a = t->work;
     int rc = B2G_OK;
-    for (;; groups = (groups + 1) / 2) {
+    const int groups = allocate_groups(replay_groups(wanted, each, free_bytes), [&](int n) {
         tape_free_work(t);
         a = AdjWork{};
         std::vector<void*>& m = t->work_mem;
         size_t& by = t->work_bytes;
         rc = B2G_OK;
-        auto A = [&](auto** ptr, size_t n) {
-            if (rc == B2G_OK) rc = talloc(w, m, by, ptr, n);
+        auto A = [&](auto** ptr, size_t count) {
+            if (rc == B2G_OK) rc = talloc(w, m, by, ptr, count);
         };
-        const size_t g = (size_t)groups;
+        const size_t g = (size_t)n;
         A(&a.cur_pos, g * nb);
         A(&a.cur_vel, g * nb);
         A(&a.ws_pos, g * seg * nb);
@@ -3600,17 +3602,18 @@ int tape_work(World* w, TapeHost* t, int slots, int vi, int pi, int groups) {
         A(&a.g_end[1], ns);
         A(&a.cnt, g * CNT_SIZE);
         A(&a.mismatch, (size_t)1);
-        if (rc == B2G_OK || groups == 1) break;
-        cudaGetLastError();
-    }
-    if (rc != B2G_OK) {
+        if (rc != B2G_OK) cudaGetLastError();
+        return rc == B2G_OK;
+    });
+    if (groups == 0) {
         tape_free_work(t);
         return rc;
     }
     t->work_groups = groups;
-    t->work_slots = slots;
-    t->work_vi = vi;
-    t->work_pi = pi;
+    t->work_for.slots = slots;
+    t->work_for.vi = vi;
+    t->work_for.pi = pi;
+    t->work_for.wanted = wanted;
     a.max_slots = slots;
     a.max_vi = vi;
     a.max_pi = pi;

@@ -1,11 +1,12 @@
 /*
  * b2g_launch.h — host-side choices about launches that need no CUDA call, so that they can be tested without a
- * GPU: values found once for each device, the largest cluster that fits, the backward pass's blocks.
+ * GPU: values found once for each device, the largest cluster that fits, the backward pass's blocks and buffers.
  */
 #ifndef B2G_LAUNCH_H
 #define B2G_LAUNCH_H
 
 #include <algorithm>
+#include <cstddef>
 #include <map>
 #include <mutex>
 
@@ -57,6 +58,32 @@ inline AdjointBlocks adjoint_blocks(int max_slots, int parts, int num_sms, int l
     }
     return {std::max(1, std::min(num_sms, std::max(parts, (max_slots + 255) / 256))), false};
 }
+
+/* Segments of a backward pass whose replays get buffers side by side, `each` bytes a segment: as many as are
+ * wanted, but beyond the one it cannot do without no more than kReplayBytes and a quarter of the free memory
+ * take. 512 worlds over 240 steps hold 15 segments in 1.9 GB more than one segment's. */
+constexpr size_t kReplayBytes = (size_t)8 << 30;
+inline int replay_groups(int wanted, size_t each, size_t free_bytes) {
+    const size_t room = std::min(kReplayBytes, free_bytes / 4) / std::max<size_t>(each, 1);
+    return 1 + (int)std::min<size_t>((size_t)std::max(wanted - 1, 0), room);
+}
+
+/* fewer, down to one, while allocate(groups) fails; 0: not even one */
+template <class Allocate>
+int allocate_groups(int groups, Allocate&& allocate) {
+    for (;; groups = (groups + 1) / 2) {
+        if (allocate(groups)) return groups;
+        if (groups <= 1) return 0;
+    }
+}
+
+/* What a backward pass's buffers were allocated for. They serve every call that asks for no more, also where
+ * they hold fewer groups than were wanted: the memory was not there, and asking for it again on every call
+ * would free and allocate all of them on every call. */
+struct WorkSizes {
+    int slots = 0, vi = 0, pi = 0, wanted = 0;
+    bool serve(int s, int v, int p, int w) const { return wanted > 0 && s <= slots && v <= vi && p <= pi && w <= wanted; }
+};
 
 }  // namespace b2g
 

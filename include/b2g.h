@@ -539,7 +539,12 @@ typedef struct b2g_tape_info {
  * picks max_steps x (4 x fixtures + 1024)); body state is checkpointed every
  * checkpoint_interval steps (<= 0: 16). Needs sleeping off. Editing bodies between taped steps
  * (transforms, velocities, forces, impulses, new bodies or fixtures) invalidates the tape and
- * b2g_backward then fails; gravity, iterations, dt and warm starting may change per step. */
+ * b2g_backward then fails; gravity, iterations, dt and warm starting may change per step.
+ * b2g_backward adds work buffers for the replay of one checkpoint segment and, so that segments are
+ * replayed side by side, for as many others as the tape has, at most 8 GiB and a quarter of the free
+ * device memory (fewer if an allocation fails). They stay with the tape (b2g_tape_info.device_bytes), as
+ * both do for the next tape of the same max_steps, interval, max_slots, bodies and contact capacity; any
+ * other tape and the world's end free them. */
 int b2g_tape_begin(void* world, int32_t max_steps, int32_t checkpoint_interval, int64_t max_slots);
 /* Stop recording and checkpoint the final state. */
 int b2g_tape_end(void* world);

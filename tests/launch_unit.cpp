@@ -62,6 +62,29 @@ int main() {
     check(adjoint_blocks(5000, 1, 152, 16).cluster && adjoint_blocks(5000, 1, 152, 16).blocks == 16, "5000 slots on 16 blocks");
     check(!adjoint_blocks(5000, 1, 152, 8).cluster && adjoint_blocks(5000, 1, 152, 8).blocks == 20, "5000 slots where 16 do not fit");
     check(adjoint_blocks(4000, 1, 152, 8).cluster && adjoint_blocks(4000, 1, 152, 8).blocks == 8, "4000 slots on 8 blocks");
+    /* replay buffers: what is wanted where there is room, never past the limits, one at the least */
+    const size_t mb = (size_t)1 << 20, gb = (size_t)1 << 30;
+    check(replay_groups(15, 136 * mb, 200 * gb) == 15, "all segments of 512 worlds over 240 steps");
+    check(replay_groups(15, 136 * mb, 0) == 1 && replay_groups(1, 100 * gb, 0) == 1, "one segment whatever is free");
+    check(replay_groups(15, 136 * mb, 4 * gb) == 1 + 1024 / 136, "a quarter of the free memory");
+    check(replay_groups(1 << 20, 1 * gb, 280 * gb) == 1 + 8, "8 GiB");
+    check(replay_groups(1 << 20, 0, 280 * gb) == 1 << 20 && replay_groups(0, mb, gb) == 1, "sizes of nothing");
+    /* an allocator with a small limit: halved until it fits, not even one, and what was wanted is not asked again */
+    for (int limit : {0, 1, 2, 3, 7, 15, 100}) {
+        int calls = 0, last = 0;
+        const int got = allocate_groups(15, [&](int n) {
+            ++calls;
+            last = n;
+            return n <= limit;
+        });
+        check(got <= limit && got == (limit >= 15 ? 15 : limit >= 8 ? 8 : limit >= 4 ? 4 : limit >= 2 ? 2 : limit), "groups that fit");
+        check(got == 0 ? last == 1 && calls == 5 : last == got, "the last attempt is the one kept");
+    }
+    WorkSizes held;
+    check(!held.serve(1, 1, 1, 1), "nothing held serves nothing");
+    held.slots = 100, held.vi = 8, held.pi = 3, held.wanted = 15;
+    check(held.serve(100, 8, 3, 15) && held.serve(1, 1, 1, 1), "buffers of fewer groups than wanted serve the same call");
+    check(!held.serve(101, 8, 3, 15) && !held.serve(100, 9, 3, 15) && !held.serve(100, 8, 4, 15) && !held.serve(100, 8, 3, 16), "larger calls");
     std::printf("%d wrong\n", failures);
     return failures != 0;
 }
