@@ -63,7 +63,8 @@ struct GraphSlot {
 /* launch configuration: the user's (b2g_set_launch_config), else the autotuner's choice for the
  * world's size bucket if one was made in this process, else the defaults */
 struct LaunchCfg {
-    int coop_per_sm = 1, collide_block = 128, traverse_block = 256, solver_block = 256, collide_group = kCollideGroup;
+    int coop_per_sm = 1, collide_block = 128, traverse_block = 256, solver_block = 0 /* by the world's size */,
+        collide_group = kCollideGroup;
 };
 
 std::mutex g_tune_mutex;
@@ -211,21 +212,16 @@ int mixed_shapes(const World* w) {
 }
 
 void apply_launch_config(World* w) {
-    bool chosen = w->cfg_set;
     if (!w->cfg_set) {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         const int b = size_bucket(w);
         for (auto& e : g_tuned)
-            if (e.first == b) {
-                w->cfg = e.second;
-                chosen = true;
-            }
+            if (e.first == b) w->cfg = e.second;
     }
     w->d.cfg_coop_per_sm = w->cfg.coop_per_sm;
     w->d.cfg_collide_block = w->cfg.collide_block;
     w->d.cfg_traverse_block = w->cfg.traverse_block;
     w->d.cfg_solver_block = w->cfg.coop_per_sm == 1 ? w->cfg.solver_block : 256;
-    w->d.cfg_solver_auto = chosen ? 0 : 1;
     w->d.cfg_collide_group = w->cfg.collide_group;
 }
 
@@ -3382,7 +3378,8 @@ int b2g_get_launch_config(void* p, b2g_launch_config* out) {
     out->collide_block = w->cfg.collide_block;
     out->traverse_block = w->cfg.traverse_block;
     out->tuning_steps = w->tuning_steps;
-    out->solver_block = w->cfg.solver_block;
+    /* by size: the threads that the world's solver runs with */
+    out->solver_block = w->cfg.solver_block ? w->cfg.solver_block : solver_threads(w->d, w->num_sms, w->part_solve, false);
     out->collide_group = w->cfg.collide_group;
     return B2G_OK;
 }
@@ -3391,11 +3388,11 @@ int b2g_set_launch_config(void* p, const b2g_launch_config* c) {
     World* w = W(p);
     if (!w || !c) return B2G_ERR_INVALID_ARG;
     auto pow2 = [](int v, int lo, int hi) { return v >= lo && v <= hi && (v & (v - 1)) == 0; };
-    const int sb = c->solver_block == 0 ? 256 : c->solver_block;
+    const int sb = c->solver_block;
     if (c->coop_blocks_per_sm < 1 || c->coop_blocks_per_sm > 2 || !pow2(c->collide_block, 32, 256) ||
-        !pow2(c->traverse_block, 32, 256) || (sb != 256 && sb != 512) || c->collide_group < 0 || c->collide_group > 32)
+        !pow2(c->traverse_block, 32, 256) || (sb != 0 && sb != 256 && sb != 512) || c->collide_group < 0 || c->collide_group > 32)
         return fail(w, B2G_ERR_INVALID_ARG,
-                    "coop_blocks_per_sm in {1, 2}; block sizes powers of two in [32, 256]; solver_block 256 or 512; "
+                    "coop_blocks_per_sm in {1, 2}; block sizes powers of two in [32, 256]; solver_block 0, 256 or 512; "
                     "collide_group in [0, 32]");
     w->cfg.coop_per_sm = c->coop_blocks_per_sm;
     w->cfg.collide_block = c->collide_block;
@@ -3439,6 +3436,7 @@ extern "C" {
  * contact-buffer parities) and its share of `steps_per_candidate` timed steps; the fastest in
  * total is kept. With the part-local solve the
  * persistent kernels keep one block per SM.
+ * Knobs that nothing in the world's step reads keep their values and take no steps.
  * The steps are real steps of the world (the configuration never changes results). The choice is
  * applied to the world and remembered for later worlds of the same size bucket in this process. */
 int b2g_autotune(void* p, float dt, int32_t vi, int32_t pi, int32_t steps_per_candidate, b2g_launch_config* out) {
@@ -3448,10 +3446,14 @@ int b2g_autotune(void* p, float dt, int32_t vi, int32_t pi, int32_t steps_per_ca
     if (w->h_flags.empty()) return fail(w, B2G_ERR_INVALID_ARG, "the world has no bodies");
     LaunchCfg best = w->cfg;
     w->cfg_set = true;
+    if (int rc = prepare(w); rc != B2G_OK) return rc;  /* which knobs are read depends on the uploaded world */
     const int coop[] = {1, 2}, collide[] = {64, 128, 256}, traverse[] = {64, 128, 256}, solver[] = {256, 512},
               group[] = {0, 8, 32};
     /* the part-local solve caches a part in its block's shared memory: one block per SM */
     const int ncoop = use_parts(w->d, w->num_sms, w->part_solve) ? 1 : 2;
+    /* a step of a small world on one cluster, or a large batch's solver, does not read every knob */
+    const bool read[] = {reads_solver_config(w->d, w->num_sms, w->part_solve), true, !cluster_world(w->d) || w->filter_fn != nullptr,
+                         reads_solver_config(w->d, w->num_sms, w->part_solve), true};
     /* the world keeps evolving while candidates are timed, so the candidates take turns over
      * several rounds (a step each) instead of running one after another */
     const int rounds = std::max(1, std::min(steps_per_candidate / 2, 4));
@@ -3462,6 +3464,7 @@ int b2g_autotune(void* p, float dt, int32_t vi, int32_t pi, int32_t steps_per_ca
                : knob == 3 ? c.solver_block : c.collide_group;
     };
     for (int knob = 0; knob < 5; ++knob) {
+        if (!read[knob]) continue;
         const int* cand = knob == 0 ? coop : knob == 1 ? collide : knob == 2 ? traverse : knob == 3 ? solver : group;
         /* 512 solver threads only with one block per SM (the registers of two would not fit) */
         const int nc = knob == 0 ? ncoop : knob == 3 ? (best.coop_per_sm == 1 ? 2 : 1) : 3;

@@ -199,8 +199,8 @@ struct DevWorld {
     int cfg_coop_per_sm;      /* blocks per SM of the cooperative colouring and solver kernels */
     int cfg_collide_block;    /* threads per block of the narrowphase */
     int cfg_traverse_block;   /* threads per block of the broadphase traversal */
-    int cfg_solver_block;     /* threads per block of the persistent solver (256, or 512 at one block per SM) */
-    int cfg_solver_auto;      /* nobody chose it: by the world's size */
+    int cfg_solver_block;     /* threads per block of the persistent solver (256, or 512 at one block per SM; 0: by
+                                 the world's size) */
     int mixed_shapes;         /* circles and polygons are both a good share of the fixtures */
     int cfg_collide_group;    /* narrowphase: a warp batch with at most this many polygon pairs evaluates
                                  them eight lanes to a pair (collide_polygons_group); more, a lane each */
@@ -494,6 +494,10 @@ void launch_phase_stamp(const DevWorld& w, int phase, cudaStream_t s);
 /* parts: allow the part-local solve (used where the world's size suits it) */
 void launch_colouring(const DevWorld& w, cudaStream_t s, int num_sms, bool parts, bool taped);
 int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int num_sms, bool parts, bool taped);
+/* threads per block of the kernel that sweeps such a world's constraints, and whether that kernel takes them
+ * (and the blocks per SM) from the launch configuration */
+int solver_threads(const DevWorld& w, int num_sms, bool parts, bool taped);
+bool reads_solver_config(const DevWorld& w, int num_sms, bool parts);
 /* time of impact of n shape pairs; every pointer is memory the device reaches. A definition that is no
  * circle, polygon or edge sets *bad, and no result is written then */
 void launch_time_of_impact(const b2g_fixture_def* da, const b2g_sweep* swa, const b2g_fixture_def* db,

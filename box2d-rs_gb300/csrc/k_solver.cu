@@ -1982,8 +1982,7 @@ int launch_solver(const DevWorld& w, const StepParams& sp, cudaStream_t s, int n
         launch_pdl(k_batch_positions, many, kBlock, kBatchSmem, s, w, spc);
         B2G_LAUNCHED(2);
     } else {
-        const bool wide = w.cfg_solver_auto ? wide_solver(w, num_sms) : w.cfg_solver_block == kSolveMaxBlock;
-        const int threads = w.cfg_coop_per_sm == 1 && wide ? kSolveMaxBlock : kBlock;
+        const int threads = solver_threads(w, num_sms, parts, taped);
         rc = (int)cudaLaunchCooperativeKernel((const void*)k_solve, dim3(blocks), dim3(threads), args, smem, s);
     }
     launch_pdl(k_solve_bodies, gb, kBlock, 0, s, w, spc);
@@ -2015,6 +2014,16 @@ int cluster_size(const DevWorld& w) {
 bool cluster_world(const DevWorld& w) {
     return w.n_fixtures > 0 && w.n_fixtures <= kClusterMaxProxies && w.n_bodies <= 2 * kClusterMaxProxies &&
            cluster_size(w) <= max_cluster();
+}
+
+bool reads_solver_config(const DevWorld& w, int num_sms, bool parts) {
+    return !cluster_world(w) && !(use_parts(w, num_sms, parts) && batch_parts(w, num_sms, false) > 0);
+}
+
+int solver_threads(const DevWorld& w, int num_sms, bool parts, bool taped) {
+    if (cluster_world(w) || (use_parts(w, num_sms, parts) && batch_parts(w, num_sms, taped) > 0)) return kBlock;
+    const bool wide = w.cfg_solver_block ? w.cfg_solver_block == kSolveMaxBlock : wide_solver(w, num_sms);
+    return w.cfg_coop_per_sm == 1 && wide ? kSolveMaxBlock : kBlock;
 }
 
 int launch_front(const DevWorld& w, const StepParams& sp, cudaStream_t s, bool parts, const TapeDev* tape) {

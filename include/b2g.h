@@ -595,10 +595,9 @@ typedef struct b2g_launch_config {
     int32_t traverse_block;       /* broadphase traversal threads per block: 32..256, power of two */
     int32_t tuning_steps;         /* out: steps the world's last b2g_autotune ran (ignored on set) */
     int32_t solver_block;         /* solver threads per block: 256, or 512 with one block per SM (more
-                                     loads in flight on large worlds); 0 on set: 256. A world that no
-                                     configuration was set for or tuned to reads 256 and takes 512
-                                     where it is larger or a batch; a large batch's sweeps have block
-                                     sizes of their own */
+                                     loads in flight on large worlds); 0 on set: by the world's size, as
+                                     where no configuration was set or tuned. Reads as what was set, or
+                                     as the threads that the world's solver runs with */
     int32_t collide_group;        /* narrowphase pairs per warp: a warp's batch of 32 contacts with at
                                      most this many polygon pairs evaluates each of them on 8 lanes (4
                                      pairs at a time); more, one lane per pair. 0..32, default 0: one
@@ -608,8 +607,8 @@ int b2g_get_launch_config(void* world, b2g_launch_config* out);
 int b2g_set_launch_config(void* world, const b2g_launch_config* config);
 /* Time the world's next steps under candidate configurations (one knob at a time: blocks per SM,
  * narrowphase block, traversal block, solver block, narrowphase pairs per warp (collide_group 0, 8 or
- * 32); each candidate 2 untimed steps and its share of steps_per_candidate timed steps),
- * keep the fastest for this world and for later worlds of the same size bucket (log2 bodies per
+ * 32); each candidate 2 untimed steps and its share of steps_per_candidate timed steps; knobs that the
+ * world's step does not read are left as they are), keep the fastest for this world and for later worlds of the same size bucket (log2 bodies per
  * world, single or batch) created in this process. The tuning steps are ordinary steps of the
  * world with the given dt and iterations. */
 int b2g_autotune(void* world, float dt, int32_t velocity_iterations, int32_t position_iterations,
