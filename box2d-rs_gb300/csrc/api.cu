@@ -3215,18 +3215,22 @@ struct QueryResult {
     unsigned long long total, counter;  /* the find's counter */
 };
 
-/* Device buffers of one query call, pieces of an allocation the world keeps for the next call (it is freed
- * with the world; a call that needed more than kQueryKeep bytes leaves none). The arrays themselves only
- * where the device cannot reach the caller's. */
-struct QueryBuffers {
-    QueryResult* result;
-    int2* lists;
-    uint32_t* found;
-    float* query;
-    uint32_t* world;
-    void* out;
-};
+/* Device buffers of one query call: pieces of an allocation that the world keeps for the next call (and frees
+ * with itself), or, for a call that needs more than kQueryKeep bytes, of one that the call frees. The arrays
+ * themselves only where the device cannot reach the caller's. */
 constexpr size_t kQueryKeep = 64u << 20;
+struct QueryBuffers {
+    QueryResult* result = nullptr;
+    int2* lists = nullptr;
+    uint32_t* found = nullptr;
+    float* query = nullptr;
+    uint32_t* world = nullptr;
+    void* out = nullptr;
+    unsigned char* own = nullptr; /* what the call frees */
+    QueryBuffers() = default;
+    QueryBuffers(const QueryBuffers&) = delete;
+    ~QueryBuffers() { cudaFree(own); }
+};
 
 int query_buffers(World* w, QueryBuffers& b, const float* query, const uint32_t* world, int n, int found, size_t out_bytes) {
     const size_t size[6] = {sizeof(QueryResult), found > 0 ? n * sizeof(int2) : 0, (size_t)found * sizeof(uint32_t),
@@ -3236,21 +3240,33 @@ int query_buffers(World* w, QueryBuffers& b, const float* query, const uint32_t*
         at[k] = total;
         total += (size[k] + 255) & ~(size_t)255;
     }
-    if (w->query_bytes < total || (w->query_bytes > kQueryKeep && total <= kQueryKeep)) {
-        CUDA_OK(w, cudaStreamSynchronize(w->stream));
-        cudaFree(w->query_mem);
-        w->query_mem = nullptr;
-        w->query_bytes = 0;
-        if (cudaMalloc((void**)&w->query_mem, total) != cudaSuccess) {
-            cudaGetLastError();
+    const bool keep = total <= kQueryKeep;
+    unsigned char* m = w->query_mem;
+    if (!keep || w->query_bytes < total) {
+        if (keep) {
+            CUDA_OK(w, cudaStreamSynchronize(w->stream));
+            cudaFree(w->query_mem);
             w->query_mem = nullptr;
+            w->query_bytes = 0;
+        }
+        m = nullptr;
+        if (cudaMalloc((void**)&m, total) != cudaSuccess) {
+            cudaGetLastError();
             return fail(w, B2G_ERR_OUT_OF_MEMORY, "no memory for a query's buffers");
         }
-        w->query_bytes = total;
+        if (keep) {
+            w->query_mem = m;
+            w->query_bytes = total;
+        } else {
+            b.own = m;
+        }
     }
-    unsigned char* m = w->query_mem;
-    b = {(QueryResult*)(m + at[0]), (int2*)(m + at[1]), (uint32_t*)(m + at[2]), (float*)(m + at[3]), world ? (uint32_t*)(m + at[4]) : nullptr,
-         m + at[5]};
+    b.result = (QueryResult*)(m + at[0]);
+    b.lists = (int2*)(m + at[1]);
+    b.found = (uint32_t*)(m + at[2]);
+    b.query = (float*)(m + at[3]);
+    b.world = world ? (uint32_t*)(m + at[4]) : nullptr;
+    b.out = m + at[5];
     if (query) CUDA_OK(w, cudaMemcpyAsync(b.query, query, size[3], cudaMemcpyHostToDevice, w->stream));
     if (world) CUDA_OK(w, cudaMemcpyAsync(b.world, world, size[4], cudaMemcpyHostToDevice, w->stream));
     return B2G_OK;
