@@ -1304,7 +1304,9 @@ int recover_overflow(World* w, const StepParams& sp) {
         int rc = grow_capacities(w, cc, pc);
         if (rc != B2G_OK) return rc;
         launch_touch_all_proxies(w->d, w->stream);
-        launch_broadphase(w->d, sp, w->stream, w->num_sms, PH_SOLVER, nullptr, BP_REPEAT);
+        DevWorld repeat = w->d;  /* the step's phase times are those of its own passes */
+        repeat.stamps += PH_COUNT;
+        launch_broadphase(repeat, sp, w->stream, w->num_sms, PH_SOLVER, nullptr, BP_REPEAT);
         swap_contacts(w);
         CUDA_OK(w, cudaGetLastError());
     }
@@ -1567,9 +1569,10 @@ int b2g_world_create(const b2g_world_def* def, void** out) {
         return B2G_ERR_UNSUPPORTED;
     }
     /* the phase stamps are not part of a saved state: an allocation of their own */
-    if (cudaMalloc((void**)&w->d.stamps, PH_COUNT * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMemsetAsync(w->d.stamps, 0, PH_COUNT * sizeof(unsigned long long), w->stream) != cudaSuccess) {
+    if (cudaMalloc((void**)&w->d.stamps, 2 * PH_COUNT * sizeof(unsigned long long)) != cudaSuccess ||
+        cudaMemsetAsync(w->d.stamps, 0, 2 * PH_COUNT * sizeof(unsigned long long), w->stream) != cudaSuccess) {
         cudaGetLastError();
+        cudaFree(w->d.stamps);
         cudaStreamDestroy(w->stream);
         delete w;
         return B2G_ERR_OUT_OF_MEMORY;

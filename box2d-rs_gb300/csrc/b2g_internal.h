@@ -354,7 +354,8 @@ struct DevWorld {
     uint32_t* sort_hist;
     int sort_hist_cap;
     int* cnt;
-    unsigned long long* stamps;  /* PH_COUNT: when the last step's phases ended (globaltimer, ns) */
+    unsigned long long* stamps;  /* PH_COUNT: when the last step's phases ended (globaltimer, ns); as many more take those
+                                    of a pass that the host repeats after growing the world's capacities */
 };
 
 /* The phases of a step whose ends are stamped, for the profile calls: a phase's end is written by one
