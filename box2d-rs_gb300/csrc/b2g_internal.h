@@ -533,12 +533,7 @@ void launch_query_write(const DevWorld& w, int n, const uint32_t* found, const i
                         cudaStream_t s);
 
 /* primitives (k_prims.cu) */
-void scan_exclusive_u32(const uint32_t* in, uint32_t* out, const int* d_n, int max_n, uint32_t* tmp, int* d_total,
-                        cudaStream_t s);
-/* stable LSD radix sort of (key, value) pairs by key bits [0, bits); n from device; result in *_a. */
-void radix_sort_pairs(unsigned long long* key_a, uint32_t* val_a, unsigned long long* key_b, uint32_t* val_b,
-                      const int* d_n, int max_n, int bits, uint32_t* hist, cudaStream_t s);
-/* the same sort as one cooperative launch (2 grid barriers per 8-bit pass; inputs of at most
+/* a stable sort by key bits [0, bits) as one cooperative launch (2 grid barriers per 8-bit pass; inputs of at most
  * 2048 items are sorted by a single block, inputs of at most 8192 by a rank count in three small
  * kernels). The caller has zeroed cnt[barrier_word] (the launch's grid barriers) and, unless zero_or_max
  * and max_n > kSortRankWords, hist[0, kSortRankWords). zero_or_max: the count is known to be 0 or max_n (no
