@@ -141,6 +141,7 @@ enum {
     CNT_BP_LIST = 60,        /* leaves of moved proxies listed for this pass's traversal (in bp_val_alt) */
     CNT_PART_SPLIT = 61,     /* a kept partition of more parts than SMs has split a world */
     CNT_ISLAND_SPAN = 62,    /* a kinematic body may have made an island of several parts */
+    CNT_PART_REMADE = 63,    /* partitions made afresh because a kept one had split a world, since the world was made */
     CNT_SIZE = 64
 };
 

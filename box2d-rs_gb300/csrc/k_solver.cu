@@ -461,6 +461,7 @@ __device__ __forceinline__ bool colour_pass(const DevWorld& w, int nparts) {
         if (!grid_barrier(w)) return false;
         if (P <= w.num_sms || rebalance || ((volatile int*)w.cnt)[CNT_PART_SPLIT] == 0) break;
         rebalance = true;
+        if (gtid == 0) ++w.cnt[CNT_PART_REMADE];
     }
     /* the kept colours are taken at their bodies; the constraints without one are listed (in s_cons, free
      * until the slots are placed): the rounds go over the list alone, as only its members ever offer */
