@@ -776,7 +776,7 @@ def main():
         with open(tf) as f:
             rec = json.load(f)
         if rec.get("workload") == WORKLOAD and rec.get("window") == window:
-            traffic_rec = rec.get("dram_bytes_per_launch", {})
+            traffic_rec = rec.get("dram_bytes_per_step", {})  # by phase, over its kernels
     phases = {}
     for ph, ms in phase_time.items():
         if ms <= 0:
@@ -785,7 +785,7 @@ def main():
         ach = b / (ms / args.steps / 1e3) / 1e9
         kern = PHASE_KERNEL[ph]
         phases[ph] = {"kernel": kern, "ms_per_step": ms / args.steps, "algorithmic_bytes_per_step": b,
-                      "achieved": ach, "frac": ach / peak, "traffic": traffic_rec.get(kern)}
+                      "achieved": ach, "frac": ach / peak, "traffic": traffic_rec.get(ph)}
     dominant = max(phases, key=lambda k: phases[k]["ms_per_step"])
     d = phases[dominant]
     line = {
@@ -801,8 +801,8 @@ def main():
         "roofline": {"bound": "hbm", "kernel": d["kernel"], "kernel_phase": dominant, "achieved": d["achieved"],
                      "peak": peak, "unit": "GB/s", "frac": d["frac"], "peak_kind": peak_kind,
                      "traffic": d["traffic"], "algorithmic_bytes_per_launch": d["algorithmic_bytes_per_step"],
-                     "traffic_note": ("DRAM bytes per launch from one ncu capture of the same window "
-                                      "(profiles/roofline_traffic.json)") if d["traffic"] else None},
+                     "traffic_note": ("DRAM bytes a step of all kernels of the phase, from an ncu capture of steps "
+                                      "in the same window (profiles/roofline_traffic.json)") if d["traffic"] else None},
         "roofline_phases": phases,
         "work_per_step": {k: v / args.steps for k, v in work.items()},
         "phase_ms_per_step": {k: v / args.steps for k, v in fine_ms.items()},
