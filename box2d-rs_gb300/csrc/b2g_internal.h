@@ -482,7 +482,10 @@ void launch_islands_and_constraints(const DevWorld& w, const StepParams& sp, cud
 /* Worlds of up to kClusterMaxProxies proxies (and twice as many bodies) run the whole of islands,
  * colouring and solver, and of a taped step's recording (tape), as one kernel on one thread-block cluster, and the whole
  * broadphase and contact merge as another (launch_back): cluster_world says whether a world does, given
- * the device's largest cluster. */
+ * the device's largest cluster. The step on the cluster and on the grid, us: a settled world of 1000 bodies 275 and
+ * 297, of 4000 402 and 463; boxes in a pile, 1000 290 and 300, 3000 380 and 445, 4000 434 and 443; 60 bridges 415
+ * and 490; 4000 that may sleep, 445 and 469; but 4000 bodies in flight with few contacts 342 and 312, and 4000 of
+ * eight constraints each 1744 and 1524. */
 constexpr int kClusterMaxProxies = kClusterMaxBlocks * 256;
 bool cluster_world(const DevWorld& w);
 int cluster_size(const DevWorld& w);

@@ -31,13 +31,11 @@
  * to the same float (2^-42 relative, above the error of either computation; with k != 0 also 2^-60,
  * the reduction's): then the true value and the double evaluation round to that float too. Otherwise
  * (about one call in 2^17), and for |x| > 8192, inf and NaN, the double routine runs.
- * The solver's position sweeps are chains of these calls (two bodies, two points), so their length
- * is what counts: about 40 dependent operations here. The earlier form (a 1/32 table, pairs throughout,
- * and the double routine for x = 0, the angle of most static bodies) took 4.0 us per colour of the
- * 210-box pyramid's position sweeps, this one takes 1.3 us (a call 380 -> 220 cycles against this file's
- * form with branches, integer conversions and a normalised remainder). tests/trig_check.cpp compares the two routines on every float in
- * the fast range.
- */
+ * The solver's position sweeps are chains of these calls (two bodies, two points), so their length is what
+ * counts: about 40 dependent operations and 220 cycles a call, 374 for two side by side (double-precision
+ * evaluation, which static bodies' zero angles once took, made a colour of the 210-box pyramid's position
+ * sweeps 4.0 us; it takes 1.3). tests/trig_check.cpp compares the two routines on floats of the fast range,
+ * tests/trig_check_gpu.cu on every one; tests/test_trig_table.py makes the table's rows again. */
 #ifndef B2G_TRIG_H
 #define B2G_TRIG_H
 

@@ -277,7 +277,6 @@ __device__ __forceinline__ float4 box_union(float4 a, float4 b) {
     return make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fmaxf(a.z, b.z), fmaxf(a.w, b.w));
 }
 
-/* arrival count with release (this thread's box store before it) and acquire (the sibling's after it) */
 /* puts a box in a node's first record and returns what was there, in one 16-byte exchange */
 __device__ __forceinline__ float4 exchange_box(float4* p, float4 v) {
     float4 old;
@@ -621,7 +620,8 @@ __device__ __forceinline__ unsigned check_batch(const DevWorld& w, const StepPar
 /* Threads of an SM, the four blocks its registers allow: 100k bodies in flight (55k moved proxies) take
  * 99 us, and took 146 with a warp for every 32 proxies, moved or not; 120 and 162 with three and two blocks,
  * 116 with a second wave, 120 with five blocks of 48 registers. 10k bodies: 34 (100) us, a 250k pile of 14k
- * moved ones: 52 (104). */
+ * moved ones: 52 (104). In the falling 100k scene the unmoved neighbours diluted a dense region's warps, which
+ * now hold its moved proxies alone: 150 (92) us at step 312, 172 (195) at step 606. */
 constexpr int kTraverseThreads = 1024;
 constexpr int kLeafQueue = 224;  /* 31 left over + 32 lanes x 4 leaves in one round, or the setup's
                                     2 single-proxy roots per lane */
@@ -921,7 +921,7 @@ __device__ __forceinline__ void sort_cluster(const DevWorld& w, unsigned long lo
 
 /* update_pairs, add_pair and the merge of a world of a few thousand proxies as one kernel on one
  * cluster: the passes of the kernels above, separated by cluster barriers instead of launches. A kept
- * hierarchy with no new pair takes five barriers; as 20 launches the same pass took 62 us for a 16-body
+ * hierarchy with no new pair takes four barriers; as 20 launches the same pass took 62 us for a 16-body
  * world, most of it launch and drain times. The merge counts each block's chunk of the table, so that
  * one more barrier gives every contact its rank. */
 __global__ void __launch_bounds__(kBlock) k_back(const __grid_constant__ DevWorld w, const __grid_constant__ StepParams sp) {

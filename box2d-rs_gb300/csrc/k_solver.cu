@@ -806,8 +806,8 @@ constexpr int kBndBytes = kBndSlots * (int)sizeof(VelSlot);
  * each, between the halves of one grid barrier, instead of a grid barrier after each colour's share of
  * every block. Solver, us, spread and in one block: 37 boundary slots of 31 parts 146 and 130, 170 of 117
  * parts 174 and 165, 390 of 152 parts 213 and 214, 2400 of 39 parts 366 and 503; on a cluster, whose blocks
- * load the slots' bodies from L2 again after each barrier, 50 slots of 5 parts 237 and 208, 290 of 11 parts
- * 290 and 262. */
+ * load the slots' bodies from L2 again after each barrier, 390 slots of 11 parts 246 and 219, 470 of 15 parts
+ * 263 and 240, 500 of 11 parts 250 and 222, 820 of 15 parts 246 and 247. */
 constexpr int kOneBlockSlots = 256, kOneBlockSlotsCluster = 1024;
 
 __device__ __forceinline__ void bnd_range(const PartCtx& pc, int c, int* lo, int* hi) {

@@ -11,7 +11,7 @@
  * bit.
  *
  * The caller's arrays (144-byte definitions, 40-byte sweeps) are read as they are, and the shapes
- * (gift-wrapped hulls among them) are built by the pair's thread: 100k pairs take 0.60 ms with the call's
+ * (gift-wrapped hulls among them) are built by the pair's thread: 100k pairs take 0.45 ms with the call's
  * overheads, where a host loop over the shapes, copies and allocations took 10.7 ms. A block reads its definitions (up to 128) in one contiguous piece into shared memory
  * (8 bytes a thread, coalesced: the array may lie in host memory, across C2C) and every thread takes
  * its own from there, rows an odd number of words apart so that lanes meet different banks.
