@@ -2125,7 +2125,7 @@ int b2g_get_body_states_async(void* p, uint32_t first, uint32_t count, b2g_body_
     B2G_LAUNCHED(1);
     CUDA_OK(w, cudaEventRecord(w->ev_packed[i], w->stream));
     CUDA_OK(w, cudaStreamWaitEvent(w->copy_stream, w->ev_packed[i], 0));
-    if (w->pageable) {
+    if (w->pageable && ((uintptr_t)out & 15u) == 0) {  /* (an array off 16 bytes cannot take the kernel's stores) */
         const size_t n4 = (size_t)count * sizeof(b2g_body_state) / sizeof(float4);
         k_copy_states<<<grid_for((int)std::min<size_t>(n4, 1u << 30), 256, w->num_sms * 4), 256, 0, w->copy_stream>>>(
             (const float4*)w->d_ring[i], (float4*)out, n4);
@@ -2156,10 +2156,10 @@ int b2g_get_body_states(void* p, uint32_t first, uint32_t count, b2g_body_state*
     if (count == 0) return B2G_OK;
     if (w->device_authoritative && (int)(first + count) <= w->uploaded_bodies) {
         /* one kernel packs the caller's layout; with coherent access to pageable host memory
-         * (Grace's C2C link) it writes straight into the caller's buffer, else into a device
-         * buffer that is copied out in one piece */
+         * (Grace's C2C link) it writes straight into the caller's buffer, else (or where that is off a
+         * 4-byte boundary) into a device buffer that is copied out in one piece */
         const int grid = grid_for((int)count, 256, w->num_sms * 8);
-        if (w->pageable) {
+        if (w->pageable && ((uintptr_t)out & 3u) == 0) {
             int status = 0;
             k_pack_states<<<grid, kPackBlock, 0, w->stream>>>(w->d, first, count, out, &status);
             B2G_LAUNCHED(1);
