@@ -76,8 +76,9 @@ def _batch_on_kinematic(worlds, per):
     return s, ground
 
 
-def test_batch_with_kinematic_bodies_lockstep(built):
-    s, _ = _batch_on_kinematic(60, 100)
+@pytest.mark.parametrize("worlds", [30, 60])  # on one cluster and on the grid
+def test_batch_with_kinematic_bodies_lockstep(built, worlds):
+    s, _ = _batch_on_kinematic(worlds, 100)
     recs, gpu, _ = parity.lockstep(dict(s, allow_sleep=False), 60)
     for r in recs:
         assert r["hook_misses"] == 0 and r["bitexact_bodies"], r
